@@ -39,6 +39,9 @@ StepLaunch get_learned_step_d2q9(int, int, int);
 StepLaunch get_learned_step_d3q19(int, int, int);
 StepLaunch get_learned_step_d3q27(int, int, int);
 void pack_closure(const lbm_closure_t& c, ClosureDev& d, ClosureUniform& u);
+cudaError_t launch_rho_u_d2q9(const RhoUArgs&, bool, bool, bool, cudaStream_t);
+cudaError_t launch_rho_u_d3q19(const RhoUArgs&, bool, bool, bool, cudaStream_t);
+cudaError_t launch_rho_u_d3q27(const RhoUArgs&, bool, bool, bool, cudaStream_t);
 }  // namespace lbm
 
 using namespace lbm;
@@ -294,6 +297,13 @@ lbm_status step_once(lbm_handle* h, const void* f_in, void* f_out, float* bc, co
 
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 int ilog2(int v) { int r = 0; while ((1 << r) < v) ++r; return r; }
+
+// Density and velocity, or with qcrit the Q-criterion.
+cudaError_t launch_rho_u(int lattice, const RhoUArgs& a, bool f16, bool eso, bool qcrit, cudaStream_t s) {
+    return lattice == LBM_D2Q9 ? launch_rho_u_d2q9(a, f16, eso, qcrit, s)
+         : lattice == LBM_D3Q19 ? launch_rho_u_d3q19(a, f16, eso, qcrit, s)
+                                : launch_rho_u_d3q27(a, f16, eso, qcrit, s);
+}
 
 template <class F>
 lbm_status dispatch_lattice(int lattice, F&& f) {
@@ -740,6 +750,7 @@ lbm_status lbm_q_criterion(lbm_handle* h, float* q, const void* f, const float* 
     if (!q || !u || !f || !bc || !flags) return fail(LBM_EINVAL, "null buffer");
     RhoUArgs a;
     a.lay = h->lay;
+    a.brick = make_brick(h->lay, lattice_d(h->grid.lattice));
     a.f = f;
     a.bc = bc;
     a.flags = flags;
@@ -753,19 +764,8 @@ lbm_status lbm_q_criterion(lbm_handle* h, float* q, const void* f, const float* 
     a.even = after_odd_step ? 1 : 0;
     const bool f16 = h->cfg.use_float16c != 0, eso = h->cfg.lbm_method == LBM_ESOTERIC_PULL;
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t nb = blocks_for(h->lay.ncells, 256);
-    return dispatch_lattice(h->grid.lattice, [&](auto Lt) -> lbm_status {
-        using L = decltype(Lt);
-        if (f16) {
-            if (eso) rho_u_kernel<L, true, true, true><<<nb, 256, 0, s>>>(a);
-            else rho_u_kernel<L, true, false, true><<<nb, 256, 0, s>>>(a);
-        } else {
-            if (eso) rho_u_kernel<L, false, true, true><<<nb, 256, 0, s>>>(a);
-            else rho_u_kernel<L, false, false, true><<<nb, 256, 0, s>>>(a);
-        }
-        LBM_CK(cudaGetLastError());
-        return LBM_OK;
-    });
+    LBM_CK(launch_rho_u(h->grid.lattice, a, f16, eso, true, s));
+    return LBM_OK;
 }
 
 lbm_status lbm_compute_rho_u(lbm_handle* h, float* rho, float* u, const void* f, const float* bc,
@@ -774,6 +774,7 @@ lbm_status lbm_compute_rho_u(lbm_handle* h, float* rho, float* u, const void* f,
     if (!rho || !u || !f || !bc || !flags) return fail(LBM_EINVAL, "null buffer");
     RhoUArgs a;
     a.lay = h->lay;
+    a.brick = make_brick(h->lay, lattice_d(h->grid.lattice));
     a.f = f;
     a.bc = bc;
     a.flags = flags;
@@ -787,19 +788,8 @@ lbm_status lbm_compute_rho_u(lbm_handle* h, float* rho, float* u, const void* f,
     a.even = after_odd_step ? 1 : 0;
     const bool f16 = h->cfg.use_float16c != 0, eso = h->cfg.lbm_method == LBM_ESOTERIC_PULL;
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t nb = blocks_for(h->lay.ncells, 256);
-    return dispatch_lattice(h->grid.lattice, [&](auto Lt) -> lbm_status {
-        using L = decltype(Lt);
-        if (f16) {
-            if (eso) rho_u_kernel<L, true, true><<<nb, 256, 0, s>>>(a);
-            else rho_u_kernel<L, true, false><<<nb, 256, 0, s>>>(a);
-        } else {
-            if (eso) rho_u_kernel<L, false, true><<<nb, 256, 0, s>>>(a);
-            else rho_u_kernel<L, false, false><<<nb, 256, 0, s>>>(a);
-        }
-        LBM_CK(cudaGetLastError());
-        return LBM_OK;
-    });
+    LBM_CK(launch_rho_u(h->grid.lattice, a, f16, eso, false, s));
+    return LBM_OK;
 }
 
 lbm_status lbm_reduce_mass_momentum(lbm_handle* h, const void* f, const uint8_t* flags, int32_t after_odd_step,
