@@ -75,8 +75,7 @@ struct ChunkArgs {
 template <class L, bool F16C, bool ESO>
 __global__ void __launch_bounds__(kChunkThreads) mass_chunk_kernel(const ChunkArgs a) {
     using S = typename Pop<F16C>::T;
-    constexpr int Q = L::Q, D = L::D;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    MassSum sum;
     const uint32_t begin = blockIdx.x * kChunkCells;
     for (uint32_t k = 0; k < kCellsPerThread; ++k) {
         const uint32_t n = begin + k * kChunkThreads + threadIdx.x;
@@ -85,25 +84,12 @@ __global__ void __launch_bounds__(kChunkThreads) mass_chunk_kernel(const ChunkAr
         if ((flag & 0x0F) == LBM_FLAG_SOLID || (flag & LBM_FLAG_EXCLUDE)) continue;
         Nbr nb;
         const Cell c = decode_cell<L>(a.lay, n, nb);
-        float f[Q];
+        float f[L::Q];
         gather_post<L, F16C, ESO>((const S*)a.f, a.lay, c, nb, a.after_odd != 0, f);
-        double rho = a.ddf ? 1.0 : 0.0;
-        double m[3] = {0.0, 0.0, 0.0};
-        static_for<0, Q>([&](auto qc) {
-            constexpr int q = qc.value;
-            rho += (double)f[q];
-            static_for<0, D>([&](auto dc) {
-                constexpr int d = dc.value;
-                if constexpr (L::c(q, d) > 0) m[d] += (double)f[q];
-                else if constexpr (L::c(q, d) < 0) m[d] -= (double)f[q];
-            });
-        });
-        acc[0] += rho;
-        acc[1] += m[0];
-        acc[2] += m[1];
-        acc[3] += m[2];
+        sum.add<L>(f, a.ddf != 0);
     }
-    block_sum_store<4>(acc, a.partial + (size_t)blockIdx.x * 4);
+    sum.flush<L::D>();
+    block_sum_store<4>(sum.acc, a.partial + (size_t)blockIdx.x * 4);
 }
 
 lbm_status nfail(lbm_status s, const std::string& m) {

@@ -1,7 +1,8 @@
 """The kernels between the lattice and the row-major fields (lbm_fields.cuh), against the oracle bit
 for bit, at the sizes where their bricks of 32 lanes x 32 planes have remainders: extents around a
 brick's along every axis, tile rows shorter and longer than a warp, the untiled layout, and domains
-with walls, mixed flags or none (a brick without any flag takes the form that gathers none)."""
+with walls, mixed flags or none (a brick without any flag takes the form that gathers none); the
+mass and momentum sums."""
 from __future__ import annotations
 
 import numpy as np
@@ -58,3 +59,40 @@ def test_outputs_at_brick_edges(lat, shape, tile, kind, meth, f16):
     q_ref = oracle.q_criterion(cfg, grid, 32, f0, bc, flags, u_ref, 0.7, True, fill=-7.0)
     assert np.array_equal(q.cpu().numpy().reshape(grid.shape), q_ref, equal_nan=True)
 
+@pytest.mark.parametrize("scale", ["flow", "tiny", "huge", "mixed"])
+@pytest.mark.parametrize("lat,meth,ddf", [("D2Q9", "db", False), ("D3Q19", "db", True), ("D3Q27", "eso", True)])
+def test_mass_momentum_sums(lat, meth, ddf, scale):
+    """The reduction's split sums against a float64 sum of the same populations: ordinary cells, cells
+    too small or too large for the split (added in float64) and both in one domain.  Float64
+    summation bounds both errors by 2^-53 times the terms of a cell and of the reduction tree
+    (below 2^10 of them) relative to the sum of magnitudes."""
+    shape = {"D2Q9": (48, 34, 1), "D3Q19": (20, 18, 16), "D3Q27": (12, 10, 9)}[lat]
+    grid = make_grid(lat, shape, "untiled")
+    m = LBM_method.DOUBLE_BUFFER if meth == "db" else LBM_method.ESOTERIC_PULL
+    cfg = LBM_Config(m, DDF_shift=ddf)
+    rng = np.random.default_rng(11)
+    f = initial_f(grid, cfg, rng).reshape(grid.Q, -1)
+    if scale == "tiny":
+        f *= np.float32(2.0 ** -40)
+    elif scale == "huge":
+        f *= np.float32(1e30)
+    elif scale == "mixed":
+        f *= np.float32(2.0) ** rng.integers(-60, 12, f.shape[1]).astype(np.float32)
+        f[:, rng.random(f.shape[1]) < 0.2] = 0.0
+    f = np.ascontiguousarray(f).reshape(-1)
+    nat = grid.layouts.from_layout(f, grid.Q).transpose(3, 0, 1, 2).astype(np.float64)
+    g = nat.copy()
+    if meth == "eso":  # after an odd step: f[pos] was stored at x + c in slot pos, f[neg] at x in slot neg
+        for p in range(1, grid.Q, 2):
+            c = [int(v) for v in grid.lattice.directions[p]]
+            g[p] = np.roll(nat[p], [-v for v in c[:grid.D]], axis=tuple(range(grid.D)))
+    want = [g.sum() + (grid.num_points if ddf else 0)]
+    size = [np.abs(g).sum() + (grid.num_points if ddf else 0)]
+    for d in range(grid.D):
+        c = grid.lattice.directions[:, d].astype(np.float64)
+        want.append((g * c[:, None, None, None]).sum())
+        size.append(np.abs(g * c[:, None, None, None]).sum())
+    flags = torch.zeros(grid.num_points, dtype=torch.uint8, device="cuda")
+    got = Solver(grid, cfg).mass_momentum(to_dev(f), flags, after_odd_step=True)
+    for k in range(grid.D + 1):
+        assert abs(got[k] - want[k]) <= 2.0 ** -43 * size[k], (k, got[k], want[k])
