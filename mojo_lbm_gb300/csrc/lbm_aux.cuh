@@ -1,5 +1,5 @@
-// Auxiliary kernels around the step: initial state, float64 conservation reductions, link-wise
-// interpolated bounce-back, momentum-exchange drag (macroscopic outputs: lbm_fields.cuh).
+// Auxiliary kernels around the step: float64 conservation reductions, link-wise interpolated
+// bounce-back, momentum-exchange drag (initial state and macroscopic outputs: lbm_fields.cuh).
 #pragma once
 
 #include "lbm_fields.cuh"
@@ -26,74 +26,6 @@ __device__ __forceinline__ Cell decode_cell(const LayoutDesc& lay, uint32_t n, N
     c.r = ((uint32_t)c.x * (uint32_t)lay.ny + (uint32_t)c.y) * (uint32_t)lay.nz + (uint32_t)c.z;
     cell_nbr<L>(lay, c, nb);
     return c;
-}
-
-struct InitArgs {
-    LayoutDesc lay;
-    void* f;
-    const float* u;     // D * ncells, row-major per component, or null
-    const float* grad;  // D*D * ncells, or null
-    float rho, tau;
-    int32_t ddf, esoteric;
-};
-
-// initialize_f_from_func (src/lbm/preprocess/initial_condition.mojo:86-179) with fi_neq
-// (:182-234); esoteric pull stores with the odd-step pattern (:172-174).
-template <class L, bool F16C>
-__global__ void init_kernel(const InitArgs a) {
-    using P = Pop<F16C>;
-    using S = typename P::T;
-    constexpr int Q = L::Q, D = L::D;
-    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= a.lay.ncells) return;
-    Nbr nb;
-    const Cell c = decode_cell<L>(a.lay, n, nb);
-    const uint32_t N = a.lay.ncells, T = a.lay.T;
-    float u[3] = {0.f, 0.f, 0.f};
-    if (a.u) static_for<0, D>([&](auto dc) { u[dc.value] = a.u[(size_t)N * dc.value + c.r]; });
-    float uu = 0.f;
-    static_for<0, D>([&](auto dc) { uu += u[dc.value] * u[dc.value]; });
-    float S_[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    if (a.grad)
-        static_for<0, D>([&](auto ac) {
-            static_for<0, D>([&](auto bc) {
-                constexpr int A = ac.value, B = bc.value;
-                S_[A][B] = 0.5f * (a.grad[(size_t)N * (A * D + B) + c.r] + a.grad[(size_t)N * (B * D + A) + c.r]);
-            });
-        });
-    float f[Q];
-    static_for<0, Q>([&](auto qc) {
-        constexpr int q = qc.value;
-        float fi = feq<L, q>(a.rho, u, uu, a.ddf != 0);
-        if (a.grad) {
-            float neq = 0.f;
-            static_for<0, D>([&](auto ac) {
-                static_for<0, D>([&](auto bc) {
-                    constexpr int A = ac.value, B = bc.value;
-                    constexpr float Qab = (float)(L::c(q, A) * L::c(q, B)) - (A == B ? (float)(1.0 / 3.0) : 0.f);
-                    neq += Qab * S_[A][B];
-                });
-            });
-            neq *= (-wf<L>(q) * a.rho * a.tau * 3.f) * ((a.tau - 1.f) / a.tau);
-            fi += neq;
-        }
-        f[q] = fi;
-    });
-    S* fs = (S*)a.f;
-    const uint64_t TQ = (uint64_t)T * Q;
-    const uint64_t own = c.loc + TQ * c.tile;
-    if (!a.esoteric) {
-        static_for<0, Q>([&](auto qc) { P::st(fs + own + (uint64_t)T * qc.value, f[qc.value]); });
-    } else {
-        P::st(fs + own, f[0]);
-        static_for<1, Q - 1, 2>([&](auto qc) {
-            constexpr int pos = qc.value, neg = pos + 1;
-            constexpr int sx = L::c(pos, 0), sy = L::c(pos, 1), sz = L::c(pos, 2);
-            const uint64_t nbase = nb.template loc<sx, sy, sz>() + TQ * nb.template til<sx, sy, sz>();
-            P::st(fs + nbase + (uint64_t)T * pos, f[pos]);
-            P::st(fs + own + (uint64_t)T * neg, f[neg]);
-        });
-    }
 }
 
 // Post-collision populations a cell owns after the last completed step, before streaming:

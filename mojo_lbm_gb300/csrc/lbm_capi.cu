@@ -39,6 +39,9 @@ StepLaunch get_learned_step_d2q9(int, int, int);
 StepLaunch get_learned_step_d3q19(int, int, int);
 StepLaunch get_learned_step_d3q27(int, int, int);
 void pack_closure(const lbm_closure_t& c, ClosureDev& d, ClosureUniform& u);
+cudaError_t launch_init_d2q9(const InitArgs&, bool, cudaStream_t);
+cudaError_t launch_init_d3q19(const InitArgs&, bool, cudaStream_t);
+cudaError_t launch_init_d3q27(const InitArgs&, bool, cudaStream_t);
 cudaError_t launch_rho_u_d2q9(const RhoUArgs&, bool, bool, bool, cudaStream_t);
 cudaError_t launch_rho_u_d3q19(const RhoUArgs&, bool, bool, bool, cudaStream_t);
 cudaError_t launch_rho_u_d3q27(const RhoUArgs&, bool, bool, bool, cudaStream_t);
@@ -273,8 +276,6 @@ lbm_status tile_summary(lbm_handle* h, const uint8_t* flags, cudaStream_t s) {
     return LBM_OK;
 }
 
-uint32_t blocks_for(uint32_t n, int threads) { return (n + (uint32_t)threads - 1u) / (uint32_t)threads; }
-
 lbm_status check_handle(const lbm_handle* h) {
     if (!h) return fail(LBM_EINVAL, "null handle");
     return LBM_OK;
@@ -297,6 +298,12 @@ lbm_status step_once(lbm_handle* h, const void* f_in, void* f_out, float* bc, co
 
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 int ilog2(int v) { int r = 0; while ((1 << r) < v) ++r; return r; }
+
+cudaError_t launch_init(int lattice, const InitArgs& a, bool f16, cudaStream_t s) {
+    return lattice == LBM_D2Q9 ? launch_init_d2q9(a, f16, s)
+         : lattice == LBM_D3Q19 ? launch_init_d3q19(a, f16, s)
+                                : launch_init_d3q27(a, f16, s);
+}
 
 // Density and velocity, or with qcrit the Q-criterion.
 cudaError_t launch_rho_u(int lattice, const RhoUArgs& a, bool f16, bool eso, bool qcrit, cudaStream_t s) {
@@ -725,6 +732,7 @@ lbm_status lbm_init_equilibrium(lbm_handle* h, void* f, float rho, float tau, co
     if (!f) return fail(LBM_EINVAL, "null f");
     InitArgs a;
     a.lay = h->lay;
+    a.brick = make_brick(h->lay, lattice_d(h->grid.lattice));
     a.f = f;
     a.u = u;
     a.grad = grad;
@@ -732,16 +740,8 @@ lbm_status lbm_init_equilibrium(lbm_handle* h, void* f, float rho, float tau, co
     a.tau = tau;
     a.ddf = h->cfg.DDF_shift;
     a.esoteric = h->cfg.lbm_method == LBM_ESOTERIC_PULL;
-    const bool f16 = h->cfg.use_float16c != 0;
-    cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t nb = blocks_for(h->lay.ncells, 256);
-    return dispatch_lattice(h->grid.lattice, [&](auto Lt) -> lbm_status {
-        using L = decltype(Lt);
-        if (f16) init_kernel<L, true><<<nb, 256, 0, s>>>(a);
-        else init_kernel<L, false><<<nb, 256, 0, s>>>(a);
-        LBM_CK(cudaGetLastError());
-        return LBM_OK;
-    });
+    LBM_CK(launch_init(h->grid.lattice, a, h->cfg.use_float16c != 0, (cudaStream_t)stream));
+    return LBM_OK;
 }
 
 lbm_status lbm_q_criterion(lbm_handle* h, float* q, const void* f, const float* bc, const uint8_t* flags,

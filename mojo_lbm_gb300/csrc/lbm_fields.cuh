@@ -1,4 +1,5 @@
-// Kernels between the lattice and the row-major fields (rho, u, Q): macroscopic outputs.
+// Kernels between the lattice and the row-major fields (rho, u, Q): initial state and macroscopic
+// outputs.
 //
 // The lattice's tiles run x fastest (src/lbm/layoutstruct.mojo:37-92), the fields z fastest in 3D
 // and y fastest in 2D (examples/LDC.mojo:47-48), so a warp that reads 32 consecutive cells of a
@@ -456,6 +457,142 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
             a.q[r] = 0.25f * w2 - 0.5f * field[0][slot];
         }
     }
+}
+
+struct InitArgs {
+    LayoutDesc lay;
+    Brick brick;
+    void* f;
+    const float* u;     // D * ncells, row-major per component, or null
+    const float* grad;  // D*D * ncells, or null
+    float rho, tau;
+    int32_t ddf, esoteric;
+};
+
+// initialize_f_from_func (src/lbm/preprocess/initial_condition.mojo:86-179) with fi_neq
+// (:182-234); esoteric pull stores with the odd-step pattern (:172-174).
+// One block per brick: u and the symmetric part of grad come in in the fields' order and wait in
+// shared memory (38 KB in 3D), then the populations are computed and stored plane by plane in the
+// lattice's order.  256^3 D3Q19 float32 with u and grad (2.07 GB, floor 305 us): 1080 us with one
+// thread per cell in tile order, 428 us with bricks (at rest, 1.27 GB: 376 and 260 us); bound by the
+// arithmetic of the non-equilibrium part (issue-active 68 %).
+template <class L, bool F16C, class Off>
+__global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_constant__ InitArgs a) {
+    using P = Pop<F16C>;
+    using S = typename P::T;
+    constexpr int Q = L::Q, D = L::D, NS = L::NS;
+    __shared__ float field[D + NS][kBrickField];
+    __shared__ PlaneTable<Off> planes;
+    const Brick& b = a.brick;
+    const uint32_t N = a.lay.ncells;
+    const Off oT = (Off)a.lay.T, TQ = oT * Q;
+    int32_t x0, y0, z0;
+    brick_origin(b, D, x0, y0, z0);
+    if constexpr (D == 3) fill_planes<Off>(a.lay, b, z0, TQ, planes);
+    const uint32_t sf = b.sf;
+    if (a.u || a.grad) {
+#pragma unroll 2
+        for (uint32_t i = threadIdx.x; i < (32u << b.sp); i += kBrickThreads) {
+            const uint32_t fast = i & ((1u << sf) - 1u), g = i >> sf;
+            const int32_t x = x0 + (int32_t)(D == 3 ? g >> b.sby : g);
+            const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : 0;
+            if (x >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
+            const uint32_t slot = g * ((1u << sf) + 1u) + fast;
+            const uint32_t r = ((uint32_t)x * (uint32_t)a.lay.ny + (uint32_t)y) * (uint32_t)a.lay.nz + (uint32_t)z;
+            if (a.u) static_for<0, D>([&](auto dc) { field[dc.value][slot] = __ldg(a.u + (size_t)N * dc.value + r); });
+            if (a.grad)
+                static_for<0, NS>([&](auto nc) {
+                    constexpr int n = nc.value, A = sa<L>(n), B = sb<L>(n);
+                    field[D + n][slot] = 0.5f * (__ldg(a.grad + (size_t)N * (A * D + B) + r) +
+                                                 __ldg(a.grad + (size_t)N * (B * D + A) + r));
+                });
+        }
+        __syncthreads();
+    }
+
+    const uint32_t lane = threadIdx.x & 31u;
+    const int32_t lx = (int32_t)(lane & ((1u << b.sbx) - 1u)), ly = (int32_t)(lane >> b.sbx);
+    const int32_t x = x0 + lx;
+    S* fs = (S*)a.f;
+    CellDeltas<Off> d;
+    Off own_xy;
+    auto row_deltas = [&](int32_t y) -> Off {
+        const uint32_t by = a.lay.d_ty.div((uint32_t)y), iy = (uint32_t)y - by * (uint32_t)a.lay.ty;
+        axis_deltas<Off>(iy, (uint32_t)a.lay.ty, by, (uint32_t)a.lay.nty, (Off)a.lay.tx, TQ * (Off)a.lay.ntx, d.y);
+        return (Off)iy * (Off)a.lay.tx + TQ * (Off)a.lay.ntx * (Off)by;
+    };
+    {
+        const uint32_t bx = a.lay.d_tx.div((uint32_t)x), ix = (uint32_t)x - bx * (uint32_t)a.lay.tx;
+        axis_deltas<Off>(ix, (uint32_t)a.lay.tx, bx, (uint32_t)a.lay.ntx, 1, TQ, d.x);
+        own_xy = (Off)ix + TQ * (Off)bx;
+        if constexpr (D == 3) own_xy += row_deltas(y0 + ly);
+    }
+#pragma unroll 1
+    for (int32_t p = (int32_t)(threadIdx.x >> 5); p < (1 << b.sp); p += (int32_t)(kBrickThreads / 32u)) {
+        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : 0;
+        if (x >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
+        const uint32_t slot = D == 3 ? ((uint32_t)((lx << b.sby) + ly) * ((1u << sf) + 1u) + (uint32_t)p)
+                                     : (uint32_t)lx * ((1u << sf) + 1u) + (uint32_t)((p << b.sby) + ly);
+        if constexpr (D == 3) {
+            const Off oz = planes.own[p + 1];
+            d.own = own_xy + oz;
+            d.z[0] = planes.own[p] - oz;
+            d.z[2] = planes.own[p + 2] - oz;
+        } else {
+            d.own = own_xy + row_deltas(y);
+        }
+        float u[3] = {0.f, 0.f, 0.f};
+        if (a.u) static_for<0, D>([&](auto dc) { u[dc.value] = field[dc.value][slot]; });
+        float uu = 0.f;
+        static_for<0, D>([&](auto dc) { uu += u[dc.value] * u[dc.value]; });
+        float S_[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        if (a.grad)
+            static_for<0, NS>([&](auto nc) {
+                constexpr int n = nc.value, A = sa<L>(n), B = sb<L>(n);
+                S_[A][B] = S_[B][A] = field[D + n][slot];
+            });
+        auto population = [&](auto qc) -> float {
+            constexpr int q = decltype(qc)::value;
+            float fi = feq<L, q>(a.rho, u, uu, a.ddf != 0);
+            if (a.grad) {
+                float neq = 0.f;
+                static_for<0, D>([&](auto ac) {
+                    static_for<0, D>([&](auto bc) {
+                        constexpr int A = ac.value, B = bc.value;
+                        constexpr float Qab = (float)(L::c(q, A) * L::c(q, B)) - (A == B ? (float)(1.0 / 3.0) : 0.f);
+                        neq += Qab * S_[A][B];
+                    });
+                });
+                neq *= (-wf<L>(q) * a.rho * a.tau * 3.f) * ((a.tau - 1.f) / a.tau);
+                fi += neq;
+            }
+            return fi;
+        };
+        if (!a.esoteric) {
+            static_for<0, Q>([&](auto qc) { P::st(fs + (d.own + oT * qc.value), population(qc)); });
+        } else {
+            P::st(fs + d.own, population(std::integral_constant<int, 0>{}));
+            static_for<1, Q - 1, 2>([&](auto qc) {
+                constexpr int pos = qc.value, neg = pos + 1;
+                P::st(fs + (d.template at<L::c(pos, 0), L::c(pos, 1), L::c(pos, 2)>() + oT * pos), population(qc));
+                P::st(fs + (d.own + oT * neg), population(std::integral_constant<int, neg>{}));
+            });
+        }
+    }
+}
+
+template <class L>
+cudaError_t launch_init(const InitArgs& a, bool f16, cudaStream_t s) {
+    const uint32_t blocks = a.brick.nbx * a.brick.nby * a.brick.nbz;
+    const bool narrow = (uint64_t)a.lay.ncells * L::Q < (1ull << 31);
+    if (f16) {
+        if (narrow) init_kernel<L, true, int32_t><<<blocks, kBrickThreads, 0, s>>>(a);
+        else init_kernel<L, true, int64_t><<<blocks, kBrickThreads, 0, s>>>(a);
+    } else {
+        if (narrow) init_kernel<L, false, int32_t><<<blocks, kBrickThreads, 0, s>>>(a);
+        else init_kernel<L, false, int64_t><<<blocks, kBrickThreads, 0, s>>>(a);
+    }
+    return cudaGetLastError();
 }
 
 // Launches the outputs of one lattice (lbm_fields_*.cu): rho and u, or with qcrit the Q-criterion.

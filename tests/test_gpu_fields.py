@@ -59,6 +59,24 @@ def test_outputs_at_brick_edges(lat, shape, tile, kind, meth, f16):
     q_ref = oracle.q_criterion(cfg, grid, 32, f0, bc, flags, u_ref, 0.7, True, fill=-7.0)
     assert np.array_equal(q.cpu().numpy().reshape(grid.shape), q_ref, equal_nan=True)
 
+@pytest.mark.parametrize("meth,f16,given", [("db", False, "u+grad"), ("eso", True, "u+grad"), ("eso", False, "grad"),
+                                            ("db", True, "u"), ("db", False, "rest")])
+@pytest.mark.parametrize("lat,shape,tile", GRIDS)
+def test_init_at_brick_edges(lat, shape, tile, meth, f16, given):
+    grid = make_grid(lat, shape, tile)
+    m = LBM_method.DOUBLE_BUFFER if meth == "db" else LBM_method.ESOTERIC_PULL
+    cfg = LBM_Config(m, DDF_shift=f16, use_float16c=f16)
+    rng = np.random.default_rng(grid.num_points)
+    u = rng.normal(0, 0.03, (grid.D,) + grid.shape).astype(np.float32) if "u" in given else None
+    g = rng.normal(0, 1e-3, (grid.D * grid.D,) + grid.shape).astype(np.float32) if "grad" in given else None
+    ref = np.zeros(grid.num_points * grid.Q, oracle.f_dtype(cfg, 32))
+    oracle.init(cfg, grid, 32, ref, 1.01, 0.7, u, g)
+    fd = torch.zeros(ref.size, dtype=torch.int16 if f16 else torch.float32, device="cuda")
+    dev = lambda a: None if a is None else torch.from_numpy(a).cuda()  # noqa: E731
+    Solver(grid, cfg).init_equilibrium(fd, 1.01, 0.7, dev(u), dev(g))
+    assert np.array_equal(fd.cpu().numpy().view(ref.dtype), ref)
+
+
 @pytest.mark.parametrize("scale", ["flow", "tiny", "huge", "mixed"])
 @pytest.mark.parametrize("lat,meth,ddf", [("D2Q9", "db", False), ("D3Q19", "db", True), ("D3Q27", "eso", True)])
 def test_mass_momentum_sums(lat, meth, ddf, scale):
