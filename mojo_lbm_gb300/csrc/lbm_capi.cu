@@ -919,6 +919,46 @@ __global__ void f16c_decode_kernel(const uint16_t* in, float* out, int64_t n) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = f16c_decode(in[i]);
 }
+
+// The codec over whole 16-byte words of both arrays (eight codes, two float4), two words of codes per
+// thread; n is a multiple of 8 and both arrays are 16-byte aligned.  HBM-bound at 6 bytes a value; one
+// value per thread moved 2-byte words and ran 319 M values (a 256^3 D3Q19 lattice, floor 282 us) in
+// 795 us, these words 286 us.
+constexpr int64_t kCodecWords = 512;  // words of 8 codes per block of 256 threads
+__global__ void __launch_bounds__(256) f16c_decode_words_kernel(const uint4* __restrict__ in, float4* __restrict__ out,
+                                                                int64_t words) {
+    const int64_t w0 = (int64_t)blockIdx.x * kCodecWords + threadIdx.x;
+    uint4 c[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (w0 + 256 * k < words) c[k] = __ldg(in + w0 + 256 * k);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int64_t w = w0 + 256 * k;
+        if (w >= words) break;
+        auto lo = [](uint32_t v) { return f16c_decode_sx((int32_t)(v << 16) >> 16); };
+        auto hi = [](uint32_t v) { return f16c_decode_sx((int32_t)v >> 16); };
+        out[2 * w] = make_float4(lo(c[k].x), hi(c[k].x), lo(c[k].y), hi(c[k].y));
+        out[2 * w + 1] = make_float4(lo(c[k].z), hi(c[k].z), lo(c[k].w), hi(c[k].w));
+    }
+}
+__global__ void __launch_bounds__(256) f16c_encode_words_kernel(const float4* __restrict__ in, uint4* __restrict__ out,
+                                                                int64_t words) {
+    const int64_t w0 = (int64_t)blockIdx.x * kCodecWords + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int64_t w = w0 + 256 * k;
+        if (w >= words) break;
+        const float4 a = __ldg(in + 2 * w), b = __ldg(in + 2 * w + 1);
+        auto two = [](float l, float h) { return __byte_perm(f16c_encode(l), f16c_encode(h), 0x5410); };
+        out[w] = make_uint4(two(a.x, a.y), two(a.z, a.w), two(b.x, b.y), two(b.z, b.w));
+    }
+}
+
+// Codes handled as whole words: all but the last n % 8, when both arrays are 16-byte aligned.
+int64_t codec_words(const void* a, const void* b, int64_t n) {
+    return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15u) == 0u ? n / 8 : 0;
+}
 }  // namespace
 
 extern "C" {
@@ -926,7 +966,13 @@ extern "C" {
 lbm_status lbm_float16c_encode(const float* in, uint16_t* out, int64_t n, void* stream) {
     if (n < 0 || (n > 0 && (!in || !out))) return fail(LBM_EINVAL, "bad codec arguments");
     if (n == 0) return LBM_OK;
-    f16c_encode_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(in, out, n);
+    cudaStream_t s = (cudaStream_t)stream;
+    const int64_t words = codec_words(in, out, n), done = 8 * words;
+    if (words > 0)
+        f16c_encode_words_kernel<<<(unsigned)((words + kCodecWords - 1) / kCodecWords), 256, 0, s>>>(
+            reinterpret_cast<const float4*>(in), reinterpret_cast<uint4*>(out), words);
+    LBM_CK(cudaGetLastError());
+    if (done < n) f16c_encode_kernel<<<(unsigned)((n - done + 255) / 256), 256, 0, s>>>(in + done, out + done, n - done);
     LBM_CK(cudaGetLastError());
     return LBM_OK;
 }
@@ -934,7 +980,13 @@ lbm_status lbm_float16c_encode(const float* in, uint16_t* out, int64_t n, void* 
 lbm_status lbm_float16c_decode(const uint16_t* in, float* out, int64_t n, void* stream) {
     if (n < 0 || (n > 0 && (!in || !out))) return fail(LBM_EINVAL, "bad codec arguments");
     if (n == 0) return LBM_OK;
-    f16c_decode_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(in, out, n);
+    cudaStream_t s = (cudaStream_t)stream;
+    const int64_t words = codec_words(in, out, n), done = 8 * words;
+    if (words > 0)
+        f16c_decode_words_kernel<<<(unsigned)((words + kCodecWords - 1) / kCodecWords), 256, 0, s>>>(
+            reinterpret_cast<const uint4*>(in), reinterpret_cast<float4*>(out), words);
+    LBM_CK(cudaGetLastError());
+    if (done < n) f16c_decode_kernel<<<(unsigned)((n - done + 255) / 256), 256, 0, s>>>(in + done, out + done, n - done);
     LBM_CK(cudaGetLastError());
     return LBM_OK;
 }

@@ -2,7 +2,7 @@
 for bit, at the sizes where their bricks of 32 lanes x 32 planes have remainders: extents around a
 brick's along every axis, tile rows shorter and longer than a warp, the untiled layout, and domains
 with walls, mixed flags or none (a brick without any flag takes the form that gathers none); the
-mass and momentum sums."""
+Float16C codec over arrays, and the mass and momentum sums."""
 from __future__ import annotations
 
 import numpy as np
@@ -10,7 +10,7 @@ import pytest
 import torch
 
 import oracle
-from mojo_lbm_gb300 import Flags, LBM_Config, LBM_method
+from mojo_lbm_gb300 import Flags, LBM_Config, LBM_method, _capi
 from mojo_lbm_gb300.solver import Solver
 from tests.lbm_cases import initial_f, make_grid, mixed_flags
 from tests.test_gpu_step import to_dev
@@ -59,6 +59,7 @@ def test_outputs_at_brick_edges(lat, shape, tile, kind, meth, f16):
     q_ref = oracle.q_criterion(cfg, grid, 32, f0, bc, flags, u_ref, 0.7, True, fill=-7.0)
     assert np.array_equal(q.cpu().numpy().reshape(grid.shape), q_ref, equal_nan=True)
 
+
 @pytest.mark.parametrize("meth,f16,given", [("db", False, "u+grad"), ("eso", True, "u+grad"), ("eso", False, "grad"),
                                             ("db", True, "u"), ("db", False, "rest")])
 @pytest.mark.parametrize("lat,shape,tile", GRIDS)
@@ -75,6 +76,26 @@ def test_init_at_brick_edges(lat, shape, tile, meth, f16, given):
     dev = lambda a: None if a is None else torch.from_numpy(a).cuda()  # noqa: E731
     Solver(grid, cfg).init_equilibrium(fd, 1.01, 0.7, dev(u), dev(g))
     assert np.array_equal(fd.cpu().numpy().view(ref.dtype), ref)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 4096, 4096 * 3 + 5])
+@pytest.mark.parametrize("shift", [0, 1, 8])
+def test_codec_words_and_remainders(n, shift):
+    """The codec by whole 16-byte words, its remainder and arrays that are not 16-byte aligned."""
+    rng = np.random.default_rng(n)
+    x = np.concatenate([rng.normal(0, 1, n), rng.normal(0, 1e-6, n)]).astype(np.float32)[rng.permutation(2 * n)[:n]]
+    want = oracle.f16c_encode(x)
+    src = torch.zeros(n + shift, device="cuda")[shift:]
+    src.copy_(torch.from_numpy(x))
+    out = torch.zeros(n + shift + 1, dtype=torch.int16, device="cuda")
+    code = out[shift:shift + n]
+    _capi.check(_capi.lib().lbm_float16c_encode(src.data_ptr(), code.data_ptr(), n, None))
+    assert np.array_equal(code.cpu().numpy().view(np.uint16), want)
+    assert int(out[shift + n]) == 0  # nothing past the end
+    back = torch.zeros(n + shift + 1, device="cuda")
+    _capi.check(_capi.lib().lbm_float16c_decode(code.data_ptr(), back[shift:].data_ptr(), n, None))
+    assert np.array_equal(back[shift:shift + n].cpu().numpy().view(np.uint32), oracle.f16c_decode(want).view(np.uint32))
+    assert float(back[shift + n]) == 0.0
 
 
 @pytest.mark.parametrize("scale", ["flow", "tiny", "huge", "mixed"])
