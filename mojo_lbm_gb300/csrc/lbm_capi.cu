@@ -83,6 +83,64 @@ __global__ void __launch_bounds__(256) cell_mask_kernel(const StepArgs a, uint2*
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) tile_cell_masks<L>(a, tile, masks);
 }
 
+// The generic kernel's masks (any tile): bit (n / 32) % 8 of near[n / 256] and the neighbour-solid masks
+// of the cells of such warps, from flags and flags_seen.  Both start as those of a domain whose
+// flags are all 0.
+// flags_check_kernel compares the flags with flags_seen, 16 bytes a thread (byte by byte when the flags
+// are not 16-byte aligned), takes over what differs and sets *changed = gen.
+__global__ void __launch_bounds__(256) flags_check_kernel(const uint8_t* __restrict__ flags, uint8_t* __restrict__ seen,
+                                                          uint32_t ncells, uint32_t* changed, uint32_t gen) {
+    const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * 16u;
+    if (i >= ncells) return;
+    bool differ = false;
+    if ((reinterpret_cast<uintptr_t>(flags) & 15u) == 0u && i + 16u <= ncells) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(flags + i));
+        uint4* sp = reinterpret_cast<uint4*>(seen + i);
+        const uint4 o = *sp;
+        differ = w.x != o.x || w.y != o.y || w.z != o.z || w.w != o.w;
+        if (differ) *sp = w;
+    } else {
+        for (uint32_t k = 0; k < 16u && i + k < ncells; ++k) {
+            const uint8_t w = __ldg(flags + i + k);
+            if (w != seen[i + k]) {
+                seen[i + k] = w;
+                differ = true;
+            }
+        }
+    }
+    if (differ) *changed = gen;
+}
+
+// Rebuilds the masks after a change of the flags in this round (*changed == gen): one thread per cell,
+// blocks striding over the 256-cell chunks.
+template <class L>
+__global__ void __launch_bounds__(256) any_mask_kernel(const uint8_t* __restrict__ flags, const LayoutDesc l,
+                                                       uint8_t* __restrict__ near, uint2* __restrict__ masks,
+                                                       const uint32_t* changed, uint32_t gen) {
+    if (*changed != gen) return;  // the same value for every thread
+    __shared__ uint32_t bits;
+    const uint32_t chunks = l.ncells / 256u + (l.ncells % 256u != 0u);
+    for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
+        if (threadIdx.x == 0) bits = 0u;
+        __syncthreads();
+        const uint32_t n = chunk * 256u + threadIdx.x;
+        const bool in = threadIdx.x < l.ncells - chunk * 256u;
+        uint32_t any = 0u;
+        uint2 m = make_uint2(0u, 0u);
+        if (in) {
+            any = __ldg(flags + n);
+            Nbr nb;
+            AnyCell<L, int64_t>(l, n).nbr(l, nb);
+            m = any_solid_masks<L>(flags, l, nb, any);
+        }
+        const bool warp_any = __any_sync(0xffffffffu, any != 0u);
+        if (warp_any && in) masks[n] = m;
+        if (warp_any && (threadIdx.x & 31u) == 0u) atomicOr(&bits, 1u << (threadIdx.x >> 5));
+        __syncthreads();
+        if (threadIdx.x == 0) near[chunk] = (uint8_t)bits;
+    }
+}
+
 thread_local std::string g_err;
 
 lbm_status fail(lbm_status s, const std::string& msg) {
@@ -216,6 +274,11 @@ StepArgs step_args(const lbm_handle* h, const void* f_in, void* f_out, float* bc
     return a;
 }
 
+// Threads per block of the generic kernel unless the caller sets them: a block keeps its registers until
+// its slowest warp, one next to a wall, is done, and smaller blocks free them sooner (150 x 131 x 97
+// untiled float32 D3Q19 cavity: 84.0 us a step at 256 threads, 73.8 at 128, 72.5 at 64, 72.4 at 32).
+constexpr int kAnyThreads = 64;
+
 bool use_tile(const lbm_handle* h) { return h->step_tile != nullptr && h->path != 1; }
 
 // Two waves of the cell-pair kernel's CTAs (8 per SM) on the 152 SMs of a GB300.
@@ -276,6 +339,30 @@ lbm_status tile_summary(lbm_handle* h, const uint8_t* flags, cudaStream_t s) {
     return LBM_OK;
 }
 
+// The same for the generic kernel's masks (a handle without them gathers the neighbours' flags in every
+// step).
+lbm_status any_summary(lbm_handle* h, const uint8_t* flags, cudaStream_t s) {
+    if (!h->tile_near) return LBM_OK;
+    if (++h->summary_gen == 0u) ++h->summary_gen;  // 0 is the initial value of *changed
+    const uint32_t gen = h->summary_gen, n = h->lay.ncells;
+    flags_check_kernel<<<(uint32_t)(((uint64_t)n + 4095u) / 4096u), 256, 0, s>>>(flags, h->flags_seen, n, h->changed, gen);
+    LBM_CK(cudaGetLastError());
+    const uint32_t chunks = (uint32_t)(((uint64_t)n + 255u) / 256u), grid = std::min<uint32_t>(chunks, (uint32_t)h->sm_count * 8u);
+    uint2* masks = h->cell_masks;
+    switch (h->grid.lattice) {
+        case LBM_D2Q9: any_mask_kernel<D2Q9><<<grid, 256, 0, s>>>(flags, h->lay, h->tile_near, masks, h->changed, gen); break;
+        case LBM_D3Q19: any_mask_kernel<D3Q19><<<grid, 256, 0, s>>>(flags, h->lay, h->tile_near, masks, h->changed, gen); break;
+        default: any_mask_kernel<D3Q27><<<grid, 256, 0, s>>>(flags, h->lay, h->tile_near, masks, h->changed, gen); break;
+    }
+    LBM_CK(cudaGetLastError());
+    return LBM_OK;
+}
+
+// Brings the masks of the kernel that will step up to date with `flags`.
+lbm_status summary(lbm_handle* h, const uint8_t* flags, cudaStream_t s) {
+    return h->step_tile ? tile_summary(h, flags, s) : any_summary(h, flags, s);
+}
+
 lbm_status check_handle(const lbm_handle* h) {
     if (!h) return fail(LBM_EINVAL, "null handle");
     return LBM_OK;
@@ -286,11 +373,9 @@ lbm_status check_handle(const lbm_handle* h) {
 lbm_status step_once(lbm_handle* h, const void* f_in, void* f_out, float* bc, const uint8_t* flags, float tau,
                      int even, cudaStream_t s, bool with_summary = true) {
     const StepArgs a = step_args(h, f_in, f_out, bc, flags, tau, even);
-    if (use_tile(h)) {
-        if (with_summary) {
-            const lbm_status st = tile_summary(h, flags, s);
-            if (st != LBM_OK) return st;
-        }
+    if (with_summary) {
+        const lbm_status st = summary(h, flags, s);
+        if (st != LBM_OK) return st;
     }
     LBM_CK(step_fn(h, a)(a, h->threads, s));
     return LBM_OK;
@@ -447,7 +532,7 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
     h->summary_gen = 0;
     h->summary_valid = 0;
     h->tile_near = nullptr;
-    h->threads = 256;
+    h->threads = kAnyThreads;
     h->scratch = nullptr;
     h->closure = nullptr;
     std::memset(&h->closure_uniform, 0, sizeof(h->closure_uniform));
@@ -475,6 +560,32 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
     if (e == cudaSuccess && !segs.empty()) e = cudaMalloc(&h->stage_segs, sizeof(StageSeg) * segs.size());
     if (e == cudaSuccess && !segs.empty())
         e = cudaMemcpy(h->stage_segs, segs.data(), sizeof(StageSeg) * segs.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !h->step_tile) {
+        // the generic kernel's masks, 9 bytes per cell: without the memory for them every step gathers
+        // the neighbours' flags instead
+        const size_t n = h->lay.ncells, chunks = (n + 255u) / 256u;
+        cudaError_t m = cudaMalloc(&h->flags_seen, n);
+        if (m == cudaSuccess) m = cudaMalloc(&h->cell_masks, sizeof(uint2) * n);
+        if (m == cudaSuccess) m = cudaMalloc(&h->changed, sizeof(uint32_t));
+        if (m == cudaSuccess) m = cudaMalloc(&h->tile_near, chunks);
+        if (m == cudaSuccess) {
+            e = cudaMemset(h->flags_seen, 0, n);
+            if (e == cudaSuccess) e = cudaMemset(h->changed, 0, sizeof(uint32_t));
+            if (e == cudaSuccess) e = cudaMemset(h->tile_near, 0, chunks);
+        } else if (m == cudaErrorMemoryAllocation) {
+            cudaGetLastError();  // cleared: the handle works without
+            cudaFree(h->flags_seen);
+            cudaFree(h->cell_masks);
+            cudaFree(h->changed);
+            cudaFree(h->tile_near);
+            h->flags_seen = nullptr;
+            h->cell_masks = nullptr;
+            h->changed = nullptr;
+            h->tile_near = nullptr;
+        } else {
+            e = m;
+        }
+    }
     if (e != cudaSuccess) {
         lbm_destroy(h);
         return fail(LBM_ECUDA, std::string("lbm_create: ") + cudaGetErrorString(e));
@@ -588,7 +699,7 @@ lbm_status lbm_set_closure(lbm_handle* h, const lbm_closure_t* closure) {
 
 lbm_status lbm_set_block_threads(lbm_handle* h, int32_t threads) {
     if (check_handle(h)) return LBM_EINVAL;
-    if (threads == 0) threads = 256;
+    if (threads == 0) threads = kAnyThreads;
     if (threads < 32 || threads > 256 || threads % 32)
         return fail(LBM_EINVAL, "threads per block must be a multiple of 32 in [32, 256]");
     h->threads = threads;
@@ -676,10 +787,8 @@ lbm_status lbm_run(lbm_handle* h, void* f_a, void* f_b, float* bc, const uint8_t
         return fail(LBM_EINVAL, "bc is required by this configuration");
     cudaStream_t s = (cudaStream_t)stream;
     if (n_steps == 0) return LBM_OK;
-    if (use_tile(h)) {
-        const lbm_status st = tile_summary(h, flags, s);
-        if (st != LBM_OK) return st;
-    }
+    const lbm_status sum = summary(h, flags, s);
+    if (sum != LBM_OK) return sum;
     auto launch_k = [&](int64_t k) -> lbm_status {
         const bool a_is_src = ((first_step + k) % 2) == 0;
         if (eso) return step_once(h, f_a, f_a, bc, flags, tau, a_is_src ? 1 : 0, s, false);

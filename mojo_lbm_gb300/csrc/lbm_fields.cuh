@@ -119,30 +119,6 @@ __device__ __forceinline__ Cell locate_cell(const LayoutDesc& l, const Brick& b,
     return c;
 }
 
-// Element deltas along one axis for shifts -1, 0, +1 (periodic): `l` of `t` cells into tile `b` of
-// `nt`, with in-tile stride ls and tile stride ts (both in population elements).
-template <class Off>
-__device__ __forceinline__ void axis_deltas(uint32_t l, uint32_t t, uint32_t b, uint32_t nt, Off ls, Off ts, Off (&d)[3]) {
-    d[1] = 0;
-    d[0] = l > 0u ? -ls : (Off)(t - 1u) * ls + (b > 0u ? -ts : (Off)(nt - 1u) * ts);
-    d[2] = l + 1u < t ? ls : -(Off)(t - 1u) * ls + (b + 1u < nt ? ts : -(Off)(nt - 1u) * ts);
-}
-
-// Population offsets of a cell and its neighbours.  Off: int32_t when the lattice has fewer than
-// 2^31 elements (one three-input add and one wide multiply-add per load), else int64_t.
-template <class Off>
-struct CellDeltas {
-    Off own, x[3], y[3], z[3];
-    template <int SX, int SY, int SZ>
-    __device__ __forceinline__ Off at() const {
-        Off o = own;
-        if constexpr (SY != 0) o += y[SY + 1];
-        if constexpr (SZ != 0) o += z[SZ + 1];
-        if constexpr (SX != 0) o += x[SX + 1];
-        return o;
-    }
-};
-
 // Per plane of a 3D brick and its rim (index 0: the plane below the brick): the plane's part of a
 // cell's flag index and of its population offset (periodic; planes past the neighbour of the grid's
 // last one are nobody's neighbour and repeat it).

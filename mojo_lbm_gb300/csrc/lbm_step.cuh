@@ -34,8 +34,8 @@ struct StepArgs {
     // block-per-tile path (256-cell tiles with power-of-two sides)
     const ClosureDev* closure; // learned LES closure's fragments (learned-closure kernels only)
     ClosureUniform cl;         // and its warp-uniform part
-    const uint8_t* tile_near;  // per tile: bit w set if a cell of warp w or a cell it pulls from
-                               // holds a flag other than plain FLUID (warp_near)
+    const uint8_t* tile_near;  // per tile (generic kernel: per 256 cells): bit w set if a cell of
+                               // warp w or a cell it pulls from holds a flag other than plain FLUID
     const uint2* cell_masks;   // per cell of such a warp: (raw_solid, nib_solid), cell_solid_masks
     uint32_t mx, my, shx, shxy; // lx = t & mx, ly = (t >> shx) & my, lz = t >> shxy
     // interpolated bounce-back fused into the step (block-per-tile kernels, double buffer): per
@@ -114,6 +114,30 @@ struct Nbr {
     __device__ __forceinline__ uint32_t loc() const { return ax.loc[SX + 1] + ay.loc[SY + 1] + az.loc[SZ + 1]; }
     template <int SX, int SY, int SZ>
     __device__ __forceinline__ uint32_t til() const { return ax.til[SX + 1] + ay.til[SY + 1] + az.til[SZ + 1]; }
+};
+
+// Element deltas along one axis for shifts -1, 0, +1 (periodic): `l` of `t` cells into tile `b` of
+// `nt`, with in-tile stride ls and tile stride ts (both in population elements).
+template <class Off>
+__device__ __forceinline__ void axis_deltas(uint32_t l, uint32_t t, uint32_t b, uint32_t nt, Off ls, Off ts, Off (&d)[3]) {
+    d[1] = 0;
+    d[0] = l > 0u ? -ls : (Off)(t - 1u) * ls + (b > 0u ? -ts : (Off)(nt - 1u) * ts);
+    d[2] = l + 1u < t ? ls : -(Off)(t - 1u) * ls + (b + 1u < nt ? ts : -(Off)(nt - 1u) * ts);
+}
+
+// Population offsets of a cell and its neighbours.  Off: int32_t when the lattice has fewer than
+// 2^31 elements (one three-input add and one wide multiply-add per load), else int64_t.
+template <class Off>
+struct CellDeltas {
+    Off own, x[3], y[3], z[3];
+    template <int SX, int SY, int SZ>
+    __device__ __forceinline__ Off at() const {
+        Off o = own;
+        if constexpr (SY != 0) o += y[SY + 1];
+        if constexpr (SZ != 0) o += z[SZ + 1];
+        if constexpr (SX != 0) o += x[SX + 1];
+        return o;
+    }
 };
 
 template <class L>
@@ -543,123 +567,210 @@ __device__ __forceinline__ void equilibrium_bc(float (&f)[L::Q], const float* bc
     for_each_feq<L>(rs, us, uu, ddf, [&](auto qc, float e) { f[decltype(qc)::value] = e; });
 }
 
-template <class L, int METHOD, bool F16C, int COLL, int LES>
-__global__ void __launch_bounds__(256) step_kernel(const StepArgs a) {
+// Programmatic dependent launch of the step kernels (launch_pdl): wait until the previous grid in
+// the stream has completed and its writes are visible, then let the next grid (the next step) be
+// scheduled onto the SMs while this one runs, so that its launch latency overlaps this step.  The
+// wait comes before any access to the populations, flags or masks; both instructions are no-ops
+// for a grid launched without the attribute.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches a step kernel with programmatic stream serialization allowed (see pdl_enter).
+template <class Kernel>
+cudaError_t launch_pdl(Kernel kernel, uint32_t grid, uint32_t block, cudaStream_t s, const StepArgs& a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+// Position of cell n of any layout, and its population offsets.
+template <class L, class Off>
+struct AnyCell {
+    uint32_t loc, tile, lx, ly, lz, bx, by, bz;
+    CellDeltas<Off> d;
+    __device__ __forceinline__ AnyCell(const LayoutDesc& l, uint32_t n) {
+        constexpr int D = L::D;
+        tile = l.d_T.div(n);
+        loc = n - tile * l.T;
+        const uint32_t lyz = l.d_tx.div(loc);
+        lx = loc - lyz * (uint32_t)l.tx;
+        lz = D == 3 ? l.d_ty.div(lyz) : 0u;
+        ly = lyz - lz * (uint32_t)l.ty;
+        const uint32_t byz = l.d_ntx.div(tile);
+        bx = tile - byz * (uint32_t)l.ntx;
+        bz = D == 3 ? l.d_nty.div(byz) : 0u;
+        by = byz - bz * (uint32_t)l.nty;
+        const Off TQ = (Off)l.T * L::Q;
+        d.own = (Off)loc + TQ * (Off)tile;
+        axis_deltas<Off>(lx, (uint32_t)l.tx, bx, (uint32_t)l.ntx, 1, TQ, d.x);
+        axis_deltas<Off>(ly, (uint32_t)l.ty, by, (uint32_t)l.nty, (Off)l.tx, TQ * (Off)l.ntx, d.y);
+        if constexpr (D == 3)
+            axis_deltas<Off>(lz, (uint32_t)l.tz, bz, (uint32_t)l.ntz, (Off)l.tx * (Off)l.ty,
+                             TQ * (Off)l.ntx * (Off)l.nty, d.z);
+    }
+    // neighbour tables (flag and bc indices), for the cells next to a flag
+    __device__ __forceinline__ void nbr(const LayoutDesc& l, Nbr& nb) const {
+        nb.ax.init(lx, bx, l.tx, l.ntx, 1u, 1u);
+        nb.ay.init(ly, by, l.ty, l.nty, (uint32_t)l.tx, (uint32_t)l.ntx);
+        if constexpr (L::D == 3)
+            nb.az.init(lz, bz, l.tz, l.ntz, (uint32_t)(l.tx * l.ty), (uint32_t)(l.ntx * l.nty));
+        else { nb.az.loc[0] = nb.az.loc[1] = nb.az.loc[2] = 0u; nb.az.til[0] = nb.az.til[1] = nb.az.til[2] = 0u; }
+    }
+};
+
+// set_adjacent_flags (ops/load_and_store.mojo:270-291) of a cell of any layout: bit q of .x when the
+// flag at x - c_q is SOLID (raw compare), of .y when its enum nibble is; any: an own or neighbouring
+// flag is not 0.
+template <class L>
+__device__ __forceinline__ uint2 any_solid_masks(const uint8_t* __restrict__ flags, const LayoutDesc& l, const Nbr& nb,
+                                                 uint32_t& any) {
+    uint32_t raw_solid = 0u, nib_solid = 0u;
+    static_for<1, L::Q>([&](auto qc) {
+        constexpr int q = qc.value;
+        constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
+        const uint8_t pf = __ldg(flags + (nb.template loc<sx, sy, sz>() + l.T * nb.template til<sx, sy, sz>()));
+        any |= pf;
+        if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
+        if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
+    });
+    return make_uint2(raw_solid, nib_solid);
+}
+
+// The per-thread body of the generic kernel (any tile, any size).  As in tile_cell below, GENERAL =
+// false is the form of a warp whose cells and pull neighbours are all plain FLUID; GENERAL = true
+// reads the flags and takes the neighbour masks built when they last changed (a.cell_masks), or
+// gathers the neighbours' flags when the handle holds no masks.
+template <class L, int METHOD, bool F16C, int COLL, int LES, class Off, bool GENERAL>
+__device__ __forceinline__ void any_cell(const StepArgs& a, const uint32_t n) {
     using P = Pop<F16C>;
     using S = typename P::T;
     constexpr int Q = L::Q, D = L::D, K = D + 1;
     constexpr bool ESO = METHOD == LBM_ESOTERIC_PULL;
-
-    static_assert(LES != kLesLearned, "the learned closure runs in the block-per-tile kernel");
-    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= a.lay.ncells) return;
-    const uint8_t flag = __ldg(a.flags + n);
-    // is_valid_thread (src/lbm/kernels/utils/checks.mojo:55-60)
-    if ((flag & 0x0F) == LBM_FLAG_SOLID || (flag & LBM_FLAG_EXCLUDE)) return;
-
+    uint8_t flag = 0;
+    if constexpr (GENERAL) {
+        flag = __ldg(a.flags + n);
+        // is_valid_thread (src/lbm/kernels/utils/checks.mojo:55-60)
+        if ((flag & 0x0F) == LBM_FLAG_SOLID || (flag & LBM_FLAG_EXCLUDE)) return;
+    }
+    const AnyCell<L, Off> c(a.lay, n);
     const uint32_t T = a.lay.T;
-    const uint32_t tile = a.lay.d_T.div(n);
-    const uint32_t loc = n - tile * T;
-    const uint32_t lyz = a.lay.d_tx.div(loc);
-    const uint32_t lx = loc - lyz * (uint32_t)a.lay.tx;
-    const uint32_t lz = a.lay.d_ty.div(lyz);
-    const uint32_t ly = lyz - lz * (uint32_t)a.lay.ty;
-    const uint32_t byz = a.lay.d_ntx.div(tile);
-    const uint32_t bx = tile - byz * (uint32_t)a.lay.ntx;
-    const uint32_t bz = a.lay.d_nty.div(byz);
-    const uint32_t by = byz - bz * (uint32_t)a.lay.nty;
-
-    Nbr nb;
-    const uint32_t txy = (uint32_t)(a.lay.tx * a.lay.ty);
-    const uint32_t ntxy = (uint32_t)(a.lay.ntx * a.lay.nty);
-    nb.ax.init(lx, bx, a.lay.tx, a.lay.ntx, 1u, 1u);
-    nb.ay.init(ly, by, a.lay.ty, a.lay.nty, (uint32_t)a.lay.tx, (uint32_t)a.lay.ntx);
-    if constexpr (D == 3) nb.az.init(lz, bz, a.lay.tz, a.lay.ntz, txy, ntxy);
-    else { nb.az.loc[0] = nb.az.loc[1] = nb.az.loc[2] = 0u; nb.az.til[0] = nb.az.til[1] = nb.az.til[2] = 0u; }
-
-    const uint64_t TQ = (uint64_t)T * Q;
+    const Off oT = (Off)T;
     const S* fin = (const S*)a.f_in;
     S* fout = (S*)a.f_out;
-    const uint64_t own = loc + TQ * tile;
 
-    // ---- stream.  The pull loads are issued first and do not wait for the neighbour flags; the
-    // few populations whose pull neighbour is SOLID are re-loaded afterwards from the cell's own
-    // opposite slot (mid-grid bounce-back on a raw SOLID compare, ops/load_and_store.mojo:210-219,
-    // which also loads the pull value first).
+    // ---- stream (pull loads first, independent of the flags)
     float f[Q];
     if constexpr (!ESO) {
         static_for<0, Q>([&](auto qc) {
             constexpr int q = qc.value;
-            constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
-            f[q] = P::ld(fin + nb.template loc<sx, sy, sz>() + TQ * nb.template til<sx, sy, sz>() + (uint64_t)T * q);
+            f[q] = P::ld(fin + (c.d.template at<-L::c(q, 0), -L::c(q, 1), -L::c(q, 2)>() + oT * q));
         });
     } else {
+        // slot pos + 1 = neg: the parity folds into two base pointers
         const bool ev = a.even != 0;
-        f[0] = P::ld_rw(fin + own);
+        const S* finA = fin + (ev ? 0u : T);
+        const S* finB = fin + (ev ? T : 0u);
+        f[0] = P::ld_rw(fin + c.d.own);
         static_for<1, Q - 1, 2>([&](auto qc) {
             constexpr int pos = qc.value, neg = pos + 1;
-            constexpr int sx = L::c(pos, 0), sy = L::c(pos, 1), sz = L::c(pos, 2);
-            const uint64_t nbase = nb.template loc<sx, sy, sz>() + TQ * nb.template til<sx, sy, sz>();
-            const uint32_t sA = ev ? pos : neg, sB = ev ? neg : pos;
-            f[pos] = P::ld_rw(fin + own + (uint64_t)T * sA);
-            f[neg] = P::ld_rw(fin + nbase + (uint64_t)T * sB);
+            f[pos] = P::ld_rw(finA + (c.d.own + oT * pos));
+            f[neg] = P::ld_rw(finB + (c.d.template at<L::c(pos, 0), L::c(pos, 1), L::c(pos, 2)>() + oT * pos));
         });
     }
 
-    // ---- neighbour flags at x - c_q (set_adjacent_flags, ops/load_and_store.mojo:270-291)
-    uint32_t raw_solid = 0u, nib_solid = 0u;
-    const bool need_flags = !ESO || a.moving;
-    if (need_flags) {
-        static_for<1, Q>([&](auto qc) {
-            constexpr int q = qc.value;
-            constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
-            const uint32_t m = nb.template loc<sx, sy, sz>() + T * nb.template til<sx, sy, sz>();
-            const uint8_t pf = __ldg(a.flags + m);
-            if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
-            if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
-        });
-    }
-    if constexpr (!ESO) {
-        if (raw_solid) {
-            static_for<1, Q>([&](auto qc) {
-                constexpr int q = qc.value;
-                if ((raw_solid >> q) & 1u) f[q] = P::ld(fin + own + (uint64_t)T * opp<L>(q));
+    if constexpr (GENERAL) {
+        uint32_t raw_solid = 0u, nib_solid = 0u;
+        if (!ESO || a.moving) {
+            uint2 m;
+            if (a.cell_masks) {
+                m = __ldg(a.cell_masks + n);
+            } else {
+                Nbr nb;
+                c.nbr(a.lay, nb);
+                uint32_t any = 0u;
+                m = any_solid_masks<L>(a.flags, a.lay, nb, any);
+            }
+            raw_solid = m.x;
+            nib_solid = m.y;
+        }
+        if constexpr (!ESO) {
+            // mid-grid bounce-back on a raw SOLID compare (ops/load_and_store.mojo:210-219)
+            if (raw_solid)
+                static_for<1, Q>([&](auto qc) {
+                    constexpr int q = qc.value;
+                    if ((raw_solid >> q) & 1u) f[q] = P::ld(fin + (c.d.own + oT * opp<L>(q)));
+                });
+        }
+        // boundary conditions (steps/apply_boundary_condition.mojo:10-41)
+        if (a.moving && nib_solid) {
+            Nbr nb;
+            c.nbr(a.lay, nb);
+            const uint64_t TK = (uint64_t)T * K;
+            moving_wall<L>(f, nib_solid, a.bc, T, [&](auto qc) -> uint64_t {
+                constexpr int q = decltype(qc)::value;
+                constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
+                return nb.template loc<sx, sy, sz>() + TK * nb.template til<sx, sy, sz>();
             });
         }
+        if (a.eqbc && (flag & 0x0F) == LBM_FLAG_EQUILIBRIUM)
+            equilibrium_bc<L>(f, a.bc, c.loc + (uint64_t)T * K * c.tile, T, (int32_t)(c.bx * a.lay.tx + c.lx),
+                              (int32_t)(c.by * a.lay.ty + c.ly), (int32_t)(c.bz * a.lay.tz + c.lz), a.lay, a.ddf != 0);
     }
 
-    // ---- boundary conditions (steps/apply_boundary_condition.mojo:10-41)
-    if (a.moving && nib_solid) {
-        const uint64_t TK = (uint64_t)T * K;
-        moving_wall<L>(f, nib_solid, a.bc, T, [&](auto qc) -> uint64_t {
-            constexpr int q = decltype(qc)::value;
-            constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
-            return nb.template loc<sx, sy, sz>() + TK * nb.template til<sx, sy, sz>();
-        });
-    }
-    const uint64_t own_bc = loc + (uint64_t)T * K * tile;
-    if (a.eqbc && (flag & 0x0F) == LBM_FLAG_EQUILIBRIUM)
-        equilibrium_bc<L>(f, a.bc, own_bc, T, (int32_t)(bx * a.lay.tx + lx), (int32_t)(by * a.lay.ty + ly),
-                          (int32_t)(bz * a.lay.tz + lz), a.lay, a.ddf != 0);
-
-    collide<L, COLL, LES>(f, a.tau, a, a.bc + own_bc, T, flag);
+    collide<L, COLL, LES>(f, a.tau, a, a.bc + (c.loc + (uint64_t)T * K * c.tile), T, flag);
 
     // ---- store
     if constexpr (!ESO) {
-        static_for<0, Q>([&](auto qc) { P::st(fout + own + (uint64_t)T * qc.value, f[qc.value]); });
+        static_for<0, Q>([&](auto qc) { P::st(fout + (c.d.own + oT * qc.value), f[qc.value]); });
     } else {
         // esoteric_pull_store_f_vec (ops/load_and_store.mojo:89-159): the same slots as loaded
         const bool ev = a.even != 0;
-        P::st(fout + own, f[0]);
+        S* foA = fout + (ev ? 0u : T);
+        S* foB = fout + (ev ? T : 0u);
+        P::st(fout + c.d.own, f[0]);
         static_for<1, Q - 1, 2>([&](auto qc) {
             constexpr int pos = qc.value, neg = pos + 1;
-            constexpr int sx = L::c(pos, 0), sy = L::c(pos, 1), sz = L::c(pos, 2);
-            const uint64_t nbase = nb.template loc<sx, sy, sz>() + TQ * nb.template til<sx, sy, sz>();
-            const uint32_t sA = ev ? pos : neg, sB = ev ? neg : pos;
-            P::st(fout + nbase + (uint64_t)T * sB, f[pos]);
-            P::st(fout + own + (uint64_t)T * sA, f[neg]);
+            P::st(foB + (c.d.template at<L::c(pos, 0), L::c(pos, 1), L::c(pos, 2)>() + oT * pos), f[pos]);
+            P::st(foA + (c.d.own + oT * pos), f[neg]);
         });
     }
+}
+
+// Resident blocks of 256 threads per SM the generic kernels are built for (64 registers; KBC and
+// D3Q27 80).  5 (48 registers) ran the cavity above in 83.1 us a step against 72.5, the periodic box in
+// 49.0 against 49.8.
+template <class L, int COLL>
+constexpr int any_min_blocks() { return COLL == LBM_KBC || L::Q == 27 ? 3 : 4; }
+
+// The generic kernel: one thread per cell in memory order, any tile and size.  A warp reads its bit of
+// a.tile_near (bit (n / 32) % 8 of byte n / 256: a cell of the warp or one it pulls from holds a flag
+// other than plain FLUID) and takes the form of any_cell without flags when it is clear; without masks
+// (a.tile_near null) every warp takes the general form.  Off: population offsets in 32 bits when the
+// lattice has fewer than 2^31 elements.
+// HBM-bound away from walls (150 x 131 x 97 untiled float32 D3Q19: floor 42.6 us a step, periodic box
+// 49.8 us); with 18 flag bytes gathered and 19 offsets formed in 64 bits in every cell it ran 148 us on
+// the cavity, with the masks and 32-bit offsets 72.5 us.  The difference to the periodic box is the
+// general form: 40 % of that grid's warps hold an end of an x row.
+template <class L, int METHOD, bool F16C, int COLL, int LES, class Off>
+__global__ void __launch_bounds__(256, (any_min_blocks<L, COLL>())) step_kernel(const StepArgs a) {
+    static_assert(LES != kLesLearned, "the learned closure runs in the block-per-tile kernel");
+    pdl_enter();
+    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    // (uniform over the warp: blocks are multiples of 32 threads)
+    const bool general = !a.tile_near || ((__ldg(a.tile_near + (n >> 8)) >> ((n >> 5) & 7u)) & 1u) != 0u;
+    if (n >= a.lay.ncells) return;
+    if (!general) any_cell<L, METHOD, F16C, COLL, LES, Off, false>(a, n);
+    else any_cell<L, METHOD, F16C, COLL, LES, Off, true>(a, n);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1168,32 +1279,6 @@ constexpr int tile_min_blocks() {
     else return (L::Q == 9) ? 5 : (heavy ? LBM_TILE_MIN_BLOCKS_HEAVY : LBM_TILE_MIN_BLOCKS);
 }
 
-// Programmatic dependent launch of the step kernels (launch_pdl): wait until the previous grid in
-// the stream has completed and its writes are visible, then let the next grid (the next step) be
-// scheduled onto the SMs while this one runs, so that its launch latency overlaps this step.  The
-// wait comes before any access to the populations, flags or masks; both instructions are no-ops
-// for a grid launched without the attribute.
-__device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-// Launches a step kernel with programmatic stream serialization allowed (see pdl_enter).
-template <class Kernel>
-cudaError_t launch_pdl(Kernel kernel, uint32_t grid, uint32_t block, cudaStream_t s, const StepArgs& a) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a);
-}
-
 template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST = false, bool LINKS = false>
 __global__ void __launch_bounds__(256, (tile_min_blocks<L, COLL, LINKS>()))
     step_kernel_tile(const StepArgs a) {
@@ -1239,8 +1324,9 @@ using StepLaunch = cudaError_t (*)(const StepArgs&, int threads, cudaStream_t);
 template <class L, int METHOD, bool F16C, int COLL, int LES>
 cudaError_t launch_step(const StepArgs& a, int threads, cudaStream_t s) {
     const uint32_t blocks = (a.lay.ncells + (uint32_t)threads - 1u) / (uint32_t)threads;
-    step_kernel<L, METHOD, F16C, COLL, LES><<<blocks, threads, 0, s>>>(a);
-    return cudaGetLastError();
+    if ((uint64_t)a.lay.ncells * L::Q < (1ull << 31))
+        return launch_pdl(step_kernel<L, METHOD, F16C, COLL, LES, int32_t>, blocks, (uint32_t)threads, s, a);
+    return launch_pdl(step_kernel<L, METHOD, F16C, COLL, LES, int64_t>, blocks, (uint32_t)threads, s, a);
 }
 
 template <class L, int METHOD, bool F16C, int COLL, int LES>
