@@ -128,10 +128,9 @@ __global__ void __launch_bounds__(256) any_mask_kernel(const uint8_t* __restrict
         uint32_t any = 0u;
         uint2 m = make_uint2(0u, 0u);
         if (in) {
-            any = __ldg(flags + n);
             Nbr nb;
             AnyCell<L, int64_t>(l, n).nbr(l, nb);
-            m = any_solid_masks<L>(flags, l, nb, any);
+            m = any_solid_masks<L>(flags, __ldg(flags + n), l, nb, any);
         }
         const bool warp_any = __any_sync(0xffffffffu, any != 0u);
         if (warp_any && in) masks[n] = m;
@@ -255,6 +254,7 @@ StepArgs step_args(const lbm_handle* h, const void* f_in, void* f_out, float* bc
     a.cl = h->closure_uniform;
     a.tile_near = h->tile_near;
     a.cell_masks = h->cell_masks;
+    a.masks_ready = 0;
     a.mx = h->mx;
     a.my = h->my;
     a.shx = h->shx;
@@ -369,10 +369,12 @@ lbm_status check_handle(const lbm_handle* h) {
 }
 
 // One step.  with_summary: rebuild the tile summary from `flags` first (single-step calls; a
-// multi-step run builds it once, since flags cannot change inside the run).
+// multi-step run builds it once, since flags cannot change inside the run).  masks_ready: the previous
+// kernel in the stream is a step of the same run.
 lbm_status step_once(lbm_handle* h, const void* f_in, void* f_out, float* bc, const uint8_t* flags, float tau,
-                     int even, cudaStream_t s, bool with_summary = true) {
-    const StepArgs a = step_args(h, f_in, f_out, bc, flags, tau, even);
+                     int even, cudaStream_t s, bool with_summary = true, bool masks_ready = false) {
+    StepArgs a = step_args(h, f_in, f_out, bc, flags, tau, even);
+    a.masks_ready = masks_ready ? 1 : 0;
     if (with_summary) {
         const lbm_status st = summary(h, flags, s);
         if (st != LBM_OK) return st;
@@ -791,9 +793,9 @@ lbm_status lbm_run(lbm_handle* h, void* f_a, void* f_b, float* bc, const uint8_t
     if (sum != LBM_OK) return sum;
     auto launch_k = [&](int64_t k) -> lbm_status {
         const bool a_is_src = ((first_step + k) % 2) == 0;
-        if (eso) return step_once(h, f_a, f_a, bc, flags, tau, a_is_src ? 1 : 0, s, false);
-        return a_is_src ? step_once(h, f_a, f_b, bc, flags, tau, 0, s, false)
-                        : step_once(h, f_b, f_a, bc, flags, tau, 0, s, false);
+        if (eso) return step_once(h, f_a, f_a, bc, flags, tau, a_is_src ? 1 : 0, s, false, k > 0);
+        return a_is_src ? step_once(h, f_a, f_b, bc, flags, tau, 0, s, false, k > 0)
+                        : step_once(h, f_b, f_a, bc, flags, tau, 0, s, false, k > 0);
     };
     // Chunks of an even number of steps keep the buffer/parity pattern of every replay identical.
     const int64_t chunk = 64;
@@ -809,9 +811,10 @@ lbm_status lbm_run(lbm_handle* h, void* f_a, void* f_b, float* bc, const uint8_t
             lbm_status st = LBM_OK;
             for (int64_t k = 0; k < chunk && st == LBM_OK; ++k) {
                 const bool a_is_src = ((first_step + k) % 2) == 0;
-                const StepArgs a = eso ? step_args(h, f_a, f_a, bc, flags, tau, a_is_src ? 1 : 0)
-                                       : (a_is_src ? step_args(h, f_a, f_b, bc, flags, tau, 0)
-                                                   : step_args(h, f_b, f_a, bc, flags, tau, 0));
+                StepArgs a = eso ? step_args(h, f_a, f_a, bc, flags, tau, a_is_src ? 1 : 0)
+                                 : (a_is_src ? step_args(h, f_a, f_b, bc, flags, tau, 0)
+                                             : step_args(h, f_b, f_a, bc, flags, tau, 0));
+                a.masks_ready = k > 0 ? 1 : 0;
                 const StepLaunch fn = step_fn(h, a);
                 if (fn(a, h->threads, h->capture_stream) != cudaSuccess) st = LBM_ECUDA;
             }

@@ -100,11 +100,11 @@ __device__ __forceinline__ void pair_deltas(const StepArgs& a, uint32_t bx, uint
 // The two cells of one thread.  GENERAL = false is the all-fluid form (the warp's two boxes hold
 // no flag and pull from no flagged cell): no flag is read, both cells are active and the code is
 // straight-line from the loads to the stores, so the scheduler interleaves the two collisions.
-// GENERAL = true reads the flags of the cells whose box bit is set and handles them as tile_step
-// does.
+// GENERAL = true takes the masks of both cells, m (x, y of A, z, w of B; 0 in a box without a flag), and
+// handles them as tile_step does.
 template <class L, bool F16C, int COLL, int LES, bool FAST, bool GENERAL>
 __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t tile, const uint32_t t,
-                                           const uint32_t mask, const uint32_t bx, const uint32_t by,
+                                           const uint4 m, const uint32_t bx, const uint32_t by,
                                            const uint32_t bz) {
     using P = Pop<F16C>;
     using S = typename P::T;
@@ -123,17 +123,15 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
 
     const uint32_t tA = 2u * t;         // cell A; B = tA + 1
     const uint32_t nA = tA + T * tile;  // flag offset of A
-    const bool flagged = GENERAL && ((mask >> (tA >> 5)) & 1u);  // the pair's box (both cells)
 
     uint8_t flagA = 0, flagB = 0;
     bool actA = true, actB = true;
-    if (flagged) {
-        flagA = __ldg(a.flags + nA);
-        flagB = __ldg(a.flags + nA + 1u);
-        // is_valid_thread (src/lbm/kernels/utils/checks.mojo:55-60), per cell
-        actA = !((flagA & 0x0F) == LBM_FLAG_SOLID || (flagA & LBM_FLAG_EXCLUDE));
-        actB = !((flagB & 0x0F) == LBM_FLAG_SOLID || (flagB & LBM_FLAG_EXCLUDE));
+    if constexpr (GENERAL) {
+        actA = (m.x & 1u) == 0u;
+        actB = (m.z & 1u) == 0u;
         if (!actA && !actB) return;
+        if (m.y & 1u) flagA = __ldg(a.flags + nA);
+        if (m.w & 1u) flagB = __ldg(a.flags + nA + 1u);
     }
 
     const uint32_t lxA = tA & a.mx, ly = (tA >> a.shx) & a.my, lz = tA >> a.shxy;
@@ -164,23 +162,26 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
         }
     });
 
-    if (flagged) {
-        // ---- cell-solid masks of both cells (written for every cell of a flagged box): x, z the
-        // SOLID pull neighbours of A, B; y, w those with a moving-wall bc.  Loaded after the pulls,
-        // whose latency they share.
-        const uint4 m = __ldg(reinterpret_cast<const uint4*>(a.cell_masks + nA));
-        // mid-grid bounce-back on a raw SOLID compare (ops/load_and_store.mojo:216)
-        if (m.x)
+    if constexpr (GENERAL) {
+        // mid-grid bounce-back on a raw SOLID compare (ops/load_and_store.mojo:216); selecting the
+        // address before the pull, as the per-cell kernels do, was slower here (393.3 against 389.8 us a
+        // step of the 256^3 float32 cavity, 269.9 against 262.1 in Float16C)
+        const uint32_t backA = m.x & ~1u, backB = m.z & ~1u;
+        if (backA)
             static_for<1, Q>([&](auto qc) {
                 constexpr int q = qc.value;
-                if ((m.x >> q) & 1u) fa[q] = ld(fin + own + (int32_t)(T * opp<L>(q)));
+                if ((backA >> q) & 1u) fa[q] = ld(fin + own + (int32_t)(T * opp<L>(q)));
             });
-        if (m.z)
+        if (backB)
             static_for<1, Q>([&](auto qc) {
                 constexpr int q = qc.value;
-                if ((m.z >> q) & 1u) fb[q] = ld(fin + own + 1 + (int32_t)(T * opp<L>(q)));
+                if ((backB >> q) & 1u) fb[q] = ld(fin + own + 1 + (int32_t)(T * opp<L>(q)));
             });
-        if (a.moving && (m.y | m.w)) {
+    }
+
+    if constexpr (GENERAL) {
+        const uint32_t wallA = m.y & ~1u, wallB = m.w & ~1u;
+        if (a.moving && (wallA | wallB)) {
             // moving_wall_bc with the bc of each cell's SOLID pull neighbours
             auto wall = [&](float (&f)[Q], uint32_t nib, uint32_t tc) {
                 int32_t dc[3][3], dp[3][3];
@@ -194,8 +195,8 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
                     return (uint64_t)(mm - mt * T) + (uint64_t)T * K * mt;
                 });
             };
-            if (m.y) wall(fa, m.y, tA);
-            if (m.w) wall(fb, m.w, tA + 1u);
+            if (wallA) wall(fa, wallA, tA);
+            if (wallB) wall(fb, wallB, tA + 1u);
         }
         if (a.eqbc) {
             const int32_t gx = (int32_t)(bx * (uint32_t)a.lay.tx + lxA), gy = (int32_t)(by * (uint32_t)a.lay.ty + ly),
@@ -243,20 +244,6 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
     }
 }
 
-template <class L, bool F16C, int COLL, int LES, bool FAST>
-__device__ __forceinline__ void pair_step(const StepArgs& a, const uint32_t tile, const uint32_t t) {
-    const uint32_t byz = a.lay.d_ntx.div(tile);
-    const uint32_t bx = tile - byz * (uint32_t)a.lay.ntx;
-    const uint32_t bz = a.lay.d_nty.div(byz);
-    const uint32_t by = byz - bz * (uint32_t)a.lay.nty;
-    // ---- the warp's two boxes (cells 64w .. 64w + 63) all plain FLUID with FLUID neighbours?
-    const uint32_t mask = (uint32_t)__ldg(a.tile_near + tile);
-    if (__all_sync(0xffffffffu, ((mask >> ((t >> 5) * 2u)) & 3u) == 0u))
-        pair_cells<L, F16C, COLL, LES, FAST, false>(a, tile, t, mask, bx, by, bz);
-    else
-        pair_cells<L, F16C, COLL, LES, FAST, true>(a, tile, t, mask, bx, by, bz);
-}
-
 // Resident CTAs (of 128 threads) per SM the pair kernels are built for: the populations of two
 // cells stay in registers across both collisions, so the budget is wider than the per-cell
 // kernel's.  Float16C in the fast arithmetic 8 (64 registers: 63.7 GLUPs on the 256^3 Float16C
@@ -287,8 +274,21 @@ constexpr int pair_min_blocks() {
 template <class L, bool F16C, int COLL, int LES, bool FAST>
 __global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, F16C, COLL, FAST>())) step_kernel_pair(const StepArgs a) {
     static_assert(LES != kLesLearned, "the learned closure runs in step_kernel_learned");
-    pdl_enter();
-    pair_step<L, F16C, COLL, LES, FAST>(a, blockIdx.x, threadIdx.x);
+    const uint32_t tile = blockIdx.x, t = threadIdx.x;
+    pdl_wait_before_masks(a);
+    // ---- the warp's two boxes (cells 64w .. 64w + 63) all plain FLUID with FLUID neighbours?
+    const uint32_t mask = (uint32_t)__ldg(a.tile_near + tile);
+    const bool general = !__all_sync(0xffffffffu, ((mask >> ((t >> 5) * 2u)) & 3u) == 0u);
+    // the masks of both cells (written for every cell of a box with its bit set)
+    uint4 m = make_uint4(0u, 0u, 0u, 0u);
+    if (general && ((mask >> (t >> 4)) & 1u)) m = __ldg(reinterpret_cast<const uint4*>(a.cell_masks + (2u * t + kTileCells * tile)));
+    pdl_wait_after_masks(a);
+    const uint32_t byz = a.lay.d_ntx.div(tile);
+    const uint32_t bx = tile - byz * (uint32_t)a.lay.ntx;
+    const uint32_t bz = a.lay.d_nty.div(byz);
+    const uint32_t by = byz - bz * (uint32_t)a.lay.nty;
+    if (!general) pair_cells<L, F16C, COLL, LES, FAST, false>(a, tile, t, m, bx, by, bz);
+    else pair_cells<L, F16C, COLL, LES, FAST, true>(a, tile, t, m, bx, by, bz);
 }
 
 template <class L, int METHOD, bool F16C, int COLL, int LES>

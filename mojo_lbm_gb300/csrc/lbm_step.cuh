@@ -36,7 +36,8 @@ struct StepArgs {
     ClosureUniform cl;         // and its warp-uniform part
     const uint8_t* tile_near;  // per tile (generic kernel: per 256 cells): bit w set if a cell of
                                // warp w or a cell it pulls from holds a flag other than plain FLUID
-    const uint2* cell_masks;   // per cell of such a warp: (raw_solid, nib_solid), cell_solid_masks
+    const uint2* cell_masks;   // per cell of such a warp: cell_masks_of
+    int32_t masks_ready;       // the kernel before this one in the stream is a step with the same masks
     uint32_t mx, my, shx, shxy; // lx = t & mx, ly = (t >> shx) & my, lz = t >> shxy
     // interpolated bounce-back fused into the step (block-per-tile kernels, double buffer): per
     // cell, (bit i set for each link whose wall node is x + c_i, index of its first link in the
@@ -570,14 +571,23 @@ __device__ __forceinline__ void equilibrium_bc(float (&f)[L::Q], const float* bc
 // Programmatic dependent launch of the step kernels (launch_pdl): wait until the previous grid in
 // the stream has completed and its writes are visible, then let the next grid (the next step) be
 // scheduled onto the SMs while this one runs, so that its launch latency overlaps this step.  The
-// wait comes before any access to the populations, flags or masks; both instructions are no-ops
-// for a grid launched without the attribute.
-__device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+// wait comes before any access to the populations; both instructions are no-ops for a grid launched
+// without the attribute.
+// The masks are read before the wait when a.masks_ready says that the previous grid is a step of the
+// same run: this grid's blocks start only after every block of that one has passed its own wait, and
+// by then the kernels that build the masks, which come before it in the stream, have completed.  Two
+// dependent loads leave the step's critical path that way; with the cell's own flag and the bounce-back
+// folded into the masks and the pull addresses (two more), the 256^2 D2Q9 cavity went from 2.81 to 2.30
+// us a step, the untiled one above from 72.5 to 67.6.
+__device__ __forceinline__ void pdl_wait_before_masks(const StepArgs& a) {
+    if (!a.masks_ready) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait_after_masks(const StepArgs& a) {
+    if (a.masks_ready) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Launches a step kernel with programmatic stream serialization allowed (see pdl_enter).
+// Launches a step kernel with programmatic stream serialization allowed (see pdl_wait_before_masks).
 template <class Kernel>
 cudaError_t launch_pdl(Kernel kernel, uint32_t grid, uint32_t block, cudaStream_t s, const StepArgs& a) {
     cudaLaunchConfig_t cfg = {};
@@ -628,13 +638,26 @@ struct AnyCell {
     }
 };
 
-// set_adjacent_flags (ops/load_and_store.mojo:270-291) of a cell of any layout: bit q of .x when the
-// flag at x - c_q is SOLID (raw compare), of .y when its enum nibble is; any: an own or neighbouring
-// flag is not 0.
+// The masks of a cell that the general forms of the step read in place of its flags, from its own flag
+// and its neighbours':
+//   .x  bit 0: the cell is not stepped (is_valid_thread, src/lbm/kernels/utils/checks.mojo:55-60);
+//       bit q: the flag at x - c_q is SOLID (raw compare: mid-grid bounce-back,
+//       ops/load_and_store.mojo:216)
+//   .y  bit 0: the cell is stepped and its own flag is not 0 (the step looks at it);
+//       bit q: the enum nibble of the flag at x - c_q is SOLID (moving wall,
+//       ops/boundary_condition.mojo:77)
+__device__ __forceinline__ uint2 cell_masks_of(uint32_t own, uint32_t raw_solid, uint32_t nib_solid) {
+    const bool inactive = (own & 0x0F) == LBM_FLAG_SOLID || (own & LBM_FLAG_EXCLUDE);
+    return make_uint2(raw_solid | (inactive ? 1u : 0u), nib_solid | (!inactive && own != 0u ? 1u : 0u));
+}
+
+// set_adjacent_flags (ops/load_and_store.mojo:270-291) of a cell of any layout: its masks; any: an own
+// or neighbouring flag is not 0.
 template <class L>
-__device__ __forceinline__ uint2 any_solid_masks(const uint8_t* __restrict__ flags, const LayoutDesc& l, const Nbr& nb,
-                                                 uint32_t& any) {
+__device__ __forceinline__ uint2 any_solid_masks(const uint8_t* __restrict__ flags, uint32_t own, const LayoutDesc& l,
+                                                 const Nbr& nb, uint32_t& any) {
     uint32_t raw_solid = 0u, nib_solid = 0u;
+    any = own;
     static_for<1, L::Q>([&](auto qc) {
         constexpr int q = qc.value;
         constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
@@ -643,24 +666,25 @@ __device__ __forceinline__ uint2 any_solid_masks(const uint8_t* __restrict__ fla
         if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
         if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
     });
-    return make_uint2(raw_solid, nib_solid);
+    return cell_masks_of(own, raw_solid, nib_solid);
 }
 
 // The per-thread body of the generic kernel (any tile, any size).  As in tile_cell below, GENERAL =
 // false is the form of a warp whose cells and pull neighbours are all plain FLUID; GENERAL = true
-// reads the flags and takes the neighbour masks built when they last changed (a.cell_masks), or
-// gathers the neighbours' flags when the handle holds no masks.
+// takes the cell's masks m (cell_masks_of).
 template <class L, int METHOD, bool F16C, int COLL, int LES, class Off, bool GENERAL>
-__device__ __forceinline__ void any_cell(const StepArgs& a, const uint32_t n) {
+__device__ __forceinline__ void any_cell(const StepArgs& a, const uint32_t n, const uint2 m) {
     using P = Pop<F16C>;
     using S = typename P::T;
     constexpr int Q = L::Q, D = L::D, K = D + 1;
     constexpr bool ESO = METHOD == LBM_ESOTERIC_PULL;
     uint8_t flag = 0;
+    uint32_t raw_solid = 0u, nib_solid = 0u;
     if constexpr (GENERAL) {
-        flag = __ldg(a.flags + n);
-        // is_valid_thread (src/lbm/kernels/utils/checks.mojo:55-60)
-        if ((flag & 0x0F) == LBM_FLAG_SOLID || (flag & LBM_FLAG_EXCLUDE)) return;
+        if (m.x & 1u) return;
+        if (m.y & 1u) flag = __ldg(a.flags + n);
+        raw_solid = m.x;
+        nib_solid = a.moving ? m.y & ~1u : 0u;
     }
     const AnyCell<L, Off> c(a.lay, n);
     const uint32_t T = a.lay.T;
@@ -668,12 +692,17 @@ __device__ __forceinline__ void any_cell(const StepArgs& a, const uint32_t n) {
     const S* fin = (const S*)a.f_in;
     S* fout = (S*)a.f_out;
 
-    // ---- stream (pull loads first, independent of the flags)
+    // ---- stream; a population whose pull neighbour is SOLID (raw compare) comes from the cell's own
+    // opposite slot instead (mid-grid bounce-back, ops/load_and_store.mojo:210-219), slot q +- 1
     float f[Q];
     if constexpr (!ESO) {
         static_for<0, Q>([&](auto qc) {
             constexpr int q = qc.value;
-            f[q] = P::ld(fin + (c.d.template at<-L::c(q, 0), -L::c(q, 1), -L::c(q, 2)>() + oT * q));
+            Off o = c.d.template at<-L::c(q, 0), -L::c(q, 1), -L::c(q, 2)>();
+            if constexpr (GENERAL && q > 0) {
+                if ((raw_solid >> q) & 1u) o = c.d.own + (opp<L>(q) > q ? oT : -oT);
+            }
+            f[q] = P::ld(fin + (o + oT * q));
         });
     } else {
         // slot pos + 1 = neg: the parity folds into two base pointers
@@ -689,30 +718,8 @@ __device__ __forceinline__ void any_cell(const StepArgs& a, const uint32_t n) {
     }
 
     if constexpr (GENERAL) {
-        uint32_t raw_solid = 0u, nib_solid = 0u;
-        if (!ESO || a.moving) {
-            uint2 m;
-            if (a.cell_masks) {
-                m = __ldg(a.cell_masks + n);
-            } else {
-                Nbr nb;
-                c.nbr(a.lay, nb);
-                uint32_t any = 0u;
-                m = any_solid_masks<L>(a.flags, a.lay, nb, any);
-            }
-            raw_solid = m.x;
-            nib_solid = m.y;
-        }
-        if constexpr (!ESO) {
-            // mid-grid bounce-back on a raw SOLID compare (ops/load_and_store.mojo:210-219)
-            if (raw_solid)
-                static_for<1, Q>([&](auto qc) {
-                    constexpr int q = qc.value;
-                    if ((raw_solid >> q) & 1u) f[q] = P::ld(fin + (c.d.own + oT * opp<L>(q)));
-                });
-        }
         // boundary conditions (steps/apply_boundary_condition.mojo:10-41)
-        if (a.moving && nib_solid) {
+        if (nib_solid) {
             Nbr nb;
             c.nbr(a.lay, nb);
             const uint64_t TK = (uint64_t)T * K;
@@ -764,13 +771,26 @@ constexpr int any_min_blocks() { return COLL == LBM_KBC || L::Q == 27 ? 3 : 4; }
 template <class L, int METHOD, bool F16C, int COLL, int LES, class Off>
 __global__ void __launch_bounds__(256, (any_min_blocks<L, COLL>())) step_kernel(const StepArgs a) {
     static_assert(LES != kLesLearned, "the learned closure runs in the block-per-tile kernel");
-    pdl_enter();
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = n < a.lay.ncells;
+    pdl_wait_before_masks(a);
     // (uniform over the warp: blocks are multiples of 32 threads)
-    const bool general = !a.tile_near || ((__ldg(a.tile_near + (n >> 8)) >> ((n >> 5) & 7u)) & 1u) != 0u;
-    if (n >= a.lay.ncells) return;
-    if (!general) any_cell<L, METHOD, F16C, COLL, LES, Off, false>(a, n);
-    else any_cell<L, METHOD, F16C, COLL, LES, Off, true>(a, n);
+    const bool general = !a.tile_near || ((__ldg(a.tile_near + (min(n, a.lay.ncells - 1u) >> 8)) >> ((n >> 5) & 7u)) & 1u) != 0u;
+    uint2 m = make_uint2(0u, 0u);
+    if (general && a.cell_masks && in) m = __ldg(a.cell_masks + n);
+    pdl_wait_after_masks(a);
+    if (!in) return;
+    if (!general) {
+        any_cell<L, METHOD, F16C, COLL, LES, Off, false>(a, n, m);
+        return;
+    }
+    if (!a.cell_masks) {
+        Nbr nb;
+        AnyCell<L, Off>(a.lay, n).nbr(a.lay, nb);
+        uint32_t any;
+        m = any_solid_masks<L>(a.flags, __ldg(a.flags + n), a.lay, nb, any);
+    }
+    any_cell<L, METHOD, F16C, COLL, LES, Off, true>(a, n, m);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -969,9 +989,7 @@ __device__ __forceinline__ void write_near_mask(uint32_t i, uint32_t nboxes, uin
 }
 
 // set_adjacent_flags (ops/load_and_store.mojo:270-291) for the cell at flag offset n with cell
-// deltas dc: bit q of raw_solid when the flag at x - c_q is SOLID (the raw compare of the
-// mid-grid bounce-back, ops/load_and_store.mojo:216), of nib_solid when its enum nibble is SOLID
-// (the moving wall, ops/boundary_condition.mojo:77).
+// deltas dc: its masks (cell_masks_of).
 template <class L>
 __device__ __forceinline__ uint2 cell_solid_masks(const uint8_t* __restrict__ flags, uint32_t n,
                                                   const int32_t (&dc)[3][3]) {
@@ -983,7 +1001,7 @@ __device__ __forceinline__ uint2 cell_solid_masks(const uint8_t* __restrict__ fl
         if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
         if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
     });
-    return make_uint2(raw_solid, nib_solid);
+    return cell_masks_of(__ldg(flags + n), raw_solid, nib_solid);
 }
 
 // The masks of every cell of the tile's warps whose mask bit is set, for the step to load instead
@@ -1088,11 +1106,11 @@ __device__ __forceinline__ void fused_links(float (&f)[L::Q], const uint2 lt, co
 // STAGED: the pull loads read the tile's shared-memory stage `stage` (stage_off; double buffer)
 // instead of global memory.
 // GENERAL = false is the form of a warp whose cells and pull neighbours are all plain FLUID: no
-// flag is read and the code is straight-line from the loads to the stores; GENERAL = true reads
-// the flags and handles every boundary.
+// flag is read and the code is straight-line from the loads to the stores; GENERAL = true takes the
+// cell's masks m (cell_masks_of) and handles every boundary.
 template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS, bool STAGED, bool GENERAL>
 __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile, const uint32_t tid,
-                                          const ClosureDev* cl, float4* fbuf, const void* stage) {
+                                          const uint2 m, const ClosureDev* cl, float4* fbuf, const void* stage) {
     using P = Pop<F16C>;
     using S = typename P::T;
     constexpr int Q = L::Q, D = L::D, K = D + 1;
@@ -1123,14 +1141,17 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
 
     uint8_t flag = 0;
     bool active = true;
+    uint32_t raw_solid = 0u, nib_solid = 0u;
     if constexpr (GENERAL) {
-        flag = __ldg(a.flags + n);
-        // is_valid_thread (src/lbm/kernels/utils/checks.mojo:55-60); the learned closure keeps
-        // every lane for its warp-wide products, the invalid ones write nothing
-        active = !((flag & 0x0F) == LBM_FLAG_SOLID || (flag & LBM_FLAG_EXCLUDE));
+        // the learned closure keeps every lane for its warp-wide products, the invalid ones write
+        // nothing
+        active = (m.x & 1u) == 0u;
         if constexpr (LES != kLesLearned) {
             if (!active) return;
         }
+        if (m.y & 1u) flag = __ldg(a.flags + n);
+        raw_solid = m.x & ~1u;
+        nib_solid = a.moving ? m.y & ~1u : 0u;
     }
 
     // ---- per-axis neighbour deltas, in cells (flags, bc) and in population elements (f)
@@ -1143,7 +1164,8 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
     const S* fin = (const S*)a.f_in;
     S* fout = (S*)a.f_out;
 
-    // ---- stream (pull loads first, independent of the flags)
+    // ---- stream; a population whose pull neighbour is SOLID (raw compare) comes from the cell's own
+    // opposite slot instead (mid-grid bounce-back, ops/load_and_store.mojo:216), slot q +- 1
     float f[Q];
     if constexpr (STAGED) {
         // the stage's regions: this cell's position, or along x the neighbour's (stage_off)
@@ -1163,7 +1185,10 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
         static_for<0, Q>([&](auto qc) {
             constexpr int q = qc.value;
             constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
-            const int32_t o = own + dp[0][sx + 1] + dp[1][sy + 1] + dp[2][sz + 1];
+            int32_t o = own + dp[0][sx + 1] + dp[1][sy + 1] + dp[2][sz + 1];
+            if constexpr (GENERAL && q > 0) {
+                if ((raw_solid >> q) & 1u) o = own + (opp<L>(q) > q ? (int32_t)T : -(int32_t)T);
+            }
             f[q] = ld(fin + o + (int32_t)(T * q));
         });
     } else {
@@ -1183,21 +1208,14 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
     }
 
     if constexpr (GENERAL) {
-        // ---- neighbour flags at x - c_q, as masks built when the flags last changed
-        // (cell_solid_masks: set_adjacent_flags, ops/load_and_store.mojo:270-291)
-        uint32_t raw_solid = 0u, nib_solid = 0u;
-        if (!ESO || a.moving) {
-            const uint2 m = __ldg(a.cell_masks + n);
-            raw_solid = m.x;
-            nib_solid = m.y;
-        }
         if constexpr (!ESO) {
-            // mid-grid bounce-back on a raw SOLID compare (ops/load_and_store.mojo:216)
-            if (raw_solid)
-                static_for<1, Q>([&](auto qc) {
-                    constexpr int q = qc.value;
-                    if ((raw_solid >> q) & 1u) f[q] = ld(fin + own + (int32_t)(T * opp<L>(q)));
-                });
+            if constexpr (STAGED) {
+                if (raw_solid)
+                    static_for<1, Q>([&](auto qc) {
+                        constexpr int q = qc.value;
+                        if ((raw_solid >> q) & 1u) f[q] = ld(fin + own + (int32_t)(T * opp<L>(q)));
+                    });
+            }
             if constexpr (LINKS) {
                 if (raw_solid) {
                     const uint2 lt = __ldg(a.link_table + n);
@@ -1205,7 +1223,7 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
                 }
             }
         }
-        if (a.moving && nib_solid) {
+        if (nib_solid) {
             moving_wall<L, SCALED>(f, nib_solid, a.bc, T, [&](auto qc) -> uint64_t {
                 constexpr int q = decltype(qc)::value;
                 constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
@@ -1247,18 +1265,29 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
     }
 }
 
+// Does a cell of the calling warp, or one it pulls from, hold a flag?  (bit w of the tile's mask byte;
+// the vote makes the choice warp-uniform)
+__device__ __forceinline__ bool tile_general(uint32_t mask, uint32_t tid) {
+    return !__all_sync(0xffffffffu, ((mask >> (tid >> 5)) & 1u) == 0u);
+}
+
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS, bool STAGED>
+__device__ __forceinline__ void tile_forms(const StepArgs& a, const uint32_t tile, const uint32_t tid, const bool general,
+                                           const uint2 m, const ClosureDev* cl, float4* fbuf, const void* stage) {
+    if (!general) tile_cell<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED, false>(a, tile, tid, m, cl, fbuf, stage);
+    else tile_cell<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED, true>(a, tile, tid, m, cl, fbuf, stage);
+}
+
 template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST = false, bool LINKS = false,
           bool STAGED = false>
 __device__ __forceinline__ void tile_step(const StepArgs& a, const uint32_t tile, const uint32_t tid,
                                           const ClosureDev* cl = nullptr, float4* fbuf = nullptr,
                                           int32_t near = -1, const void* stage = nullptr) {
-    // ---- are this warp's cells and their pull neighbours all plain FLUID?  (bit w of the tile's
-    // mask byte; the vote makes the choice warp-uniform)
     const uint32_t mask = near >= 0 ? (uint32_t)near : (uint32_t)__ldg(a.tile_near + tile);
-    if (__all_sync(0xffffffffu, ((mask >> (tid >> 5)) & 1u) == 0u))
-        tile_cell<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED, false>(a, tile, tid, cl, fbuf, stage);
-    else
-        tile_cell<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED, true>(a, tile, tid, cl, fbuf, stage);
+    const bool general = tile_general(mask, tid);
+    uint2 m = make_uint2(0u, 0u);
+    if (general) m = __ldg(a.cell_masks + (tid + kTileCells * tile));
+    tile_forms<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED>(a, tile, tid, general, m, cl, fbuf, stage);
 }
 
 #ifndef LBM_TILE_MIN_BLOCKS
@@ -1283,8 +1312,13 @@ template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST = false, 
 __global__ void __launch_bounds__(256, (tile_min_blocks<L, COLL, LINKS>()))
     step_kernel_tile(const StepArgs a) {
     static_assert(LES != kLesLearned, "the learned closure runs in step_kernel_learned");
-    pdl_enter();
-    tile_step<L, METHOD, F16C, COLL, LES, FAST, LINKS>(a, blockIdx.x, threadIdx.x);
+    const uint32_t tile = blockIdx.x, tid = threadIdx.x;
+    pdl_wait_before_masks(a);
+    const bool general = tile_general(__ldg(a.tile_near + tile), tid);
+    uint2 m = make_uint2(0u, 0u);
+    if (general) m = __ldg(a.cell_masks + (tid + kTileCells * tile));
+    pdl_wait_after_masks(a);
+    tile_forms<L, METHOD, F16C, COLL, LES, FAST, LINKS, false>(a, tile, tid, general, m, nullptr, nullptr, nullptr);
 }
 
 #ifndef LBM_LEARNED_MIN_BLOCKS
