@@ -47,6 +47,7 @@ struct lbm_batch {
     uint32_t* d_changed = nullptr;    // summary round in which a box summary last changed
     uint32_t summary_gen = 0;
     bool summary_valid = false;
+    bool masks_resting = false;       // the masks are those of the last run's bc (without_resting_walls)
     bool dirty = true;
     BatchLaunch step = nullptr;
     BatchLaunch step_links = nullptr;  // the step with the links fused in (double buffer), or null
@@ -98,15 +99,16 @@ __global__ void batch_near_kernel(const BatchArgs b, const uint8_t* box_sum, uin
 }
 
 // The neighbour-solid masks of the cells of every warp with its mask bit set, one block per unit,
-// after a change of the flags in this round (*changed == gen).
+// after a change of the flags in this round (*changed == gen), or always; resting_walls:
+// without_resting_walls.
 template <class L>
 __global__ void __launch_bounds__(256) batch_cell_mask_kernel(const BatchArgs b, const uint32_t* changed,
-                                                              uint32_t gen) {
-    if (*changed != gen) return;  // the same value for every thread
+                                                              uint32_t gen, int always, int resting_walls) {
+    if (!always && *changed != gen) return;  // the same value for every thread
     for (uint32_t u = blockIdx.x; u < b.total_units; u += gridDim.x) {  // blocks stride over the units
         const uint32_t d = find_domain(b.unit_begin, b.ndom, u);
         const StepArgs& a = b.dom[d];
-        tile_cell_masks<L>(a, u - b.unit_begin[d], const_cast<uint2*>(a.cell_masks));
+        tile_cell_masks<L>(a, u - b.unit_begin[d], const_cast<uint2*>(a.cell_masks), resting_walls != 0);
     }
 }
 
@@ -427,12 +429,17 @@ lbm_status lbm_batch_run(lbm_batch* b, int64_t n_steps, int64_t first_step, void
         LBM_BCK(cudaGetLastError());
         if (nboxes) {
             const uint32_t grid = std::min<uint32_t>(a.total_units, (uint32_t)b->sms * 8u);
+            // masks without the walls at rest serve this run only (lbm_run)
+            const bool resting = b->cfg.include_moving_boundary && !b->cfg.capture_density &&
+                                 !b->cfg.capture_velocity && n_steps >= 32;
+            const bool always = resting || b->masks_resting;
+            b->masks_resting = resting;
             if (b->lattice == LBM_D2Q9)
-                batch_cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen);
+                batch_cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen, always, resting);
             else if (b->lattice == LBM_D3Q19)
-                batch_cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen);
+                batch_cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen, always, resting);
             else
-                batch_cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen);
+                batch_cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen, always, resting);
         }
         LBM_BCK(cudaGetLastError());
     }

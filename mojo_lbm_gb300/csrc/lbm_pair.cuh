@@ -181,6 +181,12 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
 
     if constexpr (GENERAL) {
         const uint32_t wallA = m.y & ~1u, wallB = m.w & ~1u;
+        if constexpr (!FAST) {
+            if (a.moving) {
+                add_resting_walls<L>(fa, m.x & ~(m.y | 1u));
+                add_resting_walls<L>(fb, m.z & ~(m.w | 1u));
+            }
+        }
         if (a.moving && (wallA | wallB)) {
             // moving_wall_bc with the bc of each cell's SOLID pull neighbours
             auto wall = [&](float (&f)[Q], uint32_t nib, uint32_t tc) {

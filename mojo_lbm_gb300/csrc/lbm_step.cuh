@@ -651,6 +651,41 @@ __device__ __forceinline__ uint2 cell_masks_of(uint32_t own, uint32_t raw_solid,
     return make_uint2(raw_solid | (inactive ? 1u : 0u), nib_solid | (!inactive && own != 0u ? 1u : 0u));
 }
 
+// The masks without the walls at rest: bit q of .y is cleared where bit q of .x is set and the
+// moving-wall term of the wall's bc is exactly +0 (velocity component 0, a positive finite density), so
+// that the step neither reads that bc nor adds the term; it only adds the +0 (a bounced -0 becomes +0).
+// Valid for the bc values at the time of the call: a multi-step run builds these masks at its start.
+// moving_wall_bc reads 2 to 4 words of the wall's bc one direction after the other, and took 4 % of a
+// step of the 256^3 float32 cavity, 9 % of the Float16C one and 14 % of the 256^2 D2Q9 one, whose walls
+// all rest but the lid.  bc_base(q): element offset of component 0 of the pull neighbour's bc.
+template <class L, class BcBase>
+__device__ __forceinline__ uint2 without_resting_walls(uint2 m, const float* __restrict__ bc, uint32_t T, BcBase&& bc_base) {
+    static_for<1, L::Q>([&](auto qc) {
+        constexpr int q = qc.value;
+        if (((m.x & m.y) >> q) & 1u) {
+            const uint64_t b = bc_base(qc);
+            float cu = 0.f;  // as moving_wall
+            static_for<0, L::D>([&](auto dc) {
+                constexpr int d = dc.value;
+                if constexpr (L::c(q, d) > 0) cu += bc[b + (uint64_t)T * d];
+                else if constexpr (L::c(q, d) < 0) cu -= bc[b + (uint64_t)T * d];
+            });
+            const float rho = bc[b + (uint64_t)T * L::D];
+            if (cu == 0.f && rho > 0.f && rho < __int_as_float(0x7f800000)) m.y &= ~(1u << q);
+        }
+    });
+    return m;
+}
+
+// The +0 of the walls that without_resting_walls took out of the masks (exact arithmetic).
+template <class L>
+__device__ __forceinline__ void add_resting_walls(float (&f)[L::Q], uint32_t cleared) {
+    if (cleared)
+        static_for<1, L::Q>([&](auto qc) {
+            if ((cleared >> qc.value) & 1u) f[qc.value] += 0.f;
+        });
+}
+
 // set_adjacent_flags (ops/load_and_store.mojo:270-291) of a cell of any layout: its masks; any: an own
 // or neighbouring flag is not 0.
 template <class L>
@@ -719,6 +754,7 @@ __device__ __forceinline__ void any_cell(const StepArgs& a, const uint32_t n, co
 
     if constexpr (GENERAL) {
         // boundary conditions (steps/apply_boundary_condition.mojo:10-41)
+        if (a.moving) add_resting_walls<L>(f, raw_solid & ~(m.y | 1u));
         if (nib_solid) {
             Nbr nb;
             c.nbr(a.lay, nb);
@@ -1006,8 +1042,10 @@ __device__ __forceinline__ uint2 cell_solid_masks(const uint8_t* __restrict__ fl
 
 // The masks of every cell of the tile's warps whose mask bit is set, for the step to load instead
 // of gathering its neighbours' flags (the block of 256 threads of tile `tile`).
+// resting_walls: without_resting_walls (a.bc).
 template <class L>
-__device__ __forceinline__ void tile_cell_masks(const StepArgs& a, uint32_t tile, uint2* __restrict__ masks) {
+__device__ __forceinline__ void tile_cell_masks(const StepArgs& a, uint32_t tile, uint2* __restrict__ masks,
+                                                bool resting_walls) {
     const uint32_t tid = threadIdx.x;
     if (((__ldg(a.tile_near + tile) >> (tid >> 5)) & 1u) == 0u) return;  // warp-uniform
     const uint32_t byz = a.lay.d_ntx.div(tile);
@@ -1018,7 +1056,16 @@ __device__ __forceinline__ void tile_cell_masks(const StepArgs& a, uint32_t tile
     int32_t dc[3][3], dp[3][3];
     tile_deltas<L::D>(a, bx, by, bz, lx, ly, lz, (int32_t)(kTileCells * L::Q), dc, dp);
     const uint32_t n = tid + kTileCells * tile;
-    masks[n] = cell_solid_masks<L>(a.flags, n, dc);
+    uint2 m = cell_solid_masks<L>(a.flags, n, dc);
+    if (resting_walls)
+        m = without_resting_walls<L>(m, a.bc, kTileCells, [&](auto qc) -> uint64_t {
+            constexpr int q = decltype(qc)::value;
+            constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
+            const uint32_t k = (uint32_t)((int32_t)n + dc[0][sx + 1] + dc[1][sy + 1] + dc[2][sz + 1]);
+            const uint32_t kt = k / kTileCells;
+            return (uint64_t)(k - kt * kTileCells) + (uint64_t)kTileCells * (L::D + 1) * kt;
+        });
+    masks[n] = m;
 }
 
 // The shared-memory stage of the staged kernel (lbm_stage.cuh): per direction q, in q order, a region
@@ -1222,6 +1269,9 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
                     if (lt.x) fused_links<L, SCALED>(f, lt, raw_solid, a, fin, own, dp, ld);
                 }
             }
+        }
+        if constexpr (!FAST) {
+            if (a.moving) add_resting_walls<L>(f, raw_solid & ~m.y);
         }
         if (nib_solid) {
             moving_wall<L, SCALED>(f, nib_solid, a.bc, T, [&](auto qc) -> uint64_t {
