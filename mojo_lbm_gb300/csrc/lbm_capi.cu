@@ -85,6 +85,95 @@ __global__ void __launch_bounds__(256) cell_mask_kernel(const StepArgs a, uint2*
         tile_cell_masks<L>(a, tile, masks, resting_walls != 0);
 }
 
+// The masks of the block-per-tile kernels after the first build, in one launch: each block compares the
+// flags of `per_block` tiles (16 at most, 16 bytes a thread) with flags_seen, and for a tile that changed
+// it rebuilds, from the flags themselves, the mask byte and the cell masks of that tile and of the 26
+// around it (periodic), whose cells may pull from it.  A neighbour that differs from flags_seen as well
+// is left to its own block; two blocks that rebuild the same tile write the same values.  always: the
+// cell masks of every warp whose bit is set are rebuilt (a run without its walls at rest).
+// A single step with the three launches of the first build before it is bound by launches on the host
+// and by their chain on the GPU: a step of a 320 x 128 D2Q9 channel and its link pass, called from a host
+// loop, went from 18.0 to 11.2 us with this one (launched, like the steps, with programmatic dependent
+// launch).
+template <class L>
+__device__ __forceinline__ void rebuild_tile(const StepArgs& a, uint32_t tile, uint8_t* near, uint2* masks, bool resting,
+                                             uint32_t* bits) {
+    uint32_t any;
+    const uint2 m = tile_cell_mask<L>(a, tile, threadIdx.x, resting, any);
+    const bool warp_any = __any_sync(0xffffffffu, any != 0u);
+    if (warp_any) masks[threadIdx.x + kTileCells * tile] = m;
+    if (threadIdx.x == 0) *bits = 0u;
+    __syncthreads();
+    if (warp_any && (threadIdx.x & 31u) == 0u) atomicOr(bits, 1u << (threadIdx.x >> 5));
+    __syncthreads();
+    if (threadIdx.x == 0) near[tile] = (uint8_t)*bits;
+}
+
+// 16 flag bytes from p (byte loads when it is not 16-byte aligned).
+__device__ __forceinline__ uint4 load_flags16(const uint8_t* p) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0u) return __ldg(reinterpret_cast<const uint4*>(p));
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        w[k] = (uint32_t)__ldg(p + 4 * k) | ((uint32_t)__ldg(p + 4 * k + 1) << 8) | ((uint32_t)__ldg(p + 4 * k + 2) << 16) |
+               ((uint32_t)__ldg(p + 4 * k + 3) << 24);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ bool differ16(const uint4& x, const uint4& y) {
+    return x.x != y.x || x.y != y.y || x.z != y.z || x.w != y.w;
+}
+
+template <class L>
+__global__ void __launch_bounds__(256) tile_check_kernel(const StepArgs a, uint8_t* seen, uint8_t* near, uint2* masks,
+                                                         uint32_t ntiles, uint32_t per_block, int always, int resting) {
+    __shared__ uint32_t changed, bits;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tile0 = blockIdx.x * per_block, mine = threadIdx.x >> 4;
+    const bool in = mine < per_block && tile0 + mine < ntiles;
+    const size_t at = (size_t)(tile0 + mine) * kTileCells + (threadIdx.x & 15u) * 16u;
+    uint4 now = make_uint4(0u, 0u, 0u, 0u);
+    bool differ = false;
+    if (in) {
+        now = load_flags16(a.flags + at);
+        differ = differ16(now, *reinterpret_cast<const uint4*>(seen + at));
+    }
+    if (threadIdx.x == 0) changed = 0u;
+    if (__syncthreads_or(differ)) {
+        if (differ) atomicOr(&changed, 1u << mine);
+        __syncthreads();
+        for (uint32_t todo = changed; todo; todo &= todo - 1u) {
+            const uint32_t tile = tile0 + (uint32_t)__ffs(todo) - 1u;
+            const uint32_t byz = tile / (uint32_t)a.lay.ntx;
+            const int32_t bx = (int32_t)(tile - byz * (uint32_t)a.lay.ntx);
+            const int32_t bz = (int32_t)(byz / (uint32_t)a.lay.nty), by = (int32_t)byz - bz * a.lay.nty;
+            auto wrap = [](int32_t v, int32_t n) { return (uint32_t)(v < 0 ? n - 1 : (v == n ? 0 : v)); };
+            for (int32_t k = 0; k < 27; ++k) {
+                if (L::D == 2 && k / 9 != 1) continue;
+                const uint32_t t = wrap(bx + k % 3 - 1, a.lay.ntx) +
+                                   (uint32_t)a.lay.ntx * (wrap(by + k / 3 % 3 - 1, a.lay.nty) +
+                                                          (uint32_t)a.lay.nty * wrap(bz + k / 9 - 1, a.lay.ntz));
+                bool other = false;
+                if (t != tile && threadIdx.x < 16u) {
+                    const size_t o = (size_t)t * kTileCells + threadIdx.x * 16u;
+                    other = differ16(load_flags16(a.flags + o), __ldcg(reinterpret_cast<const uint4*>(seen + o)));
+                }
+                if (__syncthreads_or(other)) continue;
+                rebuild_tile<L>(a, t, near, masks, resting != 0, &bits);
+            }
+        }
+        __syncthreads();
+        if (differ) *reinterpret_cast<uint4*>(seen + at) = now;
+    }
+    if (always)
+        for (uint32_t k = 0; k < per_block && tile0 + k < ntiles; ++k)
+            if ((near[tile0 + k] >> (threadIdx.x >> 5)) & 1u) {
+                uint32_t any;
+                masks[threadIdx.x + kTileCells * (tile0 + k)] =
+                    tile_cell_mask<L>(a, tile0 + k, threadIdx.x, resting != 0, any);
+            }
+}
+
 // The generic kernel's masks (any tile): bit (n / 32) % 8 of near[n / 256] and the neighbour-solid masks
 // of the cells of such warps, from flags and flags_seen.  Both start as those of a domain whose
 // flags are all 0.
@@ -295,7 +384,9 @@ StepArgs step_args(const lbm_handle* h, const void* f_in, void* f_out, float* bc
 // Threads per block of the generic kernel unless the caller sets them: a block keeps its registers until
 // its slowest warp, one next to a wall, is done, and smaller blocks free them sooner (150 x 131 x 97
 // untiled float32 D3Q19 cavity: 84.0 us a step at 256 threads, 73.8 at 128, 72.5 at 64, 72.4 at 32).
-constexpr int kAnyThreads = 64;
+// KBC keeps 27 words per thread slot of a 256-thread block in shared memory, whatever the block's
+// size, and takes 256 (the cavity above with KBC: 118 us a step at 256 and at 128 threads, 157 at 64).
+int any_threads(const lbm_config_t& c) { return c.collision_op == LBM_KBC ? 256 : 64; }
 
 bool use_tile(const lbm_handle* h) { return h->step_tile != nullptr && h->path != 1; }
 
@@ -336,6 +427,19 @@ StepLaunch step_fn(const lbm_handle* h, const StepArgs& a) {
 // whose flags changed since the previous call are summarised again, and the masks are rebuilt
 // only if one did (every step of a run with fixed flags costs one pass over the flags).
 lbm_status tile_summary(lbm_handle* h, const uint8_t* flags, float* bc, bool always, bool resting, cudaStream_t s) {
+    if (h->summary_valid) {
+        // one tile a block until every SM has 8 blocks
+        const uint32_t per = std::max<uint32_t>(1u, std::min<uint32_t>(16u, h->ntiles / ((uint32_t)h->sm_count * 8u)));
+        const StepArgs a = step_args(h, nullptr, nullptr, bc, flags, 1.f, 0);
+        auto go = [&](auto kernel) {
+            return launch_pdl(kernel, (h->ntiles + per - 1u) / per, kTileCells, s, a, h->flags_seen, h->tile_near,
+                              h->cell_masks, h->ntiles, per, (int)always, (int)resting);
+        };
+        LBM_CK(h->grid.lattice == LBM_D2Q9 ? go(tile_check_kernel<D2Q9>)
+               : h->grid.lattice == LBM_D3Q19 ? go(tile_check_kernel<D3Q19>)
+                                              : go(tile_check_kernel<D3Q27>));
+        return LBM_OK;
+    }
     if (++h->summary_gen == 0u) ++h->summary_gen;  // 0 is the initial value of *changed
     const uint32_t gen = h->summary_gen;
     const uint32_t nboxes = h->ntiles * kTileWarps;
@@ -442,6 +546,10 @@ lbm_status step_once(lbm_handle* h, const void* f_in, void* f_out, float* bc, co
     LBM_CK(step_fn(h, a)(a, h->threads, s));
     return LBM_OK;
 }
+
+// Blocks of a reduction over n items: kReduceBlocks at most, none without an item (a block without one
+// adds 0 to the sums: the result does not depend on it).
+int reduce_blocks(uint64_t n) { return (int)std::min<uint64_t>(kReduceBlocks, (n + kReduceThreads - 1) / kReduceThreads); }
 
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 int ilog2(int v) { int r = 0; while ((1 << r) < v) ++r; return r; }
@@ -599,7 +707,7 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
     h->run_stream = nullptr;
     h->run_done = nullptr;
     h->tile_near = nullptr;
-    h->threads = kAnyThreads;
+    h->threads = any_threads(h->cfg);
     h->scratch = nullptr;
     h->closure = nullptr;
     std::memset(&h->closure_uniform, 0, sizeof(h->closure_uniform));
@@ -768,7 +876,7 @@ lbm_status lbm_set_closure(lbm_handle* h, const lbm_closure_t* closure) {
 
 lbm_status lbm_set_block_threads(lbm_handle* h, int32_t threads) {
     if (check_handle(h)) return LBM_EINVAL;
-    if (threads == 0) threads = kAnyThreads;
+    if (threads == 0) threads = any_threads(h->cfg);
     if (threads < 32 || threads > 256 || threads % 32)
         return fail(LBM_EINVAL, "threads per block must be a multiple of 32 in [32, 256]");
     h->threads = threads;
@@ -984,21 +1092,22 @@ lbm_status lbm_reduce_mass_momentum(lbm_handle* h, const void* f, const uint8_t*
     a.even = after_odd_step ? 1 : 0;
     const bool f16 = h->cfg.use_float16c != 0, eso = h->cfg.lbm_method == LBM_ESOTERIC_PULL;
     cudaStream_t s = (cudaStream_t)stream;
+    const int blocks = reduce_blocks(h->lay.ncells);
     lbm_status st = dispatch_lattice(h->grid.lattice, [&](auto Lt) -> lbm_status {
         using L = decltype(Lt);
         if (f16) {
-            if (eso) mass_partial_kernel<L, true, true><<<kReduceBlocks, kReduceThreads, 0, s>>>(a);
-            else mass_partial_kernel<L, true, false><<<kReduceBlocks, kReduceThreads, 0, s>>>(a);
+            if (eso) mass_partial_kernel<L, true, true><<<blocks, kReduceThreads, 0, s>>>(a);
+            else mass_partial_kernel<L, true, false><<<blocks, kReduceThreads, 0, s>>>(a);
         } else {
-            if (eso) mass_partial_kernel<L, false, true><<<kReduceBlocks, kReduceThreads, 0, s>>>(a);
-            else mass_partial_kernel<L, false, false><<<kReduceBlocks, kReduceThreads, 0, s>>>(a);
+            if (eso) mass_partial_kernel<L, false, true><<<blocks, kReduceThreads, 0, s>>>(a);
+            else mass_partial_kernel<L, false, false><<<blocks, kReduceThreads, 0, s>>>(a);
         }
         LBM_CK(cudaGetLastError());
         return LBM_OK;
     });
     if (st != LBM_OK) return st;
     double* res = h->scratch + kReduceBlocks * kReduceWidth;
-    final_sum_kernel<4><<<1, kReduceThreads, 0, s>>>(h->scratch, kReduceBlocks, res);
+    final_sum_kernel<4><<<1, kReduceThreads, 0, s>>>(h->scratch, blocks, res);
     LBM_CK(cudaGetLastError());
     LBM_CK(cudaMemcpyAsync(out, res, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
     LBM_CK(cudaStreamSynchronize(s));
@@ -1049,10 +1158,11 @@ lbm_status lbm_sum_link_force(lbm_handle* h, const float* link_force, int64_t n_
     if (n_links == 0) return LBM_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const int D = lattice_d(h->grid.lattice);
-    colsum_partial_kernel<<<kReduceBlocks, kReduceThreads, 0, s>>>(link_force, n_links, D, h->scratch);
+    const int blocks = reduce_blocks((uint64_t)n_links);
+    colsum_partial_kernel<<<blocks, kReduceThreads, 0, s>>>(link_force, n_links, D, h->scratch);
     LBM_CK(cudaGetLastError());
     double* res = h->scratch + kReduceBlocks * kReduceWidth;
-    final_sum_kernel<4><<<1, kReduceThreads, 0, s>>>(h->scratch, kReduceBlocks, res);
+    final_sum_kernel<4><<<1, kReduceThreads, 0, s>>>(h->scratch, blocks, res);
     LBM_CK(cudaGetLastError());
     double tmp[4];
     LBM_CK(cudaMemcpyAsync(tmp, res, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));

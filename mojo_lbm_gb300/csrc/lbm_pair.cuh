@@ -139,7 +139,7 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
     int32_t dxm, dxp, dy[3], dz[3];
     pair_deltas<D>(a, bx, by, bz, lxA, ly, lz, TQ, dxm, dxp, dy, dz);
     const int32_t own = (int32_t)tA + TQ * (int32_t)tile;
-    const S* fin = (const S*)a.f_in;
+    const S* fin = after_wait<S>(a.f_in);
     S* fout = (S*)a.f_out;
 
     // ---- stream: pull loads of both cells
@@ -283,11 +283,11 @@ __global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, F16C, COLL, 
     const uint32_t tile = blockIdx.x, t = threadIdx.x;
     pdl_wait_before_masks(a);
     // ---- the warp's two boxes (cells 64w .. 64w + 63) all plain FLUID with FLUID neighbours?
-    const uint32_t mask = (uint32_t)__ldg(a.tile_near + tile);
+    const uint32_t mask = load_near(a.tile_near + tile);
     const bool general = !__all_sync(0xffffffffu, ((mask >> ((t >> 5) * 2u)) & 3u) == 0u);
     // the masks of both cells (written for every cell of a box with its bit set)
     uint4 m = make_uint4(0u, 0u, 0u, 0u);
-    if (general && ((mask >> (t >> 4)) & 1u)) m = __ldg(reinterpret_cast<const uint4*>(a.cell_masks + (2u * t + kTileCells * tile)));
+    if (general && ((mask >> (t >> 4)) & 1u)) m = load_masks2(a.cell_masks + (2u * t + kTileCells * tile));
     pdl_wait_after_masks(a);
     const uint32_t byz = a.lay.d_ntx.div(tile);
     const uint32_t bx = tile - byz * (uint32_t)a.lay.ntx;

@@ -587,9 +587,33 @@ __device__ __forceinline__ void pdl_wait_after_masks(const StepArgs& a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Launches a step kernel with programmatic stream serialization allowed (see pdl_wait_before_masks).
-template <class Kernel>
-cudaError_t launch_pdl(Kernel kernel, uint32_t grid, uint32_t block, cudaStream_t s, const StepArgs& a) {
+// The masks' loads and the pointer to the populations, kept in order with those waits: a plain __ldg is
+// free to move above an asm statement, since the compiler takes what it reads for constant.  (volatile
+// asm statements keep their order among themselves.)
+__device__ __forceinline__ uint32_t load_near(const uint8_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 load_masks(const uint2* p) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint4 load_masks2(const uint2* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+template <class S>
+__device__ __forceinline__ const S* after_wait(const void* p) {
+    asm volatile("" : "+l"(p));
+    return static_cast<const S*>(p);
+}
+
+// Launches a kernel with programmatic stream serialization allowed (see pdl_wait_before_masks).
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kernel)(P...), uint32_t grid, uint32_t block, cudaStream_t s, const A&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -600,7 +624,7 @@ cudaError_t launch_pdl(Kernel kernel, uint32_t grid, uint32_t block, cudaStream_
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a);
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // Position of cell n of any layout, and its population offsets.
@@ -724,7 +748,7 @@ __device__ __forceinline__ void any_cell(const StepArgs& a, const uint32_t n, co
     const AnyCell<L, Off> c(a.lay, n);
     const uint32_t T = a.lay.T;
     const Off oT = (Off)T;
-    const S* fin = (const S*)a.f_in;
+    const S* fin = after_wait<S>(a.f_in);
     S* fout = (S*)a.f_out;
 
     // ---- stream; a population whose pull neighbour is SOLID (raw compare) comes from the cell's own
@@ -811,9 +835,9 @@ __global__ void __launch_bounds__(256, (any_min_blocks<L, COLL>())) step_kernel(
     const bool in = n < a.lay.ncells;
     pdl_wait_before_masks(a);
     // (uniform over the warp: blocks are multiples of 32 threads)
-    const bool general = !a.tile_near || ((__ldg(a.tile_near + (min(n, a.lay.ncells - 1u) >> 8)) >> ((n >> 5) & 7u)) & 1u) != 0u;
+    const bool general = !a.tile_near || ((load_near(a.tile_near + (min(n, a.lay.ncells - 1u) >> 8)) >> ((n >> 5) & 7u)) & 1u) != 0u;
     uint2 m = make_uint2(0u, 0u);
-    if (general && a.cell_masks && in) m = __ldg(a.cell_masks + n);
+    if (general && a.cell_masks && in) m = load_masks(a.cell_masks + n);
     pdl_wait_after_masks(a);
     if (!in) return;
     if (!general) {
@@ -1025,29 +1049,29 @@ __device__ __forceinline__ void write_near_mask(uint32_t i, uint32_t nboxes, uin
 }
 
 // set_adjacent_flags (ops/load_and_store.mojo:270-291) for the cell at flag offset n with cell
-// deltas dc: its masks (cell_masks_of).
+// deltas dc: its masks (cell_masks_of); any: an own or neighbouring flag is not 0.
 template <class L>
 __device__ __forceinline__ uint2 cell_solid_masks(const uint8_t* __restrict__ flags, uint32_t n,
-                                                  const int32_t (&dc)[3][3]) {
+                                                  const int32_t (&dc)[3][3], uint32_t& any) {
     uint32_t raw_solid = 0u, nib_solid = 0u;
+    const uint32_t own = __ldg(flags + n);
+    any = own;
     static_for<1, L::Q>([&](auto qc) {
         constexpr int q = qc.value;
         constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
         const uint8_t pf = __ldg(flags + ((int32_t)n + dc[0][sx + 1] + dc[1][sy + 1] + dc[2][sz + 1]));
+        any |= pf;
         if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
         if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
     });
-    return cell_masks_of(__ldg(flags + n), raw_solid, nib_solid);
+    return cell_masks_of(own, raw_solid, nib_solid);
 }
 
-// The masks of every cell of the tile's warps whose mask bit is set, for the step to load instead
-// of gathering its neighbours' flags (the block of 256 threads of tile `tile`).
-// resting_walls: without_resting_walls (a.bc).
+// The masks of cell `tid` of tile `tile`; resting_walls: without_resting_walls (a.bc).  any: an own or
+// neighbouring flag is not 0.
 template <class L>
-__device__ __forceinline__ void tile_cell_masks(const StepArgs& a, uint32_t tile, uint2* __restrict__ masks,
-                                                bool resting_walls) {
-    const uint32_t tid = threadIdx.x;
-    if (((__ldg(a.tile_near + tile) >> (tid >> 5)) & 1u) == 0u) return;  // warp-uniform
+__device__ __forceinline__ uint2 tile_cell_mask(const StepArgs& a, uint32_t tile, uint32_t tid, bool resting_walls,
+                                                uint32_t& any) {
     const uint32_t byz = a.lay.d_ntx.div(tile);
     const uint32_t bx = tile - byz * (uint32_t)a.lay.ntx;
     const uint32_t bz = a.lay.d_nty.div(byz);
@@ -1056,7 +1080,7 @@ __device__ __forceinline__ void tile_cell_masks(const StepArgs& a, uint32_t tile
     int32_t dc[3][3], dp[3][3];
     tile_deltas<L::D>(a, bx, by, bz, lx, ly, lz, (int32_t)(kTileCells * L::Q), dc, dp);
     const uint32_t n = tid + kTileCells * tile;
-    uint2 m = cell_solid_masks<L>(a.flags, n, dc);
+    uint2 m = cell_solid_masks<L>(a.flags, n, dc, any);
     if (resting_walls)
         m = without_resting_walls<L>(m, a.bc, kTileCells, [&](auto qc) -> uint64_t {
             constexpr int q = decltype(qc)::value;
@@ -1065,7 +1089,18 @@ __device__ __forceinline__ void tile_cell_masks(const StepArgs& a, uint32_t tile
             const uint32_t kt = k / kTileCells;
             return (uint64_t)(k - kt * kTileCells) + (uint64_t)kTileCells * (L::D + 1) * kt;
         });
-    masks[n] = m;
+    return m;
+}
+
+// The masks of every cell of the tile's warps whose mask bit is set, for the step to load instead
+// of gathering its neighbours' flags (the block of 256 threads of tile `tile`).
+template <class L>
+__device__ __forceinline__ void tile_cell_masks(const StepArgs& a, uint32_t tile, uint2* __restrict__ masks,
+                                                bool resting_walls) {
+    const uint32_t tid = threadIdx.x;
+    if (((__ldg(a.tile_near + tile) >> (tid >> 5)) & 1u) == 0u) return;  // warp-uniform
+    uint32_t any;
+    masks[tid + kTileCells * tile] = tile_cell_mask<L>(a, tile, tid, resting_walls, any);
 }
 
 // The shared-memory stage of the staged kernel (lbm_stage.cuh): per direction q, in q order, a region
@@ -1208,7 +1243,7 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
     int32_t dc[3][3], dp[3][3];
     tile_deltas<D>(a, bx, by, bz, lx, ly, lz, TQ, dc, dp);
     const int32_t own = (int32_t)tid + TQ * (int32_t)tile;
-    const S* fin = (const S*)a.f_in;
+    const S* fin = after_wait<S>(a.f_in);
     S* fout = (S*)a.f_out;
 
     // ---- stream; a population whose pull neighbour is SOLID (raw compare) comes from the cell's own
@@ -1364,9 +1399,9 @@ __global__ void __launch_bounds__(256, (tile_min_blocks<L, COLL, LINKS>()))
     static_assert(LES != kLesLearned, "the learned closure runs in step_kernel_learned");
     const uint32_t tile = blockIdx.x, tid = threadIdx.x;
     pdl_wait_before_masks(a);
-    const bool general = tile_general(__ldg(a.tile_near + tile), tid);
+    const bool general = tile_general(load_near(a.tile_near + tile), tid);
     uint2 m = make_uint2(0u, 0u);
-    if (general) m = __ldg(a.cell_masks + (tid + kTileCells * tile));
+    if (general) m = load_masks(a.cell_masks + (tid + kTileCells * tile));
     pdl_wait_after_masks(a);
     tile_forms<L, METHOD, F16C, COLL, LES, FAST, LINKS, false>(a, tile, tid, general, m, nullptr, nullptr, nullptr);
 }
