@@ -28,6 +28,9 @@ StepLaunch get_fast_tile_step_d3q27(int, int, int, int);
 StepLaunch get_pair_step_d2q9(int, int, int, int);
 StepLaunch get_pair_step_d3q19(int, int, int, int);
 StepLaunch get_pair_step_d3q27(int, int, int, int);
+StepLaunch get_pair_eso_step_d2q9(int, int, int);
+StepLaunch get_pair_eso_step_d3q19(int, int, int);
+StepLaunch get_pair_eso_step_d3q27(int, int, int);
 StepLaunch get_links_tile_step_d2q9(int, int, int, int);
 StepLaunch get_staged_step_d2q9(int, int, int, int);
 StepLaunch get_staged_step_d3q19(int, int, int, int);
@@ -277,6 +280,7 @@ struct lbm_handle {
     StepLaunch step_tile;  // block-per-tile kernel, or null when the grid does not qualify
     StepLaunch step_learned;  // block-per-tile kernel with the learned closure (LES handles), or null
     StepLaunch step_pair;  // cell-pair block-per-tile kernel (double buffer, tx >= 2), or null
+    StepLaunch step_pair_eso;  // cell-pair kernel of the in-place method (fast arithmetic), or null
     int pair_auto;         // the automatic choice takes the cell-pair kernel
     StepLaunch step_links;    // block-per-tile kernel with fused links (double buffer), or null
     StepLaunch step_staged;   // staged block-per-tile kernel (double buffer, 16-byte tile rows), or null
@@ -393,6 +397,26 @@ bool use_tile(const lbm_handle* h) { return h->step_tile != nullptr && h->path !
 // Two waves of the cell-pair kernel's CTAs (8 per SM) on the 152 SMs of a GB300.
 constexpr uint32_t kPairAutoMinTiles = 2u * 8u * 152u;
 
+// Where the cell-pair kernel measured faster than the per-cell one on large grids (us a step, pair / per
+// cell; 2048^2 D2Q9, 160^3 D3Q19, 144^3 D3Q27 cavities).  Exact arithmetic, double buffer: D2Q9 and
+// D3Q19 except KBC.  Fast arithmetic:
+//   D2Q9   all but float32 KBC (SRT f32 49.4 / 55.0, f16 36.5 / 45.2; in place f32 48.0 / 54.6, f16 30.0 /
+//          42.5; KBC f16 54.6 / 58.0, in place 45.6 / 58.9; KBC f32 59.8 / 58.2)
+//   D3Q19  Float16C (SRT 66.6 / 72.5, in place 67.3 / 82.2; TRT 77.3 / 77.3, in place 76.0 / 89.2), KBC (f32
+//          112.7 / 117.2, in place 108.4 / 119.4) and the in-place method (SRT f32 94.3 / 101.3); not the
+//          other float32 double-buffer ones (SRT 97.4 / 95.8, with LES 100.5 / 96.3)
+//   D3Q27  Float16C in place except KBC (SRT 84.4 / 91.7; KBC 133 / 117; double buffer SRT 91.5 / 83.6; f32
+//          in place 111.8 / 109.6): its 54 populations leave 4 blocks per SM
+bool pair_pays(int lattice, int method, bool f16, int coll, bool les, bool fast) {
+    const bool eso = method == LBM_ESOTERIC_PULL, kbc = coll == LBM_KBC;
+    if (!fast) return lattice != LBM_D3Q27 && !kbc;  // (double buffer)
+    switch (lattice) {
+        case LBM_D2Q9: return !kbc || f16;
+        case LBM_D3Q19: return eso || f16 || kbc;
+        default: return eso && f16 && !kbc;
+    }
+}
+
 // The staged kernel is chosen (path 4) and can run: no learned closure, no fused links.
 bool use_staged(const lbm_handle* h) {
     return h->path == 4 && h->step_staged != nullptr && !h->closure_on && !h->link_table;
@@ -400,12 +424,11 @@ bool use_staged(const lbm_handle* h) {
 
 // The cell-pair kernel is chosen (path 3) and can run: no learned closure, no fused links.
 // The automatic choice (path 0) takes it where it measured faster than the per-cell kernel: the
-// double-buffer D2Q9 / D3Q19 configurations other than KBC (whose larger register demand halves the
-// pair kernel's occupancy) on grids of at least kPairAutoMinTiles tiles.  On fewer tiles the step
+// configurations of pair_pays on grids of at least kPairAutoMinTiles tiles.  On fewer tiles the step
 // is latency-bound, and the per-cell kernel, which gives each pair two threads, finishes sooner
 // (the 256^2 D2Q9 cavity, 256 tiles: 3.2 against 4.3 us a step).
 bool use_pair(const lbm_handle* h) {
-    return (h->path == 3 || (h->path == 0 && h->pair_auto)) && h->step_pair != nullptr && !h->closure_on &&
+    return ((h->path == 3 && h->step_pair != nullptr) || (h->path == 0 && h->pair_auto)) && !h->closure_on &&
            !h->link_table;
 }
 
@@ -418,8 +441,7 @@ StepLaunch step_fn(const lbm_handle* h, const StepArgs& a) {
     if (h->link_table) return h->step_links;
     const uintptr_t al = reinterpret_cast<uintptr_t>(a.f_in) | reinterpret_cast<uintptr_t>(a.f_out);
     if (use_staged(h) && (al & 15u) == 0u) return h->step_staged;  // bulk copies: 16-byte aligned rows
-    if (use_pair(h) && ((reinterpret_cast<uintptr_t>(a.f_in) | reinterpret_cast<uintptr_t>(a.f_out)) & 7u) == 0u)
-        return h->step_pair;
+    if (use_pair(h) && (al & 7u) == 0u) return h->step_pair ? h->step_pair : h->step_pair_eso;
     return h->step_tile;
 }
 
@@ -666,10 +688,15 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
                     : grid->lattice == LBM_D2Q9 ? get_learned_step_d2q9(m, f16, co)
                     : grid->lattice == LBM_D3Q19 ? get_learned_step_d3q19(m, f16, co)
                                                  : get_learned_step_d3q27(m, f16, co);
-    h->step_pair = !(tile_ok && m == LBM_DOUBLE_BUFFER && grid->tx >= 2) ? nullptr
+    const bool pair_ok = tile_ok && grid->tx >= 2;
+    h->step_pair = !(pair_ok && m == LBM_DOUBLE_BUFFER) ? nullptr
                  : grid->lattice == LBM_D2Q9 ? get_pair_step_d2q9(f16, co, les, fast)
                  : grid->lattice == LBM_D3Q19 ? get_pair_step_d3q19(f16, co, les, fast)
                                               : get_pair_step_d3q27(f16, co, les, fast);
+    h->step_pair_eso = !(pair_ok && m == LBM_ESOTERIC_PULL && fast) ? nullptr
+                     : grid->lattice == LBM_D2Q9 ? get_pair_eso_step_d2q9(f16, co, les)
+                     : grid->lattice == LBM_D3Q19 ? get_pair_eso_step_d3q19(f16, co, les)
+                                                  : get_pair_eso_step_d3q27(f16, co, les);
     h->step_links = !(tile_ok && m == LBM_DOUBLE_BUFFER) ? nullptr
                   : grid->lattice == LBM_D2Q9 ? get_links_tile_step_d2q9(f16, co, les, fast)
                   : grid->lattice == LBM_D3Q19 ? get_links_tile_step_d3q19(f16, co, les, fast)
@@ -687,8 +714,8 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
                    : grid->lattice == LBM_D2Q9 ? get_staged_step_d2q9(f16, co, les, fast)
                    : grid->lattice == LBM_D3Q19 ? get_staged_step_d3q19(f16, co, les, fast)
                                                 : get_staged_step_d3q27(f16, co, les, fast);
-    h->pair_auto = h->step_pair != nullptr && co != LBM_KBC && grid->lattice != LBM_D3Q27 &&
-                   h->lay.ncells / h->lay.T >= kPairAutoMinTiles;
+    h->pair_auto = (h->step_pair || h->step_pair_eso) && h->lay.ncells / h->lay.T >= kPairAutoMinTiles &&
+                   pair_pays(grid->lattice, m, f16 != 0, co, les != 0, fast);
     h->path = 0;
     h->ntiles = h->lay.ncells / h->lay.T;
     h->mx = (uint32_t)grid->tx - 1u;

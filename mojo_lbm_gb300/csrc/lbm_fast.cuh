@@ -35,16 +35,20 @@ __device__ __forceinline__ float rcp_approx(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+__device__ __forceinline__ F2 rcp_approx(F2 a) { return F2{rcp_approx(a.x), rcp_approx(a.y)}; }
+__device__ __forceinline__ F2 sqrt_approx(F2 a) { return F2{sqrt_approx(a.x), sqrt_approx(a.y)}; }
 
-// e_q . u with the first non-zero component taken as is (no 0 + x), for the fast build
-template <class L, int q>
-__device__ __forceinline__ float edot_fast(const float* u) {
-    constexpr int d0 = L::c(q, 0) != 0 ? 0 : (L::c(q, 1) != 0 ? 1 : 2);
-    float o = L::c(q, d0) > 0 ? u[d0] : -u[d0];
-    static_for<d0 + 1, L::D>([&](auto dc) {
+// e_q . u with the first positive component taken as is (no 0 + x), for the fast build (q odd: a
+// direction with a positive component)
+template <class L, int q, class V>
+__device__ __forceinline__ V edot_fast(const V* u) {
+    constexpr int d0 = L::c(q, 0) > 0 ? 0 : (L::c(q, 1) > 0 ? 1 : 2);
+    static_assert(L::c(q, d0) > 0, "odd directions have a positive component");
+    V o = u[d0];
+    static_for<0, L::D>([&](auto dc) {
         constexpr int d = dc.value;
-        if constexpr (L::c(q, d) > 0) o += u[d];
-        else if constexpr (L::c(q, d) < 0) o -= u[d];
+        if constexpr (d != d0 && L::c(q, d) > 0) o = o + u[d];
+        else if constexpr (d != d0 && L::c(q, d) < 0) o = o - u[d];
     });
     return o;
 }
@@ -52,188 +56,190 @@ __device__ __forceinline__ float edot_fast(const float* u) {
 template <class L, int q>
 constexpr int nnz_of() { return (L::c(q, 0) != 0) + (L::c(q, 1) != 0) + (L::c(q, 2) != 0); }
 
+// (e_q . u)^2; uc2: the squares of the components
+template <class L, int q, class V>
+__device__ __forceinline__ V edot2_fast(V eu, const V* uc2) {
+    if constexpr (nnz_of<L, q>() == 1) return uc2[L::c(q, 0) != 0 ? 0 : (L::c(q, 1) != 0 ? 1 : 2)];
+    else return eu * eu;
+}
+
 // The pair (q, q+1) of r * f_eq in units s: (plus, minus) = (A + C45 e2) +- C3 eu with
 // A = w a0, C3 = 3 w r0, C45 = 4.5 w r0, where the caller passes a0 = r s (rho (1 - 1.5 uu) - ddf)
 // and r0 = r s rho.  With ddf this is the shifted equilibrium
 // w rho (3 eu + 4.5 eu^2 - 1.5 uu) + w (rho - 1) (src/lbm/kernels/utils/equilibrium.mojo:10-39).
-template <class L, int q>
-__device__ __forceinline__ void feq_pair_fast(float a0, float r0, const float* u, const float* uc2, float& plus,
-                                              float& minus) {
+template <class L, int q, class V>
+__device__ __forceinline__ void feq_pair_fast(V a0, V r0, const V* u, const V* uc2, V& plus, V& minus) {
     constexpr float w = wf<L>(q);
-    const float eu = edot_fast<L, q>(u);
-    float e2;
-    if constexpr (nnz_of<L, q>() == 1) {
-        constexpr int d0 = L::c(q, 0) != 0 ? 0 : (L::c(q, 1) != 0 ? 1 : 2);
-        e2 = uc2[d0];
-    } else {
-        e2 = eu * eu;
-    }
-    const float c3 = (3.f * w) * r0;
-    const float base = __fmaf_rn((4.5f * w) * r0, e2, w * a0);
-    plus = __fmaf_rn(c3, eu, base);
-    minus = __fmaf_rn(-c3, eu, base);
+    const V eu = edot_fast<L, q>(u);
+    const V e2 = edot2_fast<L, q>(eu, uc2);
+    const V base = vfma(r0 * (4.5f * w), e2, a0 * w);
+    const V c3 = r0 * (3.f * w);
+    plus = vfma(c3, eu, base);
+    if constexpr (std::is_same_v<V, float>) minus = vfma(-c3, eu, base);
+    else minus = vfma(r0 * (-3.f * w), eu, base);
 }
 
-// The collision of the fast build, in place on f (in units of 2^-112 when SCALED).
-// bc_own_base, T, own_flag: the capture outputs, as collide() writes them.
-template <class L, int COLL, int LES, bool SCALED>
-__device__ __forceinline__ void collide_fast(float (&f)[L::Q], const StepArgs& a, float* bc_own_base, uint32_t T,
-                                             uint8_t own_flag, bool active = true) {
+// The collision of the fast build, in place on f (in units of 2^-112 when SCALED).  V: float, one cell,
+// or F2, two cells by packed instructions, with the same operations on each.  capture(rho, u) is called
+// with the density and velocity.
+template <class L, int COLL, int LES, bool SCALED, class V, class Capture>
+__device__ __forceinline__ void collide_fast_v(V (&f)[L::Q], const StepArgs& a, Capture&& capture) {
     static_assert(!(SCALED && (LES || COLL == LBM_KBC)), "scaled populations need a collision linear in f");
     constexpr int Q = L::Q, D = L::D, NP = (Q - 1) / 2, NS = L::NS;
     constexpr float S = SCALED ? 0x1p-112f : 1.f;  // stored units per population unit
     constexpr float IS = SCALED ? 0x1p112f : 1.f;
+    auto stored = [](V v) { if constexpr (SCALED) return v * S; else return v; };
+    auto units = [](V v) { if constexpr (SCALED) return v * IS; else return v; };
     constexpr float cs2 = (float)(1.0 / 3.0);
     const float ddf = a.ddf ? 1.f : 0.f;
 
-    // ---- moments from opposite pairs
-    float ps[NP], pd[NP];
+    // ---- moments from opposite pairs (the first direction with a component has it positive)
+    V ps[NP], pd[NP];
     static_for<0, NP>([&](auto pc) {
         constexpr int p = pc.value, q = 2 * p + 1;
         ps[p] = f[q] + f[q + 1];
         pd[p] = f[q] - f[q + 1];
     });
-    float rs = f[0];
-    static_for<0, NP>([&](auto pc) { rs += ps[pc.value]; });
-    float ms[3] = {0.f, 0.f, 0.f};
+    V rs = f[0];
+    static_for<0, NP>([&](auto pc) { rs = rs + ps[pc.value]; });
+    V ms[3] = {splat<V>(0.f), splat<V>(0.f), splat<V>(0.f)};
     static_for<0, D>([&](auto dc) {
         constexpr int d = dc.value;
-        bool first = true;
         static_for<0, NP>([&](auto pc) {
             constexpr int p = pc.value, q = 2 * p + 1;
-            if constexpr (L::c(q, d) != 0) {
-                const float v = L::c(q, d) > 0 ? pd[p] : -pd[p];
-                ms[d] = first ? v : ms[d] + v;
-                first = false;
-            }
+            if constexpr (p == d) ms[d] = pd[p];  // (the axis directions come first)
+            else if constexpr (L::c(q, d) > 0) ms[d] = ms[d] + pd[p];
+            else if constexpr (L::c(q, d) < 0) ms[d] = ms[d] - pd[p];
         });
     });
-    const float rho = __fmaf_rn(rs, IS, ddf);
-    const float k = IS * rcp_approx(rho);
-    float u[3] = {0.f, 0.f, 0.f}, uc2[3] = {0.f, 0.f, 0.f};
+    const V rho = vfma(rs, IS, ddf);
+    const V k = units(rcp_approx(rho));
+    V u[3] = {splat<V>(0.f), splat<V>(0.f), splat<V>(0.f)}, uc2[3] = {splat<V>(0.f), splat<V>(0.f), splat<V>(0.f)};
     static_for<0, D>([&](auto dc) {
         u[dc.value] = ms[dc.value] * k;
-        uc2[dc.value] = u[dc.value] * u[dc.value];
+        uc2[dc.value] = mul_apart(u[dc.value], u[dc.value]);
     });
-    float uu = uc2[0] + uc2[1];
-    if constexpr (D == 3) uu += uc2[2];
-
-    if (active && a.cap_rho && (own_flag & LBM_FLAG_CAPTURE_DENSITY)) bc_own_base[(size_t)T * D] = rho;
-    if (active && a.cap_u && (own_flag & LBM_FLAG_CAPTURE_VELOCITY))
-        static_for<0, D>([&](auto dc) { bc_own_base[(size_t)T * dc.value] = u[dc.value]; });
+    V uu = uc2[0] + uc2[1];
+    if constexpr (D == 3) uu = uu + uc2[2];
+    capture(rho, u);
 
     // rho (1 - 1.5 uu) - ddf: the part of f_eq / w without e.u
-    const float r1 = __fmaf_rn(rho, __fmaf_rn(-1.5f, uu, 1.f), -ddf);
+    const V r1 = vfma(rho, vfma(uu, -1.5f, 1.f), -ddf);
 
     // ---- non-equilibrium stress and the local relaxation time
-    float tau_l = a.tau;
-    [[maybe_unused]] float P[NS];
+    V tau_l = splat<V>(a.tau);
+    [[maybe_unused]] V P[NS];
     constexpr bool NEED_NEQ = LES || COLL == LBM_KBC || COLL == LBM_RLBM;
     if constexpr (NEED_NEQ) {
+        V nu_[3];  // -u
+        static_for<0, D>([&](auto dc) { nu_[dc.value] = u[dc.value] * -1.f; });
         static_for<0, NS>([&](auto nc) {
             constexpr int n = nc.value, A = sa<L>(n), B = sb<L>(n);
-            float raw = 0.f;
+            V raw = splat<V>(0.f);
             bool first = true;
             static_for<0, NP>([&](auto pc) {
                 constexpr int p = pc.value, q = 2 * p + 1;
                 constexpr int cc = L::c(q, A) * L::c(q, B);
                 if constexpr (cc != 0) {
-                    const float v = cc > 0 ? ps[p] : -ps[p];
-                    raw = first ? v : raw + v;
+                    raw = first ? ps[p] : cc > 0 ? raw + ps[p] : raw - ps[p];
                     first = false;
                 }
             });
             // Pi_ab = IS (raw - m_a u_b) - cs^2 (rho - ddf) delta_ab, with m_a = IS ms_a = rho u_a
-            const float t = __fmaf_rn(-ms[A], u[B], raw);
-            if constexpr (A == B) P[n] = __fmaf_rn(t, IS, -cs2 * (rho - ddf));
-            else P[n] = t * IS;
+            const V t = vfma(ms[A], nu_[B], raw);
+            if constexpr (A == B) P[n] = vfma(t, IS, mul_apart(rho - ddf, -cs2));
+            else P[n] = units(t);
         });
         if constexpr (LES) {
             // get_strain_rate_tensor / _norm_squared (moment.mojo:154-215),
             // get_Smagorinsky_LES_tau (src/lbm/kernels/ops/turbulence.mojo:12-38):
             // S = -Pi / (2 rho cs^2 tau), tau_l = tau + 3 Cs^2 sqrt(2 |S|^2)
-            const float kS = rcp_approx(2.f * cs2 * rho * a.tau);
-            float s2 = 0.f;
+            const V kS = rcp_approx(rho * (2.f * cs2) * a.tau);
+            V s2 = splat<V>(0.f);
             static_for<0, NS>([&](auto nc) {
                 constexpr int n = nc.value;
-                const float pn = P[n];
-                if constexpr (sa<L>(n) != sb<L>(n)) s2 = __fmaf_rn(2.f * pn, pn, s2);
-                else s2 = __fmaf_rn(pn, pn, s2);
+                const V pn = P[n];
+                if constexpr (sa<L>(n) != sb<L>(n)) s2 = vfma(pn * 2.f, pn, s2);
+                else s2 = vfma(pn, pn, s2);
             });
             // |S| = |Pi| kS
-            tau_l = __fmaf_rn(3.f * (a.Cs * a.Cs), sqrt_approx(2.f * s2) * kS, a.tau);
+            tau_l = vfma(sqrt_approx(s2 * 2.f) * kS, 3.f * (a.Cs * a.Cs), a.tau);
         }
     }
 
     if constexpr (COLL == LBM_SRT) {
         // SRT: f' = (1 - w) f + w f_eq
-        const float om = LES ? rcp_approx(tau_l) : a.inv_tau;
-        const float om1 = 1.f - om;
-        const float a0 = (om * S) * r1, r0 = (om * S) * rho;
-        f[0] = __fmaf_rn(om1, f[0], wf<L>(0) * a0);
+        V om1, a0, r0;
+        if constexpr (LES) {
+            const V om = rcp_approx(tau_l);
+            om1 = splat<V>(1.f) - om;
+            a0 = stored(om) * r1;
+            r0 = stored(om) * rho;
+        } else {
+            const float om = a.inv_tau;
+            om1 = splat<V>(1.f - om);
+            a0 = r1 * (om * S);
+            r0 = rho * (om * S);
+        }
+        f[0] = vfma(om1, f[0], a0 * wf<L>(0));
         static_for<0, NP>([&](auto pc) {
             constexpr int q = 2 * pc.value + 1;
-            float p, m;
+            V p, m;
             feq_pair_fast<L, q>(a0, r0, u, uc2, p, m);
-            f[q] = __fmaf_rn(om1, f[q], p);
-            f[q + 1] = __fmaf_rn(om1, f[q + 1], m);
+            f[q] = vfma(om1, f[q], p);
+            f[q + 1] = vfma(om1, f[q + 1], m);
         });
     } else if constexpr (COLL == LBM_TRT) {
         // TRT (collision.mojo:49-113), tau_asymm = 1/2 + Lambda / (tau - 1/2)
         // (steps/collide.mojo:214-215): symmetric part relaxed at 1/tau, antisymmetric at 1/tau_a
-        const float os = rcp_approx(tau_l);
-        const float tm = tau_l - 0.5f;
-        const float oa = tm * rcp_approx(__fmaf_rn(0.5f, tm, a.trt_lambda));  // 1 / (1/2 + Lambda / tm)
-        const float a0 = os * S * r1, r0s = os * S * rho, r0a = oa * S * rho;
-        const float hs = 0.5f * os, ha = 0.5f * oa;
-        f[0] = __fmaf_rn(1.f - os, f[0], wf<L>(0) * a0);
+        const V os = rcp_approx(tau_l);
+        const V tm = tau_l - 0.5f;
+        const V oa = tm * rcp_approx(vfma(tm, 0.5f, a.trt_lambda));  // 1 / (1/2 + Lambda / tm)
+        const V a0 = stored(os) * r1, r0s = stored(os) * rho, r0a = stored(oa) * rho;
+        const V hs = os * 0.5f, ha = oa * 0.5f;
+        f[0] = vfma(splat<V>(1.f) - os, f[0], a0 * wf<L>(0));
         static_for<0, NP>([&](auto pc) {
             constexpr int q = 2 * pc.value + 1;
             constexpr float w = wf<L>(q);
-            const float eu = edot_fast<L, q>(u);
-            float e2;
-            if constexpr (nnz_of<L, q>() == 1) {
-                constexpr int d0 = L::c(q, 0) != 0 ? 0 : (L::c(q, 1) != 0 ? 1 : 2);
-                e2 = uc2[d0];
-            } else {
-                e2 = eu * eu;
-            }
+            const V eu = edot_fast<L, q>(u);
+            const V e2 = edot2_fast<L, q>(eu, uc2);
             // os (f_s - feq_s) with f_s = (f_q + f_o) / 2, feq_s = w (r1 + 4.5 rho e2);
             // oa (f_a - feq_a) with f_a = (f_q - f_o) / 2, feq_a = 3 w rho eu
-            const float sym = __fmaf_rn(hs, ps[pc.value], -__fmaf_rn((4.5f * w) * r0s, e2, w * a0));
-            const float asy = __fmaf_rn(ha, pd[pc.value], -((3.f * w) * r0a) * eu);
+            const V sym = vfma(hs, ps[pc.value], vfma(r0s * (-4.5f * w), e2, a0 * -w));
+            const V asy = vfma(ha, pd[pc.value], r0a * (-3.f * w) * eu);
             f[q] = (f[q] - sym) - asy;
             f[q + 1] = (f[q + 1] - sym) + asy;
         });
     } else if constexpr (COLL == LBM_RLBM) {
         // RLBM (collision.mojo:168-223): f' = f_eq + (1 - 1/tau) w / (2 cs^4) H : Pi_neq
-        const float om = LES ? rcp_approx(tau_l) : a.inv_tau;
-        const float g = (1.f - om) * S;
-        const float a0 = S * r1, r0 = S * rho;
+        V g;
+        if constexpr (LES) g = stored(splat<V>(1.f) - rcp_approx(tau_l));
+        else g = splat<V>((1.f - a.inv_tau) * S);
+        const V a0 = stored(r1), r0 = stored(rho);
         // rest direction: H = -cs^2 delta: H : Pi = -(Pxx + Pyy (+ Pzz)) / 3
         {
-            float tr = P[0] + P[L::D == 2 ? 2 : 3];
-            if constexpr (L::D == 3) tr += P[5];
+            V tr = P[0] + P[L::D == 2 ? 2 : 3];
+            if constexpr (L::D == 3) tr = tr + P[5];
             constexpr float k0 = (float)(L::wd(0) / (2.0 / 9.0));
-            f[0] = __fmaf_rn((k0 * g) * (float)(-1.0 / 3.0), tr, wf<L>(0) * a0);
+            f[0] = vfma(g * k0 * (float)(-1.0 / 3.0), tr, a0 * wf<L>(0));
         }
         static_for<0, NP>([&](auto pc) {
             constexpr int q = 2 * pc.value + 1;
-            float dot = 0.f;
+            V dot = splat<V>(0.f);
             bool first = true;
             static_for<0, NS>([&](auto nc) {
                 constexpr int n = nc.value, A = sa<L>(n), B = sb<L>(n);
                 constexpr float Qn = (A == B) ? (float)(L::c(q, A) * L::c(q, B)) - (float)(1.0 / 3.0)
                                               : (float)(2 * L::c(q, A) * L::c(q, B));
                 if constexpr (Qn != 0.f) {
-                    dot = first ? Qn * P[n] : __fmaf_rn(Qn, P[n], dot);
+                    dot = first ? P[n] * Qn : vfma(P[n], Qn, dot);
                     first = false;
                 }
             });
             constexpr float kq = (float)(L::wd(q) / (2.0 / 9.0));
-            float p, m;
+            V p, m;
             feq_pair_fast<L, q>(a0, r0, u, uc2, p, m);
-            const float t = (kq * g) * dot;
+            const V t = mul_apart(g * kq, dot);
             f[q] = p + t;
             f[q + 1] = m + t;
         });
@@ -245,37 +251,48 @@ __device__ __forceinline__ void collide_fast(float (&f)[L::Q], const StepArgs& a
         // One pass over the directions computes f_eq and ds once: dh goes to this thread's
         // lane-fastest slots of shared memory, f_eq + (1 - 2 beta) ds stays in f; once gamma is
         // known the update adds (1 - beta gamma) dh.
-        __shared__ float dh_keep[Q][256];
+        __shared__ V dh_keep[Q][256 * sizeof(float) / sizeof(V)];
         const uint32_t slot = threadIdx.x;
-        const float beta = 0.5f * rcp_approx(tau_l);
-        const float inv_beta = 2.f * tau_l;
-        const float cds = __fmaf_rn(-2.f, beta, 1.f);
-        const float a0u = rho * __fmaf_rn(-1.5f, uu, 1.f);  // unshifted: rho (1 - 1.5 uu)
-        float sp1 = 0.f, sp2 = 0.f;
-        auto visit = [&](auto qc, float fe0) {
+        const V beta = rcp_approx(tau_l) * 0.5f;
+        const V inv_beta = tau_l * 2.f;
+        const V cds = vfma(beta, -2.f, 1.f);
+        const V a0u = rho * vfma(uu, -1.5f, 1.f);  // unshifted: rho (1 - 1.5 uu)
+        V sp1 = splat<V>(0.f), sp2 = splat<V>(0.f);
+        auto visit = [&](auto qc, V fe0) {
             constexpr int q = decltype(qc)::value;
             constexpr float w = wf<L>(q);
-            const float ds = kbc_shear<L, q>(P);
-            const float fe = __fmaf_rn(-w, ddf, fe0);  // shifted: f_eq - w
-            const float dh = (f[q] - fe) - ds;
-            const float t = dh * rcp_approx(fe0);
-            sp1 = __fmaf_rn(ds, t, sp1);
-            sp2 = __fmaf_rn(dh, t, sp2);
+            const V ds = kbc_shear<L, q>(P);
+            const V fe = fe0 - w * ddf;  // shifted: f_eq - w
+            const V dh = (f[q] - fe) - ds;
+            const V t = dh * rcp_approx(fe0);
+            sp1 = vfma(ds, t, sp1);
+            sp2 = vfma(dh, t, sp2);
             dh_keep[q][slot] = dh;
-            f[q] = __fmaf_rn(cds, ds, fe);
+            f[q] = vfma(cds, ds, fe);
         };
-        visit(std::integral_constant<int, 0>{}, wf<L>(0) * a0u);
+        visit(std::integral_constant<int, 0>{}, mul_apart(a0u, wf<L>(0)));
         static_for<0, NP>([&](auto pc) {
             constexpr int q = 2 * pc.value + 1;
-            float p, m;
+            V p, m;
             feq_pair_fast<L, q>(a0u, rho, u, uc2, p, m);
             visit(std::integral_constant<int, q>{}, p);
             visit(std::integral_constant<int, q + 1>{}, m);
         });
-        const float gamma = inv_beta - ((2.f - inv_beta) * sp1) * rcp_approx(sp2 + 1e-32f);
-        const float cdh = __fmaf_rn(-beta, gamma, 1.f);
-        static_for<0, Q>([&](auto qc) { f[qc.value] = __fmaf_rn(cdh, dh_keep[qc.value][slot], f[qc.value]); });
+        const V gamma = inv_beta - mul_apart((splat<V>(2.f) - inv_beta) * sp1, rcp_approx(sp2 + 1e-32f));
+        const V cdh = vfma(beta * -1.f, gamma, splat<V>(1.f));
+        static_for<0, Q>([&](auto qc) { f[qc.value] = vfma(cdh, dh_keep[qc.value][slot], f[qc.value]); });
     }
+}
+
+// One cell.  bc_own_base, T, own_flag: the capture outputs, as collide() writes them.
+template <class L, int COLL, int LES, bool SCALED>
+__device__ __forceinline__ void collide_fast(float (&f)[L::Q], const StepArgs& a, float* bc_own_base, uint32_t T,
+                                             uint8_t own_flag, bool active = true) {
+    collide_fast_v<L, COLL, LES, SCALED, float>(f, a, [&](float rho, const float* u) {
+        if (active && a.cap_rho && (own_flag & LBM_FLAG_CAPTURE_DENSITY)) bc_own_base[(size_t)T * L::D] = rho;
+        if (active && a.cap_u && (own_flag & LBM_FLAG_CAPTURE_VELOCITY))
+            static_for<0, L::D>([&](auto dc) { bc_own_base[(size_t)T * dc.value] = u[dc.value]; });
+    });
 }
 
 }  // namespace lbm

@@ -1,6 +1,7 @@
-// The cell-pair form of the block-per-tile step (double buffer): one thread streams and collides
-// two cells that are neighbours along x, so that half of the population traffic moves as 64-bit
-// (float32) or 32-bit (Float16C) words and half of the neighbour address arithmetic is shared.
+// The cell-pair form of the block-per-tile step: one thread streams and collides two cells that are
+// neighbours along x, so that half of the population traffic moves as 64-bit (float32) or 32-bit
+// (Float16C) words, half of the neighbour address arithmetic is shared, and the fast arithmetic runs as
+// packed two-value instructions.  Double buffer, and in the fast arithmetic also the in-place method.
 //
 // A 256-cell tile with power-of-two sides and tx >= 2 is one CTA of 128 threads; thread t owns the
 // cells tA = 2t and tB = 2t + 1 of the tile, which sit at x_A (even) and x_A + 1 of one tile row.
@@ -10,16 +11,17 @@
 //   c_q.x = -1: A from x_A + 1, B from x_A + 2 (the east tile's first cell when x_A + 2 = tx).
 // The source row (y - c_q.y, z - c_q.z) is shared by up to three directions, so a D3Q19 pair
 // computes 9 row addresses and 10 west/east addresses for its 38 populations.  Every own-cell
-// access (the stores, the mid-grid bounce-back reload) is one word per direction.
+// access (the stores, the mid-grid bounce-back reload) is one word per direction.  In place, the own
+// slots are words and the slots at x + c_q (the positive direction of each pair) are found the same
+// way, for the loads and for the stores.
 //
-// Everything else is the per-cell code of tile_step (lbm_step.cuh), applied to A and B in turn:
-// the same mid-grid bounce-back on the cell-solid masks, moving wall, equilibrium boundary,
-// collision and capture, so the results are those of step_kernel_tile bit for bit (the exact
-// build) or to its tolerance (the fast build).  A warp owns the warp boxes 2w and 2w + 1 of the
+// Everything else is the per-cell code of tile_step (lbm_step.cuh), applied to A and B in turn or to
+// both at once with the same operations: the results are those of step_kernel_tile bit for bit (the
+// exact build) or word for word (the fast build).  A warp owns the warp boxes 2w and 2w + 1 of the
 // tile (its 64 cells); it takes the all-fluid branch when both boxes' mask bits are clear.
 //
 // Requirements: the population buffers 8-byte aligned (the host falls back to the per-cell kernel
-// otherwise), tx >= 2, the double-buffer method, no learned closure.
+// otherwise), tx >= 2, no learned closure.
 #pragma once
 
 #include "lbm_step.cuh"
@@ -36,23 +38,32 @@ template <bool SCALED> struct PairWord<false, SCALED> {
         a = v.x;
         b = v.y;
     }
+    static __device__ __forceinline__ void ld_rw(const float* p, float& a, float& b) {
+        const float2 v = *reinterpret_cast<const float2*>(p);
+        a = v.x;
+        b = v.y;
+    }
     static __device__ __forceinline__ void st(float* p, float a, float b) {
         *reinterpret_cast<float2*>(p) = make_float2(a, b);
     }
 };
 template <bool SCALED> struct PairWord<true, SCALED> {
-    // low half: A's code, high half: B's (little-endian).  The high code arrives sign-extended by
-    // an arithmetic shift; the low one by shifting it to the top first.
-    static __device__ __forceinline__ void ld(const uint16_t* p, float& a, float& b) {
-        const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p));
-        const int32_t lo = (int32_t)(w << 16) >> 16, hi = (int32_t)w >> 16;
+    // low half: A's code, high half: B's (little-endian)
+    static __device__ __forceinline__ void decode(uint32_t w, float& a, float& b) {
         if constexpr (SCALED) {
-            a = f16c_decode_scaled_sx(lo);
-            b = f16c_decode_scaled_sx(hi);
+            // an arithmetic shift by 4 puts a code's magnitude at bits 12..26 and leaves its sign at 31
+            a = as_f32((uint32_t)((int32_t)(w << 16) >> 4) & 0x87FFF000u);
+            b = as_f32((uint32_t)((int32_t)w >> 4) & 0x87FFF000u);
         } else {
-            a = f16c_decode_sx(lo);
-            b = f16c_decode_sx(hi);
+            a = f16c_decode_sx((int32_t)(w << 16) >> 16);
+            b = f16c_decode_sx((int32_t)w >> 16);
         }
+    }
+    static __device__ __forceinline__ void ld(const uint16_t* p, float& a, float& b) {
+        decode(__ldg(reinterpret_cast<const uint32_t*>(p)), a, b);
+    }
+    static __device__ __forceinline__ void ld_rw(const uint16_t* p, float& a, float& b) {
+        decode(*reinterpret_cast<const uint32_t*>(p), a, b);
     }
     static __device__ __forceinline__ void st(uint16_t* p, float a, float b) {
         uint32_t w;
@@ -97,12 +108,25 @@ __device__ __forceinline__ void pair_deltas(const StepArgs& a, uint32_t bx, uint
     }
 }
 
+// Does the fast arithmetic work on both cells at once (F2)?  In lockstep they need the registers of two
+// collisions at a time: TRT in double buffer or on D3Q19, and Smagorinsky SRT on D3Q19, spill at any
+// occupancy that pays and take the cells in turn.  Float16C, us a step, packed / in turn: 160^3 D3Q19
+// double buffer SRT 66.5 / 70.5, SRT with LES 81.7 / 80.1, TRT 81.4 / 77.3; 2048^2 D2Q9 double buffer SRT
+// 36.5 / 38.5, SRT with LES 40.6 / 44.9, TRT 39.6 / 38.7; 144^3 D3Q27 in place, SRT with LES 93.9 / 100.1,
+// TRT 86.7 / 90.7; 2048^2 D2Q9 in place TRT 32.3 / 35.4.
+template <class L, int METHOD, int COLL, int LES, bool FAST>
+constexpr bool pair_packed() {
+    if (!FAST) return false;
+    if (L::Q == 19) return COLL != LBM_TRT && (!LES || COLL != LBM_SRT);
+    return COLL != LBM_TRT || METHOD == LBM_ESOTERIC_PULL;
+}
+
 // The two cells of one thread.  GENERAL = false is the all-fluid form (the warp's two boxes hold
 // no flag and pull from no flagged cell): no flag is read, both cells are active and the code is
 // straight-line from the loads to the stores, so the scheduler interleaves the two collisions.
 // GENERAL = true takes the masks of both cells, m (x, y of A, z, w of B; 0 in a box without a flag), and
 // handles them as tile_step does.
-template <class L, bool F16C, int COLL, int LES, bool FAST, bool GENERAL>
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool GENERAL>
 __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t tile, const uint32_t t,
                                            const uint4 m, const uint32_t bx, const uint32_t by,
                                            const uint32_t bz) {
@@ -110,11 +134,17 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
     using S = typename P::T;
     constexpr int Q = L::Q, D = L::D, K = D + 1;
     constexpr uint32_t T = kTileCells;
+    constexpr bool ESO = METHOD == LBM_ESOTERIC_PULL;
     constexpr bool SCALED = FAST && F16C && !LES && COLL != LBM_KBC;
     using W = PairWord<F16C, SCALED>;
     auto ld = [](const S* p) -> float {
-        if constexpr (SCALED) return P::ld_scaled(p);
-        else return P::ld(p);
+        if constexpr (ESO) {
+            if constexpr (SCALED) return P::ld_rw_scaled(p);
+            else return P::ld_rw(p);
+        } else {
+            if constexpr (SCALED) return P::ld_scaled(p);
+            else return P::ld(p);
+        }
     };
     auto st = [](S* p, float v) {
         if constexpr (SCALED) P::st_scaled(p, v);
@@ -144,25 +174,44 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
 
     // ---- stream: pull loads of both cells
     float fa[Q], fb[Q];
-    static_for<0, Q>([&](auto qc) {
-        constexpr int q = qc.value;
-        constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
-        // the source row at x_A: one 64-bit address per row (shared by its directions, whose q*T
-        // are immediate offsets) and one per x edge
-        const S* row = fin + (own + dy[sy + 1] + dz[sz + 1]);
-        constexpr int32_t qT = (int32_t)(T * q);
+    // a population slot of both cells at the neighbour (SX, .., ..) of the row `p` (at x_A)
+    auto ld2 = [&](const S* p, auto sxc, float& va, float& vb) {
+        constexpr int sx = decltype(sxc)::value;
         if constexpr (sx == 0) {
-            W::ld(row + qT, fa[q], fb[q]);
+            if constexpr (ESO) W::ld_rw(p, va, vb);
+            else W::ld(p, va, vb);
         } else if constexpr (sx < 0) {
-            fa[q] = ld(row + dxm + qT);
-            fb[q] = ld(row + qT);
+            va = ld(p + dxm);
+            vb = ld(p);
         } else {
-            fa[q] = ld(row + (qT + 1));
-            fb[q] = ld(row + dxp + (qT + 1));
+            va = ld(p + 1);
+            vb = ld(p + dxp + 1);
         }
-    });
+    };
+    // even: pos from (x, pos), neg from (x + c_pos, neg); odd: pos from (x, neg), neg from
+    // (x + c_pos, pos).  Slot pos + 1 = neg, so the parity folds into two base pointers.
+    [[maybe_unused]] const bool ev = a.even != 0;
+    if constexpr (!ESO) {
+        static_for<0, Q>([&](auto qc) {
+            constexpr int q = qc.value;
+            constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
+            // the source row at x_A: one 64-bit address per row (shared by its directions, whose q*T
+            // are immediate offsets) and one per x edge
+            ld2(fin + (own + dy[sy + 1] + dz[sz + 1]) + (int32_t)(T * q), std::integral_constant<int, sx>{}, fa[q], fb[q]);
+        });
+    } else {
+        const S* finA = fin + (ev ? 0u : T);
+        const S* finB = fin + (ev ? T : 0u);
+        W::ld_rw(fin + own, fa[0], fb[0]);
+        static_for<1, Q - 1, 2>([&](auto qc) {
+            constexpr int pos = qc.value, neg = pos + 1;
+            constexpr int sx = L::c(pos, 0), sy = L::c(pos, 1), sz = L::c(pos, 2);
+            W::ld_rw(finA + own + (int32_t)(T * pos), fa[pos], fb[pos]);
+            ld2(finB + (own + dy[sy + 1] + dz[sz + 1]) + (int32_t)(T * pos), std::integral_constant<int, sx>{}, fa[neg], fb[neg]);
+        });
+    }
 
-    if constexpr (GENERAL) {
+    if constexpr (GENERAL && !ESO) {
         // mid-grid bounce-back on a raw SOLID compare (ops/load_and_store.mojo:216); selecting the
         // address before the pull, as the per-cell kernels do, was slower here (393.3 against 389.8 us a
         // step of the 256^3 float32 cavity, 269.9 against 262.1 in Float16C)
@@ -217,37 +266,66 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
         }
     }
 
-    // ---- collide each cell
+    // ---- collide: both cells at once by packed instructions (a cell that is not stepped goes along and is
+    // not stored), or one after the other
     float* bcA = a.bc + (tA + (uint64_t)T * K * tile);
-    S* po = fout + own;
-    if constexpr (!GENERAL) {
-        if constexpr (FAST) {
-            collide_fast<L, COLL, LES, SCALED>(fa, a, bcA, T, 0);
-            collide_fast<L, COLL, LES, SCALED>(fb, a, bcA + 1, T, 0);
-        } else {
-            collide<L, COLL, LES>(fa, a.tau, a, bcA, T, 0);
-            collide<L, COLL, LES>(fb, a.tau, a, bcA + 1, T, 0);
-        }
-        static_for<0, Q>([&](auto qc) { W::st(po + (int32_t)(T * qc.value), fa[qc.value], fb[qc.value]); });
-        return;
-    }
-    if (actA) {
-        if constexpr (FAST) collide_fast<L, COLL, LES, SCALED>(fa, a, bcA, T, flagA);
-        else collide<L, COLL, LES>(fa, a.tau, a, bcA, T, flagA);
-    }
-    if (actB) {
-        if constexpr (FAST) collide_fast<L, COLL, LES, SCALED>(fb, a, bcA + 1, T, flagB);
-        else collide<L, COLL, LES>(fb, a.tau, a, bcA + 1, T, flagB);
+    if constexpr (pair_packed<L, METHOD, COLL, LES, FAST>()) {
+        F2 f[Q];
+        static_for<0, Q>([&](auto qc) { f[qc.value] = F2{fa[qc.value], fb[qc.value]}; });
+        collide_fast_v<L, COLL, LES, SCALED, F2>(f, a, [&](F2 rho, const F2* u) {
+            if constexpr (GENERAL) {
+                auto keep = [&](bool act, uint32_t flag, float* bc, float r, auto&& comp) {
+                    if (act && a.cap_rho && (flag & LBM_FLAG_CAPTURE_DENSITY)) bc[(size_t)T * D] = r;
+                    if (act && a.cap_u && (flag & LBM_FLAG_CAPTURE_VELOCITY))
+                        static_for<0, D>([&](auto dc) { bc[(size_t)T * dc.value] = comp(dc); });
+                };
+                keep(actA, flagA, bcA, rho.x, [&](auto dc) { return u[decltype(dc)::value].x; });
+                keep(actB, flagB, bcA + 1, rho.y, [&](auto dc) { return u[decltype(dc)::value].y; });
+            }
+        });
+        static_for<0, Q>([&](auto qc) {
+            fa[qc.value] = f[qc.value].x;
+            fb[qc.value] = f[qc.value].y;
+        });
+    } else if constexpr (FAST) {
+        if (!GENERAL || actA) collide_fast<L, COLL, LES, SCALED>(fa, a, bcA, T, flagA);
+        if (!GENERAL || actB) collide_fast<L, COLL, LES, SCALED>(fb, a, bcA + 1, T, flagB);
+    } else {
+        if (!GENERAL || actA) collide<L, COLL, LES>(fa, a.tau, a, bcA, T, flagA);
+        if (!GENERAL || actB) collide<L, COLL, LES>(fb, a.tau, a, bcA + 1, T, flagB);
     }
 
-    // ---- store: one word per direction, or the active cell's half
-    if (actA && actB) {
-        static_for<0, Q>([&](auto qc) { W::st(po + (int32_t)(T * qc.value), fa[qc.value], fb[qc.value]); });
-    } else if (actA) {
-        static_for<0, Q>([&](auto qc) { st(po + (int32_t)(T * qc.value), fa[qc.value]); });
-    } else {
-        static_for<0, Q>([&](auto qc) { st(po + 1 + (int32_t)(T * qc.value), fb[qc.value]); });
-    }
+    // ---- store: one word per direction, or the active cell's half (mode 0: both, 1: A, 2: B)
+    auto store = [&](auto mode) {
+        constexpr int MODE = decltype(mode)::value;
+        auto st2 = [&](S* p, auto sxc, float va, float vb) {
+            constexpr int sx = decltype(sxc)::value;
+            if constexpr (sx == 0 && MODE == 0) {
+                W::st(p, va, vb);
+            } else {
+                if constexpr (MODE != 2) st(sx == 0 ? p : sx < 0 ? p + dxm : p + 1, va);
+                if constexpr (MODE != 1) st(sx == 0 ? p + 1 : sx < 0 ? p : p + dxp + 1, vb);
+            }
+        };
+        constexpr std::integral_constant<int, 0> here{};
+        if constexpr (!ESO) {
+            static_for<0, Q>([&](auto qc) { st2(fout + own + (int32_t)(T * qc.value), here, fa[qc.value], fb[qc.value]); });
+        } else {
+            // the slots that were loaded, pos and neg exchanged
+            S* foA = fout + (ev ? 0u : T);
+            S* foB = fout + (ev ? T : 0u);
+            st2(fout + own, here, fa[0], fb[0]);
+            static_for<1, Q - 1, 2>([&](auto qc) {
+                constexpr int pos = qc.value, neg = pos + 1;
+                constexpr int sx = L::c(pos, 0), sy = L::c(pos, 1), sz = L::c(pos, 2);
+                st2(foB + (own + dy[sy + 1] + dz[sz + 1]) + (int32_t)(T * pos), std::integral_constant<int, sx>{}, fa[pos], fb[pos]);
+                st2(foA + own + (int32_t)(T * pos), here, fa[neg], fb[neg]);
+            });
+        }
+    };
+    if (!GENERAL || (actA && actB)) store(std::integral_constant<int, 0>{});
+    else if (actA) store(std::integral_constant<int, 1>{});
+    else store(std::integral_constant<int, 2>{});
 }
 
 // Resident CTAs (of 128 threads) per SM the pair kernels are built for: the populations of two
@@ -268,17 +346,21 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
 #ifndef LBM_PAIR_MIN_BLOCKS_HEAVY
 #define LBM_PAIR_MIN_BLOCKS_HEAVY 4
 #endif
-template <class L, bool F16C, int COLL, bool FAST>
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST>
 constexpr int pair_min_blocks() {
+    if constexpr (FAST) {
+        if (COLL == LBM_KBC || L::Q == 27) return LBM_PAIR_MIN_BLOCKS_HEAVY;
+        if (COLL == LBM_TRT) return L::Q == 9 && METHOD == LBM_ESOTERIC_PULL ? 7 : 6;
+        return L::Q == 19 && METHOD == LBM_ESOTERIC_PULL ? 7 : LBM_PAIR_MIN_BLOCKS_F16C_FAST;
+    }
     return (COLL == LBM_KBC || L::Q == 27) ? LBM_PAIR_MIN_BLOCKS_HEAVY
            : COLL == LBM_TRT               ? 6
-           : (F16C && FAST)                ? LBM_PAIR_MIN_BLOCKS_F16C_FAST
            : F16C                          ? LBM_PAIR_MIN_BLOCKS_F16C
                                            : LBM_PAIR_MIN_BLOCKS;
 }
 
-template <class L, bool F16C, int COLL, int LES, bool FAST>
-__global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, F16C, COLL, FAST>())) step_kernel_pair(const StepArgs a) {
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST>
+__global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, METHOD, F16C, COLL, LES, FAST>())) step_kernel_pair(const StepArgs a) {
     static_assert(LES != kLesLearned, "the learned closure runs in step_kernel_learned");
     const uint32_t tile = blockIdx.x, t = threadIdx.x;
     pdl_wait_before_masks(a);
@@ -293,19 +375,17 @@ __global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, F16C, COLL, 
     const uint32_t bx = tile - byz * (uint32_t)a.lay.ntx;
     const uint32_t bz = a.lay.d_nty.div(byz);
     const uint32_t by = byz - bz * (uint32_t)a.lay.nty;
-    if (!general) pair_cells<L, F16C, COLL, LES, FAST, false>(a, tile, t, m, bx, by, bz);
-    else pair_cells<L, F16C, COLL, LES, FAST, true>(a, tile, t, m, bx, by, bz);
+    if (!general) pair_cells<L, METHOD, F16C, COLL, LES, FAST, false>(a, tile, t, m, bx, by, bz);
+    else pair_cells<L, METHOD, F16C, COLL, LES, FAST, true>(a, tile, t, m, bx, by, bz);
 }
 
 template <class L, int METHOD, bool F16C, int COLL, int LES>
 cudaError_t launch_step_pair(const StepArgs& a, int, cudaStream_t s) {
-    static_assert(METHOD == LBM_DOUBLE_BUFFER, "the cell-pair kernel is double-buffer only");
-    return launch_pdl(step_kernel_pair<L, F16C, COLL, LES, false>, a.lay.ncells / kTileCells, kPairThreads, s, a);
+    return launch_pdl(step_kernel_pair<L, METHOD, F16C, COLL, LES, false>, a.lay.ncells / kTileCells, kPairThreads, s, a);
 }
 template <class L, int METHOD, bool F16C, int COLL, int LES>
 cudaError_t launch_step_pair_fast(const StepArgs& a, int, cudaStream_t s) {
-    static_assert(METHOD == LBM_DOUBLE_BUFFER, "the cell-pair kernel is double-buffer only");
-    return launch_pdl(step_kernel_pair<L, F16C, COLL, LES, true>, a.lay.ncells / kTileCells, kPairThreads, s, a);
+    return launch_pdl(step_kernel_pair<L, METHOD, F16C, COLL, LES, true>, a.lay.ncells / kTileCells, kPairThreads, s, a);
 }
 
 }  // namespace lbm

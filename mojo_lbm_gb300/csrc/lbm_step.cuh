@@ -201,31 +201,80 @@ __device__ __forceinline__ void for_each_feq(float rho, const float* u, float uu
     else feq_visit<L, false, BOTH>(rho, u, uu, fn);
 }
 
+// Two float32 values that one packed instruction works on (add / sub / mul / fma .f32x2, sm_100 on), each
+// rounded as the scalar instruction rounds it.  One issue slot does the arithmetic of two cells.
+// The assembler contracts a packed mul.rn whose only use is a packed add.rn or sub.rn into one fma
+// (with --fmad=false as well; it leaves scalar .rn instructions alone), so a product that is not exact
+// and is added or subtracted as it is takes mul_apart.
+struct F2 {
+    float x, y;
+};
+__device__ __forceinline__ uint64_t f2_bits(F2 a) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ F2 f2_of(uint64_t r) {
+    F2 a;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+    return a;
+}
+#define LBM_F2_OP(NAME, INSTR)                                                                        \
+    __device__ __forceinline__ F2 NAME(F2 a, F2 b) {                                                  \
+        uint64_t r;                                                                                   \
+        asm(INSTR " %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));                       \
+        return f2_of(r);                                                                              \
+    }
+LBM_F2_OP(operator+, "add.rn.f32x2")
+LBM_F2_OP(operator-, "sub.rn.f32x2")
+LBM_F2_OP(operator*, "mul.rn.f32x2")
+#undef LBM_F2_OP
+template <class V>
+__device__ __forceinline__ V splat(float c) {
+    if constexpr (std::is_same_v<V, float>) return c;
+    else return F2{c, c};
+}
+__device__ __forceinline__ F2 operator*(F2 a, float c) { return a * F2{c, c}; }
+__device__ __forceinline__ F2 operator+(F2 a, float c) { return a + F2{c, c}; }
+__device__ __forceinline__ F2 operator-(F2 a, float c) { return a - F2{c, c}; }
+__device__ __forceinline__ float mul_apart(float a, float b) { return a * b; }
+__device__ __forceinline__ F2 mul_apart(F2 a, F2 b) { return F2{a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ F2 mul_apart(F2 a, float b) { return F2{a.x * b, a.y * b}; }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
+    return f2_of(r);
+}
+__device__ __forceinline__ F2 vfma(F2 a, float b, F2 c) { return vfma(a, F2{b, b}, c); }
+__device__ __forceinline__ F2 vfma(F2 a, float b, float c) { return vfma(a, F2{b, b}, F2{c, c}); }
+__device__ __forceinline__ F2 vfma(F2 a, F2 b, float c) { return vfma(a, b, F2{c, c}); }
+
 // KBC shear part of the deviatoric non-equilibrium stress.  D2Q9 is get_shear_D2Q9
 // (src/lbm/kernels/ops/collisions/KBC_.mojo:137-175); the 3D form is the same projection for
 // D3Q19/D3Q27 (Karlin, Bösch, Chikatamarla, PRE 90, 031302, 2014).
-template <class L, int q>
-__device__ __forceinline__ float kbc_shear(const float* P) {
+template <class L, int q, class V>
+__device__ __forceinline__ V kbc_shear(const V* P) {
     constexpr int cx = L::c(q, 0), cy = L::c(q, 1), cz = L::c(q, 2);
     constexpr int nnz = (cx != 0) + (cy != 0) + (cz != 0);
     if constexpr (L::D == 2) {
-        const float N = P[0] - P[2];
-        if constexpr (nnz == 1) return cx != 0 ? N * 0.25f : -N * 0.25f;
-        else if constexpr (nnz == 2) return (cx * cy > 0) ? P[1] * 0.25f : -P[1] * 0.25f;
-        else return 0.f;
+        const V N = P[0] - P[2];
+        if constexpr (nnz == 1) return N * (cx != 0 ? 0.25f : -0.25f);
+        else if constexpr (nnz == 2) return P[1] * ((cx * cy > 0) ? 0.25f : -0.25f);
+        else return splat<V>(0.f);
     } else {
         if constexpr (nnz == 1) {
-            const float Nxz = P[0] - P[5], Nyz = P[3] - P[5];
+            const V Nxz = P[0] - P[5], Nyz = P[3] - P[5];
             constexpr float sixth = (float)(1.0 / 6.0);
-            if constexpr (cx != 0) return (2.f * Nxz - Nyz) * sixth;
-            else if constexpr (cy != 0) return (2.f * Nyz - Nxz) * sixth;
-            else return (-Nxz - Nyz) * sixth;
+            if constexpr (cx != 0) return mul_apart(Nxz * 2.f - Nyz, sixth);
+            else if constexpr (cy != 0) return mul_apart(Nyz * 2.f - Nxz, sixth);
+            else return mul_apart(Nxz + Nyz, -sixth);
         } else if constexpr (nnz == 2) {
-            if constexpr (cz == 0) return (float)(cx * cy) * P[1] * 0.25f;
-            else if constexpr (cy == 0) return (float)(cx * cz) * P[2] * 0.25f;
-            else return (float)(cy * cz) * P[4] * 0.25f;
+            if constexpr (cz == 0) return P[1] * (0.25f * (float)(cx * cy));
+            else if constexpr (cy == 0) return P[2] * (0.25f * (float)(cx * cz));
+            else return P[4] * (0.25f * (float)(cy * cz));
         } else {
-            return 0.f;
+            return splat<V>(0.f);
         }
     }
 }
@@ -1502,9 +1551,11 @@ cudaError_t launch_step_learned(const StepArgs& a, int, cudaStream_t s) {
 
 inline int step_index(int method, int f16c, int coll, int les) { return ((method * 2 + f16c) * 4 + coll) * 2 + les; }
 
-// Tables of the 16 double-buffer variants of one lattice (the cell-pair and fused-link kernels),
+// Tables of the 16 double-buffer or esoteric-pull variants of one lattice (the cell-pair and fused-link kernels),
 // indexed by (f16c*4 + collision)*2 + les.
 #define LBM_DB_TABLE(FN, L) {LBM_STEP_ROW(FN, L, LBM_DOUBLE_BUFFER, false), LBM_STEP_ROW(FN, L, LBM_DOUBLE_BUFFER, true)}
+
+#define LBM_ESO_TABLE(FN, L) {LBM_STEP_ROW(FN, L, LBM_ESOTERIC_PULL, false), LBM_STEP_ROW(FN, L, LBM_ESOTERIC_PULL, true)}
 
 inline int db_index(int f16c, int coll, int les) { return (f16c * 4 + coll) * 2 + les; }
 
