@@ -295,10 +295,10 @@ lbm_status lbm_sum_link_force(lbm_handle* h, const float* link_force, int64_t n_
 lbm_status lbm_drag_force(lbm_handle* h, float* node_force, const void* f, const uint8_t* flags,
                           const int32_t* fluid_ids, int64_t n_nodes, void* stream);
 
-/* ---- batched persistent step ----
+/* ---- batched step ----
  * No counterpart in the reference, whose grid sizes are compile-time parameters
  * (src/lbm/grid.mojo:55-66), so one kernel launch steps one domain.  A batch steps many domains
- * of different sizes (same lattice and config) in one persistent launch: every 256-cell tile of
+ * of different sizes (same lattice and config) in one launch: every 256-cell tile of
  * every domain is a work unit, and each domain is stepped exactly as lbm_*_step would step it
  * (identical results).  Each grid needs a 256-cell tile with power-of-two sides and Q*N < 2^31. */
 typedef struct lbm_batch lbm_batch;

@@ -1,8 +1,8 @@
-"""Batched persistent step of many domains of different size (lbm_batch_* in the C ABI).
+"""Batched step of many domains of different size (lbm_batch_* in the C ABI).
 
 The reference's grid sizes are compile-time parameters (src/lbm/grid.mojo:55-66): one kernel
 launch steps one domain.  BatchSolver steps many domains of one lattice and config in one
-persistent launch, each exactly as Solver would step it.
+launch, each exactly as Solver would step it.
 """
 from __future__ import annotations
 

@@ -1,23 +1,32 @@
-// Batched persistent step: many domains of different size, one launch.
+// Batched step: many domains of different size, one launch.
 //
 // Each domain is a complete single-domain problem (its own grid, tiled layout, f / bc / flags
-// buffers and tau), described by a StepArgs.  The work units are the 256-cell tiles of all
-// domains, numbered consecutively domain after domain.  A fixed grid of CTAs (SMs x resident
-// CTAs) takes equal contiguous ranges of units; a CTA keeps its current domain's StepArgs in
-// shared memory, reloads it when its range crosses into the next domain, and runs the same
-// block-per-tile body (tile_step) as the single-domain kernel, so a batched step equals the
-// single-domain steps bit for bit.  Two descriptor arrays hold the even and odd step of every
-// domain (buffers swapped, esoteric parity), so the kernel only picks one.
+// buffers and tau), described by a StepArgs.  The work units are the 256-cell tiles of all domains,
+// numbered consecutively domain after domain; a CTA steps a few consecutive ones.  It looks its domain
+// up in a table (one word per unit), brings the domain's StepArgs into shared memory, reads the first
+// unit's masks and only then waits for the previous kernel (programmatic dependent launch), so that
+// this overlaps it; each unit runs the body of the single-domain kernel (pair_cells on large double-buffer
+// batches other than KBC and D3Q27, else tile_cell), and a batched step equals the single-domain steps
+// bit for bit.  Two descriptor arrays hold the even and odd step of every domain (buffers swapped,
+// esoteric parity), so the kernel only picks one.
+// 128 cylinder channels (14.9 M D2Q9 float32 cells, links included; floor 158 us): 226 us a step with one
+// persistent CTA per slot walking 76 units a cell per thread, 213 us with the short walks, 190 us with
+// cell pairs.  Bound by issue and by the warps next to walls (a narrow channel has them everywhere).
 #pragma once
 
 #include "lbm_aux.cuh"
+#include "lbm_pair.cuh"
 
 namespace lbm {
 
 struct BatchArgs {
     const StepArgs* dom;          // ndom descriptors for this step's parity
     const uint32_t* unit_begin;   // ndom + 1 offsets of the domains' first tile units
+    const uint32_t* unit_domain;  // the domain of each unit
     uint32_t ndom, total_units;
+    uint32_t per_cta;             // consecutive units of one CTA
+    int32_t ready;                // the kernel before this one is part of the same run (its descriptors and
+                                  // masks are complete)
 };
 
 __device__ __forceinline__ uint32_t find_domain(const uint32_t* begin, uint32_t ndom, uint32_t u) {
@@ -38,33 +47,77 @@ constexpr int batch_min_blocks() {
     else return (L::Q == 9) ? 5 : ((COLL == LBM_KBC || L::Q == 27) ? 3 : 4);
 }
 
+// A CTA's walk over its units: the descriptor of the current unit's domain in shared memory (reloaded
+// where the range crosses into the next domain) and the unit's tile in that domain.
+struct BatchWalk {
+    uint32_t u, end, first, next;  // unit, end of the range, units of the current domain: [first, next)
+    __device__ __forceinline__ BatchWalk(const BatchArgs& b) {
+        u = blockIdx.x * b.per_cta;
+        end = min(u + b.per_cta, b.total_units);
+        first = next = 0u;
+    }
+    __device__ __forceinline__ uint32_t tile(const BatchArgs& b, StepArgs* sa) {
+        if (u >= next) {  // block-uniform
+            const uint32_t d = __ldg(b.unit_domain + u);
+            if (next != 0u) __syncthreads();  // every thread is done with the previous descriptor
+            static_assert(sizeof(StepArgs) % 4 == 0, "copied in words");
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(b.dom + d);
+            uint32_t* dst = reinterpret_cast<uint32_t*>(sa);
+            for (uint32_t i = threadIdx.x; i < sizeof(StepArgs) / 4; i += blockDim.x) {
+                uint32_t v;  // (volatile: kept behind the wait)
+                asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(src + i) : "memory");
+                dst[i] = v;
+            }
+            first = __ldg(b.unit_begin + d);
+            next = __ldg(b.unit_begin + d + 1);
+            __syncthreads();
+        }
+        return u - first;
+    }
+};
+
 template <class L, int METHOD, bool F16C, int COLL, int LES, bool LINKS = false>
 __global__ void __launch_bounds__(256, (batch_min_blocks<L, COLL, LINKS>())) step_kernel_batch(const BatchArgs b) {
     __shared__ StepArgs sa;
-    // a contiguous, equal share of the units per CTA: the domain changes rarely along it, so the
-    // descriptor is reloaded only when it does
-    const uint32_t per = (b.total_units + gridDim.x - 1u) / gridDim.x;
-    const uint32_t u0 = blockIdx.x * per;
-    const uint32_t u1 = min(b.total_units, u0 + per);
-    if (u0 >= u1) return;
-    uint32_t d = find_domain(b.unit_begin, b.ndom, u0);
-    uint32_t loaded = 0xffffffffu;
-    uint32_t next_begin = __ldg(b.unit_begin + d + 1);
-    for (uint32_t u = u0; u < u1; ++u) {
-        while (u >= next_begin) {  // block-uniform
-            ++d;
-            next_begin = __ldg(b.unit_begin + d + 1);
-        }
-        if (d != loaded) {  // block-uniform
-            __syncthreads();  // every thread is done with the previous descriptor
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(b.dom + d);
-            uint32_t* dst = reinterpret_cast<uint32_t*>(&sa);
-            for (uint32_t i = threadIdx.x; i < sizeof(StepArgs) / 4; i += blockDim.x) dst[i] = __ldg(src + i);
-            __syncthreads();
-            loaded = d;
-        }
-        tile_step<L, METHOD, F16C, COLL, LES, false, LINKS>(sa, u - __ldg(b.unit_begin + d), threadIdx.x);
+    if (!b.ready) asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t tid = threadIdx.x;
+    bool waited = !b.ready;
+    for (BatchWalk w(b); w.u < w.end; ++w.u) {
+        const uint32_t tile = w.tile(b, &sa);
+        const bool general = tile_general(load_near(sa.tile_near + tile), tid);
+        uint2 m = make_uint2(0u, 0u);
+        if (general) m = load_masks(sa.cell_masks + (tid + kTileCells * tile));
+        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+        waited = true;
+        tile_forms<L, METHOD, F16C, COLL, LES, false, LINKS, false>(sa, tile, tid, general, m, nullptr, nullptr, nullptr);
     }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The same with two cells per thread (double buffer).
+template <class L, bool F16C, int COLL, int LES>
+__global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, LBM_DOUBLE_BUFFER, F16C, COLL, LES, false>()))
+    step_kernel_batch_pair(const BatchArgs b) {
+    __shared__ StepArgs sa;
+    if (!b.ready) asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t t = threadIdx.x;
+    bool waited = !b.ready;
+    for (BatchWalk w(b); w.u < w.end; ++w.u) {
+        const uint32_t tile = w.tile(b, &sa);
+        const uint32_t mask = load_near(sa.tile_near + tile);
+        const bool general = !__all_sync(0xffffffffu, ((mask >> ((t >> 5) * 2u)) & 3u) == 0u);
+        uint4 m = make_uint4(0u, 0u, 0u, 0u);
+        if (general && ((mask >> (t >> 4)) & 1u)) m = load_masks2(sa.cell_masks + (2u * t + kTileCells * tile));
+        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+        waited = true;
+        const uint32_t byz = sa.lay.d_ntx.div(tile);
+        const uint32_t bx = tile - byz * (uint32_t)sa.lay.ntx;
+        const uint32_t bz = sa.lay.d_nty.div(byz);
+        const uint32_t by = byz - bz * (uint32_t)sa.lay.nty;
+        if (!general) pair_cells<L, LBM_DOUBLE_BUFFER, F16C, COLL, LES, false, false>(sa, tile, t, m, bx, by, bz);
+        else pair_cells<L, LBM_DOUBLE_BUFFER, F16C, COLL, LES, false, true>(sa, tile, t, m, bx, by, bz);
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // warp_near bit of warp box i (unit i / 8, warp i % 8) from the box summaries of its domain
@@ -107,6 +160,8 @@ struct BatchLinkArgs {
 // domains: each link carries its domain, and works on that domain's freshly written lattice.
 template <class L, bool F16C>
 __global__ void link_kernel_batch(const BatchLinkArgs b) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= b.n) return;
     const StepArgs& a = b.dom[b.domain[t]];
@@ -125,31 +180,27 @@ __global__ void link_kernel_batch(const BatchLinkArgs b) {
     link_one<L, F16C>(la, t);
 }
 
-using BatchLaunch = cudaError_t (*)(const BatchArgs&, int sms, cudaStream_t);
+using BatchLaunch = cudaError_t (*)(const BatchArgs&, cudaStream_t);
 
-template <class L, int METHOD, bool F16C, int COLL, int LES, bool LINKS = false>
-cudaError_t launch_step_batch_impl(const BatchArgs& b, int sms, cudaStream_t s) {
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, step_kernel_batch<L, METHOD, F16C, COLL, LES, LINKS>, (int)kTileCells, 0);
-        if (e != cudaSuccess) return e;
-        if (per_sm < 1) per_sm = 1;
-    }
-    uint32_t grid = (uint32_t)(sms * per_sm);
-    if (grid > b.total_units) grid = b.total_units;
-    if (grid == 0) return cudaSuccess;
-    step_kernel_batch<L, METHOD, F16C, COLL, LES, LINKS><<<grid, kTileCells, 0, s>>>(b);
-    return cudaGetLastError();
-}
+inline uint32_t batch_grid(const BatchArgs& b) { return (b.total_units + b.per_cta - 1u) / b.per_cta; }
+
 template <class L, int METHOD, bool F16C, int COLL, int LES>
-cudaError_t launch_step_batch(const BatchArgs& b, int sms, cudaStream_t s) {
-    return launch_step_batch_impl<L, METHOD, F16C, COLL, LES, false>(b, sms, s);
+cudaError_t launch_step_batch(const BatchArgs& b, cudaStream_t s) {
+    if (b.total_units == 0) return cudaSuccess;
+    return launch_pdl(step_kernel_batch<L, METHOD, F16C, COLL, LES, false>, batch_grid(b), kTileCells, s, b);
 }
 // The batched step with the links fused in (lbm_batch_set_link_mode, double buffer).
 template <class L, int METHOD, bool F16C, int COLL, int LES>
-cudaError_t launch_step_batch_links(const BatchArgs& b, int sms, cudaStream_t s) {
-    return launch_step_batch_impl<L, METHOD, F16C, COLL, LES, true>(b, sms, s);
+cudaError_t launch_step_batch_links(const BatchArgs& b, cudaStream_t s) {
+    if (b.total_units == 0) return cudaSuccess;
+    return launch_pdl(step_kernel_batch<L, METHOD, F16C, COLL, LES, true>, batch_grid(b), kTileCells, s, b);
+}
+// Two cells per thread (double buffer).
+template <class L, int METHOD, bool F16C, int COLL, int LES>
+cudaError_t launch_step_batch_pair(const BatchArgs& b, cudaStream_t s) {
+    static_assert(METHOD == LBM_DOUBLE_BUFFER, "double buffer");
+    if (b.total_units == 0) return cudaSuccess;
+    return launch_pdl(step_kernel_batch_pair<L, F16C, COLL, LES>, batch_grid(b), kPairThreads, s, b);
 }
 
 }  // namespace lbm

@@ -1,4 +1,4 @@
-// C ABI of the batched persistent step (lbm_batch_* in include/lbm_gb300.h).
+// C ABI of the batched step (lbm_batch_* in include/lbm_gb300.h).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -19,6 +19,8 @@ BatchLaunch get_batch_step_d3q27(int, int, int, int);
 BatchLaunch get_batch_links_step_d2q9(int, int, int);
 BatchLaunch get_batch_links_step_d3q19(int, int, int);
 BatchLaunch get_batch_links_step_d3q27(int, int, int);
+BatchLaunch get_batch_pair_step_d2q9(int, int, int);
+BatchLaunch get_batch_pair_step_d3q19(int, int, int);
 cudaError_t launch_link_batch_d2q9(const BatchLinkArgs&, bool, cudaStream_t);
 cudaError_t launch_link_batch_d3q19(const BatchLinkArgs&, bool, cudaStream_t);
 cudaError_t launch_link_batch_d3q27(const BatchLinkArgs&, bool, cudaStream_t);
@@ -50,6 +52,8 @@ struct lbm_batch {
     bool masks_resting = false;       // the masks are those of the last run's bc (without_resting_walls)
     bool dirty = true;
     BatchLaunch step = nullptr;
+    BatchLaunch step_pair = nullptr;   // two cells per thread (needs 8-byte aligned buffers), or null
+    uint32_t* d_unit_domain = nullptr;
     BatchLaunch step_links = nullptr;  // the step with the links fused in (double buffer), or null
     // links (caller-owned device arrays, concatenated over domains)
     const int32_t *l_dom = nullptr, *l_ids = nullptr, *l_dirs = nullptr;
@@ -65,7 +69,7 @@ struct lbm_batch {
     int32_t* d_link_id = nullptr;
     int sms = 1;
     cudaStream_t capture_stream = nullptr;
-    std::map<int, cudaGraphExec_t> graphs;  // keyed by the parity of the first step
+    std::map<int, cudaGraphExec_t> graphs;  // keyed by the parity of the first step and the step kernel
 };
 
 namespace {
@@ -80,6 +84,10 @@ lbm_status bfail(lbm_status s, const std::string& m) {
         cudaError_t e_ = (call);                                                               \
         if (e_ != cudaSuccess) return bfail(LBM_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
+
+// Units from which the batch takes the cell-pair form: one wave of its CTAs (8 per SM; 4 channels of 1,800
+// units: 11.6 us a step against 12.7 per cell).
+constexpr uint64_t kPairMinUnits = 8u * 152u;
 
 bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 int ilog2(int v) { int r = 0; while ((1 << r) < v) ++r; return r; }
@@ -142,19 +150,41 @@ lbm_status launch_links(lbm_batch* b, const StepArgs* dom, cudaStream_t s) {
 
 bool fused_links(const lbm_batch* b) { return b->link_mode == LBM_LINKS_FUSED && b->n_links > 0; }
 
-// One step of every domain: the persistent step kernel, then the link-wise bounce-back (or the
+// Two cells per thread, when every domain's populations are 8-byte aligned.
+bool use_batch_pair(const lbm_batch* b) {
+    if (!b->step_pair) return false;
+    uintptr_t al = 0;
+    for (const StepArgs& a : b->even) al |= reinterpret_cast<uintptr_t>(a.f_in) | reinterpret_cast<uintptr_t>(a.f_out);
+    return (al & 7u) == 0u;
+}
+
+// Consecutive units of a CTA: as many as leave three waves of CTAs (8 per SM), 4 at most in the cell-pair
+// form, 8 in the per-cell one.  More units share a descriptor and its load latency, fewer balance the
+// SMs (us a step of 128 / 16 / 4 channels, 58,000 / 7,200 / 1,800 units; cell pairs: 1 unit 217 / 36.2 / 11.6,
+// 2 196 / 35.3 / 12.8, 4 190 / 35.8 / 13.4, 8 195 / 40.4 / 18.4; per cell: 4 213 / 37.2 / 13.7, 8 213 / 41.6 /
+// 15.1, 16 216 / 45.2 / 21.9).
+uint32_t units_per_cta(const lbm_batch* b, bool pair) {
+    const uint32_t waves = 3u * 8u * (uint32_t)b->sms;
+    return std::max(1u, std::min(pair ? 4u : 8u, b->unit_begin.back() / waves));
+}
+
+// One step of every domain: the step kernel, then the link-wise bounce-back (or the
 // step kernel with the links fused in).
-lbm_status batch_step(lbm_batch* b, bool parity_odd, cudaStream_t s) {
+// ready: the previous kernel in the stream is part of the same run.
+lbm_status batch_step(lbm_batch* b, bool parity_odd, bool ready, cudaStream_t s) {
     BatchArgs a;
     a.dom = parity_odd ? b->d_odd : b->d_even;
+    a.ready = ready ? 1 : 0;
     a.unit_begin = b->d_begin;
+    a.unit_domain = b->d_unit_domain;
     a.ndom = (uint32_t)b->ndom;
     a.total_units = b->unit_begin.back();
+    a.per_cta = units_per_cta(b, use_batch_pair(b) && !fused_links(b));
     if (fused_links(b)) {
-        LBM_BCK(b->step_links(a, b->sms, s));
+        LBM_BCK(b->step_links(a, s));
         return LBM_OK;
     }
-    LBM_BCK(b->step(a, b->sms, s));
+    LBM_BCK((use_batch_pair(b) ? b->step_pair : b->step)(a, s));
     return launch_links(b, a.dom, s);
 }
 
@@ -259,6 +289,12 @@ lbm_status lbm_batch_create(const lbm_config_t* cfg, int32_t n_domains, const lb
                   : lat == LBM_D2Q9 ? get_batch_links_step_d2q9(f16, co, les)
                   : lat == LBM_D3Q19 ? get_batch_links_step_d3q19(f16, co, les)
                                      : get_batch_links_step_d3q27(f16, co, les);
+    // (as the single-domain choice; every tile at least two cells wide)
+    bool wide = m == LBM_DOUBLE_BUFFER && co != LBM_KBC && lat != LBM_D3Q27 && units >= kPairMinUnits;
+    for (int32_t i = 0; i < n_domains; ++i) wide = wide && grids[i].tx >= 2;
+    b->step_pair = !wide ? nullptr : lat == LBM_D2Q9 ? get_batch_pair_step_d2q9(f16, co, les) : get_batch_pair_step_d3q19(f16, co, les);
+    std::vector<uint32_t> unit_domain(units);
+    for (int32_t i = 0; i < n_domains; ++i) std::fill(unit_domain.begin() + begin[i], unit_domain.begin() + begin[i + 1], (uint32_t)i);
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
@@ -273,6 +309,9 @@ lbm_status lbm_batch_create(const lbm_config_t* cfg, int32_t n_domains, const lb
     if (e == cudaSuccess) e = cudaMemset(b->d_changed, 0, sizeof(uint32_t));
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_begin, begin.data(), sizeof(uint32_t) * (n_domains + 1), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_unit_domain, sizeof(uint32_t) * (units > 0 ? units : 1));
+    if (e == cudaSuccess && units > 0)
+        e = cudaMemcpy(b->d_unit_domain, unit_domain.data(), sizeof(uint32_t) * units, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         lbm_batch_destroy(b);
@@ -288,6 +327,7 @@ lbm_status lbm_batch_destroy(lbm_batch* b) {
     cudaFree(b->d_even);
     cudaFree(b->d_odd);
     cudaFree(b->d_begin);
+    cudaFree(b->d_unit_domain);
     cudaFree(b->d_box_sum);
     cudaFree(b->d_tile_near);
     cudaFree(b->d_flags_seen);
@@ -413,6 +453,9 @@ lbm_status lbm_batch_run(lbm_batch* b, int64_t n_steps, int64_t first_step, void
         BatchArgs a;
         a.dom = b->d_even;
         a.unit_begin = b->d_begin;
+        a.unit_domain = b->d_unit_domain;
+        a.ready = 0;
+        a.per_cta = 1;
         a.ndom = (uint32_t)b->ndom;
         a.total_units = b->unit_begin.back();
         const uint32_t nboxes = a.total_units * kTileWarps;  // < 2^32: fewer than 2^29 units
@@ -446,14 +489,14 @@ lbm_status lbm_batch_run(lbm_batch* b, int64_t n_steps, int64_t first_step, void
     const int64_t chunk = 64;
     int64_t done = 0;
     if (n_steps >= chunk) {
-        const int key = (int)(first_step % 2);
+        const int key = (int)(first_step % 2) + (use_batch_pair(b) ? 2 : 0);
         auto it = b->graphs.find(key);
         if (it == b->graphs.end()) {
             cudaGraph_t g = nullptr;
             LBM_BCK(cudaStreamBeginCapture(b->capture_stream, cudaStreamCaptureModeThreadLocal));
             lbm_status st = LBM_OK;
             for (int64_t k = 0; k < chunk && st == LBM_OK; ++k)
-                st = batch_step(b, ((first_step + k) % 2) != 0, b->capture_stream);
+                st = batch_step(b, ((first_step + k) % 2) != 0, k > 0, b->capture_stream);
             cudaError_t e = cudaStreamEndCapture(b->capture_stream, &g);
             if (st != LBM_OK || e != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
@@ -468,7 +511,7 @@ lbm_status lbm_batch_run(lbm_batch* b, int64_t n_steps, int64_t first_step, void
         for (; done + chunk <= n_steps; done += chunk) LBM_BCK(cudaGraphLaunch(it->second, s));
     }
     for (; done < n_steps; ++done) {
-        const lbm_status st = batch_step(b, ((first_step + done) % 2) != 0, s);
+        const lbm_status st = batch_step(b, ((first_step + done) % 2) != 0, done > 0, s);
         if (st != LBM_OK) return st;
     }
     return LBM_OK;

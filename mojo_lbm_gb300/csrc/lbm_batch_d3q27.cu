@@ -1,4 +1,4 @@
-// The 32 batched persistent-step variants of the D3Q27 lattice and its batched link kernel.
+// The 32 batched-step variants of the D3Q27 lattice and its batched link kernel.
 #include "lbm_batch.cuh"
 
 namespace lbm {
@@ -9,8 +9,7 @@ BatchLaunch get_batch_step_d3q27(int method, int f16c, int coll, int les) {
 
 cudaError_t launch_link_batch_d3q27(const BatchLinkArgs& b, bool f16c, cudaStream_t s) {
     const uint32_t blocks = (uint32_t)((b.n + 255) / 256);
-    if (f16c) link_kernel_batch<D3Q27, true><<<blocks, 256, 0, s>>>(b);
-    else link_kernel_batch<D3Q27, false><<<blocks, 256, 0, s>>>(b);
-    return cudaGetLastError();
+    return f16c ? launch_pdl(link_kernel_batch<D3Q27, true>, blocks, 256u, s, b)
+                : launch_pdl(link_kernel_batch<D3Q27, false>, blocks, 256u, s, b);
 }
 }  // namespace lbm

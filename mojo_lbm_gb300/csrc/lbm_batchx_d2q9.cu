@@ -1,4 +1,4 @@
-// The 16 double-buffer batched persistent-step variants of the D2Q9 lattice with the interpolated
+// The 16 double-buffer batched-step variants of the D2Q9 lattice with the interpolated
 // bounce-back fused in (lbm_batch_set_link_mode).
 #include "lbm_batch.cuh"
 
