@@ -82,7 +82,7 @@ __device__ __forceinline__ void feq_pair_fast(V a0, V r0, const V* u, const V* u
 // The collision of the fast build, in place on f (in units of 2^-112 when SCALED).  V: float, one cell,
 // or F2, two cells by packed instructions, with the same operations on each.  capture(rho, u) is called
 // with the density and velocity.
-template <class L, int COLL, int LES, bool SCALED, class V, class Capture>
+template <class L, int COLL, int LES, bool SCALED, class V, int NT = 256, class Capture>
 __device__ __forceinline__ void collide_fast_v(V (&f)[L::Q], const StepArgs& a, Capture&& capture) {
     static_assert(!(SCALED && (LES || COLL == LBM_KBC)), "scaled populations need a collision linear in f");
     constexpr int Q = L::Q, D = L::D, NP = (Q - 1) / 2, NS = L::NS;
@@ -250,8 +250,13 @@ __device__ __forceinline__ void collide_fast_v(V (&f)[L::Q], const StepArgs& a, 
         //       = f_eq + (1 - 2 beta) ds + (1 - beta gamma) dh.
         // One pass over the directions computes f_eq and ds once: dh goes to this thread's
         // lane-fastest slots of shared memory, f_eq + (1 - 2 beta) ds stays in f; once gamma is
-        // known the update adds (1 - beta gamma) dh.
-        __shared__ V dh_keep[Q][256 * sizeof(float) / sizeof(V)];
+        // known the update adds (1 - beta gamma) dh.  A single cell (V float) takes the two directions of an
+        // opposite pair, whose ds is the same, by packed instructions (256^3 D3Q27 Float16C cavity, with
+        // LES, us a step, one direction at a time / packed: in place 614.7 / 598.2, double buffer 603.7 /
+        // 571.3; bound by issue, 1061 instructions a warp at 66 % issue activity).
+        constexpr bool IN_CELL = std::is_same_v<V, float>;
+        __shared__ V dh_keep[IN_CELL ? 1 : Q][NT * sizeof(float) / sizeof(V)];
+        __shared__ F2 dh_pair[IN_CELL ? NP : 1][IN_CELL ? NT : 1];
         const uint32_t slot = threadIdx.x;
         const V beta = rcp_approx(tau_l) * 0.5f;
         const V inv_beta = tau_l * 2.f;
@@ -267,28 +272,58 @@ __device__ __forceinline__ void collide_fast_v(V (&f)[L::Q], const StepArgs& a, 
             const V t = dh * rcp_approx(fe0);
             sp1 = vfma(ds, t, sp1);
             sp2 = vfma(dh, t, sp2);
-            dh_keep[q][slot] = dh;
+            dh_keep[IN_CELL ? 0 : q][slot] = dh;
             f[q] = vfma(cds, ds, fe);
         };
         visit(std::integral_constant<int, 0>{}, mul_apart(a0u, wf<L>(0)));
-        static_for<0, NP>([&](auto pc) {
-            constexpr int q = 2 * pc.value + 1;
-            V p, m;
-            feq_pair_fast<L, q>(a0u, rho, u, uc2, p, m);
-            visit(std::integral_constant<int, q>{}, p);
-            visit(std::integral_constant<int, q + 1>{}, m);
-        });
+        if constexpr (IN_CELL) {
+            static_for<0, NP>([&](auto pc) {
+                constexpr int p = pc.value, q = 2 * p + 1;
+                constexpr float w = wf<L>(q);
+                const float eu = edot_fast<L, q>(u);
+                const float base = vfma(rho * (4.5f * w), edot2_fast<L, q>(eu, uc2), a0u * w);
+                const float c3 = rho * (3.f * w), ds = kbc_shear<L, q>(P);
+                const F2 fe0 = vfma(F2{c3, -c3}, F2{eu, eu}, F2{base, base});
+                const F2 fe = fe0 - w * ddf;  // shifted: f_eq - w
+                const F2 dh = (F2{f[q], f[q + 1]} - fe) - ds;
+                const F2 t = dh * rcp_approx(fe0);
+                sp1 = vfma(ds, t.y, vfma(ds, t.x, sp1));
+                sp2 = vfma(dh.y, t.y, vfma(dh.x, t.x, sp2));
+                dh_pair[p][slot] = dh;
+                const F2 g = vfma(F2{cds, cds}, F2{ds, ds}, fe);
+                f[q] = g.x;
+                f[q + 1] = g.y;
+            });
+        } else {
+            static_for<0, NP>([&](auto pc) {
+                constexpr int q = 2 * pc.value + 1;
+                V p, m;
+                feq_pair_fast<L, q>(a0u, rho, u, uc2, p, m);
+                visit(std::integral_constant<int, q>{}, p);
+                visit(std::integral_constant<int, q + 1>{}, m);
+            });
+        }
         const V gamma = inv_beta - mul_apart((splat<V>(2.f) - inv_beta) * sp1, rcp_approx(sp2 + 1e-32f));
         const V cdh = vfma(beta * -1.f, gamma, splat<V>(1.f));
-        static_for<0, Q>([&](auto qc) { f[qc.value] = vfma(cdh, dh_keep[qc.value][slot], f[qc.value]); });
+        if constexpr (IN_CELL) {
+            f[0] = vfma(cdh, dh_keep[0][slot], f[0]);
+            static_for<0, NP>([&](auto pc) {
+                constexpr int p = pc.value, q = 2 * p + 1;
+                const F2 g = vfma(F2{cdh, cdh}, dh_pair[p][slot], F2{f[q], f[q + 1]});
+                f[q] = g.x;
+                f[q + 1] = g.y;
+            });
+        } else {
+            static_for<0, Q>([&](auto qc) { f[qc.value] = vfma(cdh, dh_keep[qc.value][slot], f[qc.value]); });
+        }
     }
 }
 
 // One cell.  bc_own_base, T, own_flag: the capture outputs, as collide() writes them.
-template <class L, int COLL, int LES, bool SCALED>
+template <class L, int COLL, int LES, bool SCALED, int NT = 256>
 __device__ __forceinline__ void collide_fast(float (&f)[L::Q], const StepArgs& a, float* bc_own_base, uint32_t T,
                                              uint8_t own_flag, bool active = true) {
-    collide_fast_v<L, COLL, LES, SCALED, float>(f, a, [&](float rho, const float* u) {
+    collide_fast_v<L, COLL, LES, SCALED, float, NT>(f, a, [&](float rho, const float* u) {
         if (active && a.cap_rho && (own_flag & LBM_FLAG_CAPTURE_DENSITY)) bc_own_base[(size_t)T * L::D] = rho;
         if (active && a.cap_u && (own_flag & LBM_FLAG_CAPTURE_VELOCITY))
             static_for<0, L::D>([&](auto dc) { bc_own_base[(size_t)T * dc.value] = u[dc.value]; });

@@ -284,7 +284,7 @@ __device__ __forceinline__ V kbc_shear(const V* P) {
 // is false for the lanes kept alive only for it, which write nothing); the populations wait in
 // `stash` (this warp's (Q+3)/4 x 32 float4 of shared memory, lane-fastest) across the features
 // and the network, and `stash_holds_f` says the stash already holds them.
-template <class L, int COLL, int LES>
+template <class L, int COLL, int LES, int NT = 256>
 __device__ __forceinline__ void collide(float (&f)[L::Q], float tau, const StepArgs& a, float* bc_own_base,
                                         uint32_t T, uint8_t own_flag, bool active = true,
                                         const ClosureDev* cl = nullptr, float4* stash = nullptr,
@@ -478,7 +478,7 @@ __device__ __forceinline__ void collide(float (&f)[L::Q], float tau, const StepA
             // third of its usual rate on this GPU.  (dh = 0 also means ds is finite.)
             // dh of every direction waits in shared memory (lane-fastest) for the update, which
             // then needs no third f_eq per direction
-            __shared__ float dh_keep[Q][256];
+            __shared__ float dh_keep[Q][NT];
             for_each_feq<L, true>(rho, u, uu, ddf, [&](auto qc, float e, float fe0) {
                 constexpr int q = decltype(qc)::value;
                 const float ds = kbc_shear<L, q>(P);
@@ -1239,7 +1239,7 @@ __device__ __forceinline__ void fused_links(float (&f)[L::Q], const uint2 lt, co
 // GENERAL = false is the form of a warp whose cells and pull neighbours are all plain FLUID: no
 // flag is read and the code is straight-line from the loads to the stores; GENERAL = true takes the
 // cell's masks m (cell_masks_of) and handles every boundary.
-template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS, bool STAGED, bool GENERAL>
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS, bool STAGED, bool GENERAL, int NT>
 __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile, const uint32_t tid,
                                           const uint2 m, const ClosureDev* cl, float4* fbuf, const void* stage) {
     using P = Pop<F16C>;
@@ -1374,8 +1374,8 @@ __device__ __forceinline__ void tile_cell(const StepArgs& a, const uint32_t tile
         }
     }
 
-    if constexpr (FAST) collide_fast<L, COLL, LES, SCALED>(f, a, a.bc + (tid + (uint64_t)T * K * tile), T, flag);
-    else collide<L, COLL, LES>(f, a.tau, a, a.bc + (tid + (uint64_t)T * K * tile), T, flag, active, cl, fbuf);
+    if constexpr (FAST) collide_fast<L, COLL, LES, SCALED, NT>(f, a, a.bc + (tid + (uint64_t)T * K * tile), T, flag);
+    else collide<L, COLL, LES, NT>(f, a.tau, a, a.bc + (tid + (uint64_t)T * K * tile), T, flag, active, cl, fbuf);
     if constexpr (LES == kLesLearned) {
         if (!active) return;
     }
@@ -1405,11 +1405,11 @@ __device__ __forceinline__ bool tile_general(uint32_t mask, uint32_t tid) {
     return !__all_sync(0xffffffffu, ((mask >> (tid >> 5)) & 1u) == 0u);
 }
 
-template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS, bool STAGED>
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS, bool STAGED, int NT = 256>
 __device__ __forceinline__ void tile_forms(const StepArgs& a, const uint32_t tile, const uint32_t tid, const bool general,
                                            const uint2 m, const ClosureDev* cl, float4* fbuf, const void* stage) {
-    if (!general) tile_cell<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED, false>(a, tile, tid, m, cl, fbuf, stage);
-    else tile_cell<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED, true>(a, tile, tid, m, cl, fbuf, stage);
+    if (!general) tile_cell<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED, false, NT>(a, tile, tid, m, cl, fbuf, stage);
+    else tile_cell<L, METHOD, F16C, COLL, LES, FAST, LINKS, STAGED, true, NT>(a, tile, tid, m, cl, fbuf, stage);
 }
 
 template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST = false, bool LINKS = false,
@@ -1442,17 +1442,54 @@ constexpr int tile_min_blocks() {
     else return (L::Q == 9) ? 5 : (heavy ? LBM_TILE_MIN_BLOCKS_HEAVY : LBM_TILE_MIN_BLOCKS);
 }
 
+// Threads of a CTA of the block-per-tile kernels: the tile's 256 cells, or half of them.  Half CTAs retire
+// and refill in smaller pieces, so more of the warps that the registers allow are resident (KBC with 80
+// registers: 20 of 24 on average in whole CTAs), and spread few tiles more evenly over the SMs.  us a step of
+// cavities, 256 / 128 threads:
+//   256^3 D3Q27  KBC fast Float16C in place 598 / 557, float32 648 / 623, Float16C double buffer 571 / 521;
+//                others: float32 595 / 560, fast 577 / 551, TRT in place 662 / 635
+//   D3Q19        64^3 7.27 / 6.89, 96 x 64^2 fast 9.57 / 9.03; 256^3 in place 445.5 / 440.6, TRT 465 / 457,
+//                Float16C with LES 522 / 513
+//   D2Q9         64^2 1.92 / 1.85, 256^2 2.18 / 2.15, 512^2 4.24 / 4.08; KBC fast 256^2 2.18 / 1.90
+// Whole CTAs stay where they are the faster ones: exact KBC (256^3 D3Q27 1864 / 2061, D3Q19 in place 842 /
+// 869: its code is the longest, and the warps of one CTA run through it together), D2Q9 in place (256^2 2.40 /
+// 2.46) and fast (1.96 / 2.09), D3Q19 in place Float16C without LES (402 / 408) and fast (420 / 423).  (The
+// fused-link kernels were not measured and keep them.)
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS>
+constexpr int tile_threads() {
+    constexpr bool ESO = METHOD == LBM_ESOTERIC_PULL;
+    if (LINKS) return 256;
+    if (COLL == LBM_KBC) return FAST ? 128 : 256;
+    if (L::Q == 27) return 128;
+    if (FAST) return L::Q == 19 && !ESO ? 128 : 256;
+    return ESO && (L::Q == 9 || (F16C && !LES)) ? 256 : 128;
+}
+
+// Resident CTAs per SM they are built for: in CTAs of 256 threads tile_min_blocks; in CTAs of 128 the same
+// registers a thread, but 72 instead of 80 for KBC and D3Q27 (7 CTAs; D3Q27 float32 576 -> 560, KBC Float16C
+// 537 -> 521), save for their combination in place (557 -> 561).
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS>
+constexpr int tile_ctas() {
+    constexpr int full = tile_min_blocks<L, COLL, LINKS>();
+    if (tile_threads<L, METHOD, F16C, COLL, LES, FAST, LINKS>() == 256) return full;
+    if (L::Q == 27 && COLL == LBM_KBC && METHOD == LBM_ESOTERIC_PULL) return 6;
+    return L::Q == 27 || COLL == LBM_KBC ? 7 : 2 * full;
+}
+
 template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST = false, bool LINKS = false>
-__global__ void __launch_bounds__(256, (tile_min_blocks<L, COLL, LINKS>()))
+__global__ void __launch_bounds__((tile_threads<L, METHOD, F16C, COLL, LES, FAST, LINKS>()),
+                                  (tile_ctas<L, METHOD, F16C, COLL, LES, FAST, LINKS>()))
     step_kernel_tile(const StepArgs a) {
     static_assert(LES != kLesLearned, "the learned closure runs in step_kernel_learned");
-    const uint32_t tile = blockIdx.x, tid = threadIdx.x;
+    constexpr int NT = tile_threads<L, METHOD, F16C, COLL, LES, FAST, LINKS>();
+    constexpr uint32_t PARTS = kTileCells / NT;
+    const uint32_t tile = blockIdx.x / PARTS, tid = threadIdx.x + NT * (blockIdx.x % PARTS);
     pdl_wait_before_masks(a);
     const bool general = tile_general(load_near(a.tile_near + tile), tid);
     uint2 m = make_uint2(0u, 0u);
     if (general) m = load_masks(a.cell_masks + (tid + kTileCells * tile));
     pdl_wait_after_masks(a);
-    tile_forms<L, METHOD, F16C, COLL, LES, FAST, LINKS, false>(a, tile, tid, general, m, nullptr, nullptr, nullptr);
+    tile_forms<L, METHOD, F16C, COLL, LES, FAST, LINKS, false, NT>(a, tile, tid, general, m, nullptr, nullptr, nullptr);
 }
 
 #ifndef LBM_LEARNED_MIN_BLOCKS
@@ -1497,27 +1534,30 @@ cudaError_t launch_step(const StepArgs& a, int threads, cudaStream_t s) {
     return launch_pdl(step_kernel<L, METHOD, F16C, COLL, LES, int64_t>, blocks, (uint32_t)threads, s, a);
 }
 
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS>
+cudaError_t launch_tile(const StepArgs& a, cudaStream_t s) {
+    constexpr uint32_t NT = tile_threads<L, METHOD, F16C, COLL, LES, FAST, LINKS>();
+    return launch_pdl(step_kernel_tile<L, METHOD, F16C, COLL, LES, FAST, LINKS>, a.lay.ncells / NT, NT, s, a);
+}
 template <class L, int METHOD, bool F16C, int COLL, int LES>
 cudaError_t launch_step_tile(const StepArgs& a, int, cudaStream_t s) {
-    return launch_pdl(step_kernel_tile<L, METHOD, F16C, COLL, LES>, a.lay.ncells / kTileCells, kTileCells, s, a);
+    return launch_tile<L, METHOD, F16C, COLL, LES, false, false>(a, s);
 }
 
 // The fast-arithmetic build of the block-per-tile kernel (LBM_ARITH_FAST).
 template <class L, int METHOD, bool F16C, int COLL, int LES>
 cudaError_t launch_step_tile_fast(const StepArgs& a, int, cudaStream_t s) {
-    return launch_pdl(step_kernel_tile<L, METHOD, F16C, COLL, LES, true>, a.lay.ncells / kTileCells, kTileCells, s, a);
+    return launch_tile<L, METHOD, F16C, COLL, LES, true, false>(a, s);
 }
 
 // The block-per-tile kernel with fused links (lbm_set_links), exact and fast arithmetic.
 template <class L, int METHOD, bool F16C, int COLL, int LES>
 cudaError_t launch_step_tile_links(const StepArgs& a, int, cudaStream_t s) {
-    return launch_pdl(step_kernel_tile<L, METHOD, F16C, COLL, LES, false, true>, a.lay.ncells / kTileCells, kTileCells,
-                      s, a);
+    return launch_tile<L, METHOD, F16C, COLL, LES, false, true>(a, s);
 }
 template <class L, int METHOD, bool F16C, int COLL, int LES>
 cudaError_t launch_step_tile_links_fast(const StepArgs& a, int, cudaStream_t s) {
-    return launch_pdl(step_kernel_tile<L, METHOD, F16C, COLL, LES, true, true>, a.lay.ncells / kTileCells, kTileCells,
-                      s, a);
+    return launch_tile<L, METHOD, F16C, COLL, LES, true, true>(a, s);
 }
 
 template <class L, int METHOD, bool F16C, int COLL, int LES>
