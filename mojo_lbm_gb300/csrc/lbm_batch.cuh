@@ -104,18 +104,11 @@ __global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, LBM_DOUBLE_B
     bool waited = !b.ready;
     for (BatchWalk w(b); w.u < w.end; ++w.u) {
         const uint32_t tile = w.tile(b, &sa);
-        const uint32_t mask = load_near(sa.tile_near + tile);
-        const bool general = !__all_sync(0xffffffffu, ((mask >> ((t >> 5) * 2u)) & 3u) == 0u);
-        uint4 m = make_uint4(0u, 0u, 0u, 0u);
-        if (general && ((mask >> (t >> 4)) & 1u)) m = load_masks2(sa.cell_masks + (2u * t + kTileCells * tile));
+        PairMasks pm;
+        pm.load<false>(load_near(sa.tile_near + tile), sa.cell_masks, tile, t);
         if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
         waited = true;
-        const uint32_t byz = sa.lay.d_ntx.div(tile);
-        const uint32_t bx = tile - byz * (uint32_t)sa.lay.ntx;
-        const uint32_t bz = sa.lay.d_nty.div(byz);
-        const uint32_t by = byz - bz * (uint32_t)sa.lay.nty;
-        if (!general) pair_cells<L, LBM_DOUBLE_BUFFER, F16C, COLL, LES, false, false>(sa, tile, t, m, bx, by, bz);
-        else pair_cells<L, LBM_DOUBLE_BUFFER, F16C, COLL, LES, false, true>(sa, tile, t, m, bx, by, bz);
+        pair_step<L, LBM_DOUBLE_BUFFER, F16C, COLL, LES, false, false>(sa, tile, t, pm);
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -18,7 +18,8 @@
 // Everything else is the per-cell code of tile_step (lbm_step.cuh), applied to A and B in turn or to
 // both at once with the same operations: the results are those of step_kernel_tile bit for bit (the
 // exact build) or word for word (the fast build).  A warp owns the warp boxes 2w and 2w + 1 of the
-// tile (its 64 cells); it takes the all-fluid branch when both boxes' mask bits are clear.
+// tile (its 64 cells); it takes the all-fluid branch when both boxes' mask bits are clear, otherwise the pair
+// body's general form or two passes of the per-cell body (pair_by_cell).
 //
 // Requirements: the population buffers 8-byte aligned (the host falls back to the per-cell kernel
 // otherwise), tx >= 2, no learned closure.
@@ -328,12 +329,85 @@ __device__ __forceinline__ void pair_cells(const StepArgs& a, const uint32_t til
     else store(std::integral_constant<int, 2>{});
 }
 
+// Does a warp with a flag in or next to its 64 cells step them by two passes of the per-cell body (tile_cell,
+// which folds the bounce-back into the pull addresses), instead of the pair body's general form (which pulls
+// both cells by words and then reloads direction by direction)?  us a step, general form / by cell:
+//   exact double buffer   192^3 D3Q19 cavity SRT 164.0 / 162.7, Float16C 161.3 / 147.6, TRT 176.6 / 170.7, RLBM
+//                         171.7 / 163.5, Float16C with LES 238 / 213; 1024^2 D2Q9 11.8 / 11.0, TRT 13.7 / 12.8
+//   fast double buffer    1024^2 D2Q9 10.75 / 9.46, Float16C 9.42 / 8.85; D3Q19 Float16C cavity 128^3 37.5 / 36.0,
+//                         256^3 240.7 / 236.3 (a periodic box without a flag 29.7 / 30.1: the compiler's code for
+//                         the pairs differs), TRT 44.0 / 40.1; not RLBM (38.3 / 38.0, box 30.8 / 31.7) and SRT
+//                         with LES (45.9 / 43.7, box 38.6 / 40.5)
+//   in place              256^3 D3Q27 Float16C TRT with LES 491 / 456, RLBM 430 / 421, SRT 421.5 / 409.9; not SRT
+//                         with LES (448 / 472) nor the other lattices (192^3 D3Q19 112.9 / 120.1, D2Q9 9.87 / 9.97)
+// KBC keeps the general form (256^3 D3Q19 in place 387 / 396), and so does the batch, whose narrow domains have
+// such warps everywhere (128 channels 190 / 202).
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST>
+constexpr bool pair_by_cell() {
+    if (COLL == LBM_KBC) return false;
+    if (METHOD == LBM_ESOTERIC_PULL) return L::Q == 27 && !(COLL == LBM_SRT && LES);
+    return !FAST || L::Q != 19 || COLL == LBM_TRT || (COLL == LBM_SRT && !LES);
+}
+
+// What a warp of the pair kernel knows before it steps its 64 cells.  near: the tile's mask byte.
+struct PairMasks {
+    bool general;  // a flag in or next to one of its two boxes
+    uint4 m;       // the masks of the thread's two cells (0 in a box without): its pair, or by cell those of
+                   // cells cell(t) and cell(t) + 32
+    template <bool BY_CELL>
+    __device__ __forceinline__ void load(uint32_t near, const uint2* masks, uint32_t tile, uint32_t t) {
+        const uint32_t boxes = (near >> ((t >> 5) * 2u)) & 3u;
+        general = !__all_sync(0xffffffffu, boxes == 0u);
+        m = make_uint4(0u, 0u, 0u, 0u);
+        if (!general) return;
+        // (masks are written for every cell of a box with its bit set)
+        if constexpr (BY_CELL) {
+            const uint2* p = masks + (kTileCells * tile + cell(t));
+            if (boxes & 1u) {
+                const uint2 v = load_masks(p);
+                m.x = v.x;
+                m.y = v.y;
+            }
+            if (boxes & 2u) {
+                const uint2 v = load_masks(p + 32);
+                m.z = v.x;
+                m.w = v.y;
+            }
+        } else {
+            if ((near >> (t >> 4)) & 1u) m = load_masks2(masks + (2u * t + kTileCells * tile));
+        }
+    }
+    static __device__ __forceinline__ uint32_t cell(uint32_t t) { return 2u * (t & ~31u) + (t & 31u); }
+};
+
+// The 256 cells of a tile by 128 threads.  (BY_CELL: pair_by_cell, or false.)
+template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool BY_CELL>
+__device__ __forceinline__ void pair_step(const StepArgs& a, const uint32_t tile, const uint32_t t, const PairMasks& pm) {
+    if (BY_CELL && pm.general) {
+        uint32_t tl = tile;
+        asm volatile("" : "+r"(tl));  // (nothing of this form is computed ahead of the branch)
+#pragma unroll 1
+        for (uint32_t b = 0; b < 2u; ++b)
+            tile_cell<L, METHOD, F16C, COLL, LES, FAST, false, false, true, kPairThreads>(
+                a, tl, PairMasks::cell(t) + 32u * b, b ? make_uint2(pm.m.z, pm.m.w) : make_uint2(pm.m.x, pm.m.y),
+                nullptr, nullptr, nullptr);
+        return;
+    }
+    const uint32_t byz = a.lay.d_ntx.div(tile);
+    const uint32_t bx = tile - byz * (uint32_t)a.lay.ntx;
+    const uint32_t bz = a.lay.d_nty.div(byz);
+    const uint32_t by = byz - bz * (uint32_t)a.lay.nty;
+    if (BY_CELL || !pm.general) pair_cells<L, METHOD, F16C, COLL, LES, FAST, false>(a, tile, t, pm.m, bx, by, bz);
+    else pair_cells<L, METHOD, F16C, COLL, LES, FAST, true>(a, tile, t, pm.m, bx, by, bz);
+}
+
 // Resident CTAs (of 128 threads) per SM the pair kernels are built for: the populations of two
 // cells stay in registers across both collisions, so the budget is wider than the per-cell
 // kernel's.  Float16C in the fast arithmetic 8 (64 registers: 63.7 GLUPs on the 256^3 Float16C
 // cavity against 60.0 at 9, 61.2 at 7 and 58.0 at 6), float32 8 (64 registers, a few spilled
 // bytes in the wall warps' form only: 43.05 GLUPs on the float32 cavity against 42.46 at 7), the
-// exact Float16C build 7 (72 registers; at 64 it spills), TRT 6 (80), KBC and D3Q27 4 (128).
+// exact Float16C build 7 (72 registers; at 64 it spills), float32 D3Q19 SRT with LES 7 (64 registers spill 76
+// bytes; 128^3 cavity 62.3 -> 60.4 us a step, vortex 53.4 -> 49.5), TRT 6 (80), KBC and D3Q27 4 (128).
 #ifndef LBM_PAIR_MIN_BLOCKS_F16C_FAST
 #define LBM_PAIR_MIN_BLOCKS_F16C_FAST 8
 #endif
@@ -356,7 +430,8 @@ constexpr int pair_min_blocks() {
     return (COLL == LBM_KBC || L::Q == 27) ? LBM_PAIR_MIN_BLOCKS_HEAVY
            : COLL == LBM_TRT               ? 6
            : F16C                          ? LBM_PAIR_MIN_BLOCKS_F16C
-                                           : LBM_PAIR_MIN_BLOCKS;
+           : L::Q == 19 && COLL == LBM_SRT && LES ? 7
+                                                  : LBM_PAIR_MIN_BLOCKS;
 }
 
 template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST>
@@ -364,19 +439,11 @@ __global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, METHOD, F16C
     static_assert(LES != kLesLearned, "the learned closure runs in step_kernel_learned");
     const uint32_t tile = blockIdx.x, t = threadIdx.x;
     pdl_wait_before_masks(a);
-    // ---- the warp's two boxes (cells 64w .. 64w + 63) all plain FLUID with FLUID neighbours?
-    const uint32_t mask = load_near(a.tile_near + tile);
-    const bool general = !__all_sync(0xffffffffu, ((mask >> ((t >> 5) * 2u)) & 3u) == 0u);
-    // the masks of both cells (written for every cell of a box with its bit set)
-    uint4 m = make_uint4(0u, 0u, 0u, 0u);
-    if (general && ((mask >> (t >> 4)) & 1u)) m = load_masks2(a.cell_masks + (2u * t + kTileCells * tile));
+    constexpr bool BY_CELL = pair_by_cell<L, METHOD, F16C, COLL, LES, FAST>();
+    PairMasks pm;
+    pm.load<BY_CELL>(load_near(a.tile_near + tile), a.cell_masks, tile, t);
     pdl_wait_after_masks(a);
-    const uint32_t byz = a.lay.d_ntx.div(tile);
-    const uint32_t bx = tile - byz * (uint32_t)a.lay.ntx;
-    const uint32_t bz = a.lay.d_nty.div(byz);
-    const uint32_t by = byz - bz * (uint32_t)a.lay.nty;
-    if (!general) pair_cells<L, METHOD, F16C, COLL, LES, FAST, false>(a, tile, t, m, bx, by, bz);
-    else pair_cells<L, METHOD, F16C, COLL, LES, FAST, true>(a, tile, t, m, bx, by, bz);
+    pair_step<L, METHOD, F16C, COLL, LES, FAST, BY_CELL>(a, tile, t, pm);
 }
 
 template <class L, int METHOD, bool F16C, int COLL, int LES>
