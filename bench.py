@@ -57,7 +57,7 @@ WORKLOADS = {
                                   tile=(16, 16, 1), autotune=True,
                                   desc="512 D2Q9 SRT cylinder channels, nx ~ U[200,800], ny = 0.41 nx (sizes on a 32-cell granule, tile autotuned), "
                                        "Re ~ U[20,200], parabolic moving-wall inlet u_max=0.05, equilibrium outlet, "
-                                       "Bouzidi links on the cylinder, FP32, one persistent launch per step"),
+                                       "Bouzidi links on the cylinder, FP32, one launch per step"),
 }
 # The reference's published benchmark (README of JohnCSu/mojo_lbm): D3Q19 256^3, fully periodic, all
 # fluid, at rest, tau = 0.884 (benchmarks/D3.mojo:39-46), FP32 and Float16C + DDF shift; the MLUPs it
@@ -467,7 +467,7 @@ def run_ours(args, wl: dict):
                 "d2h_bytes_per_step": int(d2h / K),
                 "note": "Solver.run from pinned host buffers: upload of f, bc, flags and download of f inside the "
                         f"timed region, amortised over the {K} steps (after one untimed pass of 64 steps)"},
-        "gpu_launches": K + 3,  # per timed K-step replay
+        "gpu_launches": K + 1,  # per timed K-step replay: the steps and one flag check
         "clocks": clk,
     }
     line.update(extra)
@@ -480,7 +480,7 @@ def run_ours(args, wl: dict):
 
 
 def run_batch(args, wl: dict):
-    """512 uneven D2Q9 cylinder channels, one persistent launch per step."""
+    """512 uneven D2Q9 cylinder channels, one launch per step."""
     import torch
     from mojo_lbm_gb300.batch import BatchSolver
     from mojo_lbm_gb300.solver import Solver
@@ -552,7 +552,7 @@ def run_batch(args, wl: dict):
     clk = clocks.stop() if clocks else None
     t_ms, units = aggregate(statistics.median(reps), float(N) * K, world, dev)
     mlups = units / (t_ms * 1e-3) / 1e6
-    launch_ms = t_ms / K  # per step: the persistent step launch (+ the link launch when separate), averaged
+    launch_ms = t_ms / K  # per step: the step launch (+ the link launch when separate), averaged
 
     # end to end through the public API: every domain's f, bc and flags uploaded from pinned host
     # memory, K batched steps, every f downloaded, inside the timed region
@@ -601,7 +601,7 @@ def run_batch(args, wl: dict):
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": traffic,
                      "note": f"72 B/update x {N} cells / average per-step time over the timed region {launch_ms:.4f} "
-                             f"ms (persistent step{'' if links_mode == 'fused' else ' + link kernel'}); peak {peak_kind}; traffic = ncu dram bytes per "
+                             f"ms (batched step{'' if links_mode == 'fused' else ' + link kernel'}); peak {peak_kind}; traffic = ncu dram bytes per "
                              f"launch ({traffic_src or 'no capture committed'}, scaled by cells)"},
         "cpu_baseline": None,
         "e2e": {"value": round(e2e_units / (e2e_ms * 1e-3) / 1e6, 2), "unit": "MLUPs",

@@ -78,7 +78,8 @@ enum { LBM_BB_MID_GRID = 0, LBM_BB_BOUZIDI = 1 };
  *   Float16C codes handled in a scaled form), held to a float32 tolerance of the exact step:
  *   after one step every float32 population within 1e-6 of it (plus 2e-6 relative for KBC and
  *   LES), every Float16C code within 1 unit in the last place.  Used by the block-per-tile and
- *   batched kernels; a grid those kernels do not take runs the exact arithmetic. */
+ *   cell-pair kernels; the batched step, and a grid those kernels do not take, run the exact
+ *   arithmetic. */
 enum { LBM_ARITH_EXACT = 0, LBM_ARITH_FAST = 1 };
 
 /*

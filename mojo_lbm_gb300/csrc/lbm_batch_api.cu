@@ -98,7 +98,7 @@ void drop_graphs(lbm_batch* b) {
 }
 
 // tile_near: per unit, the warp_near bits of its 8 warp boxes; one thread per box.  Skipped unless
-// a box summary changed in this round (*changed == gen).
+// a box summary changed in this check (*changed == gen).
 __global__ void batch_near_kernel(const BatchArgs b, const uint8_t* box_sum, uint8_t* tile_near,
                                   const uint32_t* changed, uint32_t gen) {
     if (*changed != gen) return;  // the same value for every thread
@@ -107,7 +107,7 @@ __global__ void batch_near_kernel(const BatchArgs b, const uint8_t* box_sum, uin
 }
 
 // The neighbour-solid masks of the cells of every warp with its mask bit set, one block per unit,
-// after a change of the flags in this round (*changed == gen), or always; resting_walls:
+// after a change of the flags in this check (*changed == gen), or always; resting_walls:
 // without_resting_walls.
 template <class L>
 __global__ void __launch_bounds__(256) batch_cell_mask_kernel(const BatchArgs b, const uint32_t* changed,

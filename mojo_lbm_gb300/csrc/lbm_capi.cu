@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) box_summary_kernel(const uint8_t* __restr
 }
 
 // tile_near: per tile, bit w = warp_near of its warp box w; one thread per warp box.  Skipped
-// (every thread returns) unless a box summary changed in this round (*changed == gen).
+// (every thread returns) unless a box summary changed in this check (*changed == gen).
 __global__ void __launch_bounds__(256) tile_near_kernel(const uint8_t* __restrict__ box_sum, const LayoutDesc l,
                                                         uint32_t nboxes, uint8_t* __restrict__ tile_near,
                                                         const uint32_t* changed, uint32_t gen) {
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) tile_near_kernel(const uint8_t* __restric
 
 // The neighbour-solid masks of every cell in a warp with its mask bit set (256 threads per tile,
 // blocks striding over the tiles: a launch with nothing to do is one short wave), after a change of
-// the flags in this round (*changed == gen), or always.
+// the flags in this check (*changed == gen), or always.
 template <class L>
 __global__ void __launch_bounds__(256) cell_mask_kernel(const StepArgs a, uint2* __restrict__ masks,
                                                         const uint32_t* changed, uint32_t gen, uint32_t ntiles,
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256) flags_check_kernel(const uint8_t* __restr
     if (differ) *changed = gen;
 }
 
-// Rebuilds the masks after a change of the flags in this round (*changed == gen): one thread per cell,
+// Rebuilds the masks after a change of the flags in this check (*changed == gen): one thread per cell,
 // blocks striding over the 256-cell chunks.  With always, the warps whose bit is set are rebuilt without
 // one.  bc: without_resting_walls, or null.
 template <class L>
