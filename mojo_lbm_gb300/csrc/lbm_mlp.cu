@@ -36,7 +36,8 @@ uint32_t pair(float lo, float hi) { return (uint32_t)bf16_bits(lo) | ((uint32_t)
 
 constexpr int kFwdThreads = 256;
 constexpr int kBwdThreads = 128;   // one sample per thread per chunk
-constexpr int kPad = kHid + 1;                // padded row of a hidden-layer array in shared memory
+constexpr int kPad = kHid + 4;                // padded row of a hidden-layer array in shared memory: 16-byte
+                                              // aligned, and 8 threads' float4 cover all banks
 constexpr int kBwdRow = kIn + 4 * kPad + 1;   // x, h1, dh1, gy*h2, dh2, gy per sample
 
 __device__ __forceinline__ void load_theta(const float* __restrict__ theta, float* w) {
@@ -98,15 +99,18 @@ __global__ void __launch_bounds__(kFwdThreads) mlp_forward_kernel(const float* _
 
 // Per-block partial gradients over a contiguous range of samples, in chunks of kBwdThreads.  Each
 // thread recomputes its sample's activations, leaves x, h1, dh1, gy*h2, dh2 and gy in shared
-// memory, and then owns fixed parameters whose sums over the chunk it accumulates in registers
-// (a warp's lanes read consecutive hidden units, the same sample row: no bank conflicts).
+// memory, and then owns fixed parameters whose sums over the chunk it accumulates in registers, in
+// sample order.  Bound by shared-memory reads: a 4 x 2 block of w2, two entries of w1 and one of the
+// rest per thread take 5 reads and 11 multiply-adds a sample (8 entries of one column of w2 took 13
+// reads).  With the sum of the partials: 2^18 rows 168 -> 108 us, 2^20 rows 526 -> 318 us, the same bits
+// (every sum keeps its order).
 __global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* __restrict__ theta,
                                                                    const float* __restrict__ x,
                                                                    const float* __restrict__ g, int64_t n,
                                                                    float nu_scale, int64_t per_block,
                                                                    float* __restrict__ partial) {
     __shared__ __align__(16) float w[kParams];
-    extern __shared__ float rows[];  // kBwdThreads * kBwdRow
+    extern __shared__ __align__(16) float rows[];  // kBwdThreads * kBwdRow
     load_theta(theta, w);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* X = rows;
@@ -116,10 +120,14 @@ __global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* 
     float* DH2 = P3 + kBwdThreads * kPad;
     float* GY = DH2 + kBwdThreads * kPad;
 
-    float acc_w2[8], acc_w1[2], acc_x = 0.f;
+    // this thread's parameters: w2[4 kg ..][2 jg ..], w1[kg][2 jg ..] and one of b1, b2, w3, b3 (by warp)
+    const int kg = tid >> 4, jg = tid & 15;
+    float acc_w2[4][2], acc_w1[2], acc_x = 0.f;
 #pragma unroll
-    for (int r = 0; r < 8; ++r) acc_w2[r] = 0.f;
+    for (int r = 0; r < 4; ++r) acc_w2[r][0] = acc_w2[r][1] = 0.f;
     acc_w1[0] = acc_w1[1] = 0.f;
+    const float* other = warp == 0 ? DH1 + lane : warp == 1 ? DH2 + lane : warp == 2 ? P3 + lane : GY;
+    const int other_stride = warp == 3 ? 1 : kPad;
 
     const int64_t s0 = (int64_t)blockIdx.x * per_block;
     const int64_t s1 = s0 + per_block < n ? s0 + per_block : n;
@@ -143,57 +151,83 @@ __global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* 
 #pragma unroll
         for (int k = 0; k < kIn; ++k) X[tid * kIn + k] = xi[k];
 #pragma unroll
-        for (int j = 0; j < kHid; ++j) {
-            dh2[j] = h2[j] > 0.f ? gy * w[kW3 + j] : 0.f;
-            H1[tid * kPad + j] = h1[j];
-            P3[tid * kPad + j] = gy * h2[j];
-            DH2[tid * kPad + j] = dh2[j];
+        for (int j = 0; j < kHid; j += 4) {
+#pragma unroll
+            for (int k = j; k < j + 4; ++k) dh2[k] = h2[k] > 0.f ? gy * w[kW3 + k] : 0.f;
+            *reinterpret_cast<float4*>(H1 + tid * kPad + j) = make_float4(h1[j], h1[j + 1], h1[j + 2], h1[j + 3]);
+            *reinterpret_cast<float4*>(P3 + tid * kPad + j) =
+                make_float4(gy * h2[j], gy * h2[j + 1], gy * h2[j + 2], gy * h2[j + 3]);
+            *reinterpret_cast<float4*>(DH2 + tid * kPad + j) = make_float4(dh2[j], dh2[j + 1], dh2[j + 2], dh2[j + 3]);
         }
 #pragma unroll 1
-        for (int j = 0; j < kHid; ++j) {  // dh1 = (W2 dh2) masked by ReLU
-            float a = 0.f;
+        for (int j = 0; j < kHid; j += 4) {  // dh1 = (W2 dh2) masked by ReLU
+            float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int k = 0; k < kHid; k += 4) {
-                const float4 v = *reinterpret_cast<const float4*>(w + kW2 + j * kHid + k);
-                a = __fmaf_rn(v.x, dh2[k], a);
-                a = __fmaf_rn(v.y, dh2[k + 1], a);
-                a = __fmaf_rn(v.z, dh2[k + 2], a);
-                a = __fmaf_rn(v.w, dh2[k + 3], a);
-            }
-            DH1[tid * kPad + j] = H1[tid * kPad + j] > 0.f ? a : 0.f;
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int k = 0; k < kHid; k += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(w + kW2 + (j + r) * kHid + k);
+                    a[r] = __fmaf_rn(v.x, dh2[k], a[r]);
+                    a[r] = __fmaf_rn(v.y, dh2[k + 1], a[r]);
+                    a[r] = __fmaf_rn(v.z, dh2[k + 2], a[r]);
+                    a[r] = __fmaf_rn(v.w, dh2[k + 3], a[r]);
+                }
+            const float4 h = *reinterpret_cast<const float4*>(H1 + tid * kPad + j);
+            *reinterpret_cast<float4*>(DH1 + tid * kPad + j) = make_float4(
+                h.x > 0.f ? a[0] : 0.f, h.y > 0.f ? a[1] : 0.f, h.z > 0.f ? a[2] : 0.f, h.w > 0.f ? a[3] : 0.f);
         }
         GY[tid] = gy;
         __syncthreads();
         const int rows_here = (int)((s1 - c) < kBwdThreads ? (s1 - c) : kBwdThreads);
+#pragma unroll 4
         for (int s = 0; s < rows_here; ++s) {
-            const float d2 = DH2[s * kPad + lane];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) acc_w2[r] = __fmaf_rn(H1[s * kPad + warp + 4 * r], d2, acc_w2[r]);
-            const float d1 = DH1[s * kPad + lane];
-            acc_w1[0] = __fmaf_rn(X[s * kIn + warp], d1, acc_w1[0]);
-            acc_w1[1] = __fmaf_rn(X[s * kIn + warp + 4], d1, acc_w1[1]);
-            // warp 0: b1, warp 1: b2, warp 2: w3, warp 3: b3 (lane 0)
-            acc_x += warp == 0 ? d1 : warp == 1 ? d2 : warp == 2 ? P3[s * kPad + lane] : GY[s];
+            const float4 h = *reinterpret_cast<const float4*>(H1 + s * kPad + 4 * kg);
+            const float2 d2 = *reinterpret_cast<const float2*>(DH2 + s * kPad + 2 * jg);
+            const float2 d1 = *reinterpret_cast<const float2*>(DH1 + s * kPad + 2 * jg);
+            const float xv = X[s * kIn + kg];
+            acc_w2[0][0] = __fmaf_rn(h.x, d2.x, acc_w2[0][0]);
+            acc_w2[0][1] = __fmaf_rn(h.x, d2.y, acc_w2[0][1]);
+            acc_w2[1][0] = __fmaf_rn(h.y, d2.x, acc_w2[1][0]);
+            acc_w2[1][1] = __fmaf_rn(h.y, d2.y, acc_w2[1][1]);
+            acc_w2[2][0] = __fmaf_rn(h.z, d2.x, acc_w2[2][0]);
+            acc_w2[2][1] = __fmaf_rn(h.z, d2.y, acc_w2[2][1]);
+            acc_w2[3][0] = __fmaf_rn(h.w, d2.x, acc_w2[3][0]);
+            acc_w2[3][1] = __fmaf_rn(h.w, d2.y, acc_w2[3][1]);
+            acc_w1[0] = __fmaf_rn(xv, d1.x, acc_w1[0]);
+            acc_w1[1] = __fmaf_rn(xv, d1.y, acc_w1[1]);
+            acc_x += other[s * other_stride];
         }
         __syncthreads();
     }
     float* out = partial + (size_t)blockIdx.x * kParams;
 #pragma unroll
-    for (int r = 0; r < 8; ++r) out[kW2 + (warp + 4 * r) * kHid + lane] = acc_w2[r];
-    out[kW1 + warp * kHid + lane] = acc_w1[0];
-    out[kW1 + (warp + 4) * kHid + lane] = acc_w1[1];
+    for (int r = 0; r < 4; ++r) {
+        out[kW2 + (4 * kg + r) * kHid + 2 * jg] = acc_w2[r][0];
+        out[kW2 + (4 * kg + r) * kHid + 2 * jg + 1] = acc_w2[r][1];
+    }
+    out[kW1 + kg * kHid + 2 * jg] = acc_w1[0];
+    out[kW1 + kg * kHid + 2 * jg + 1] = acc_w1[1];
     if (warp == 0) out[kB1 + lane] = acc_x;
     else if (warp == 1) out[kB2 + lane] = acc_x;
     else if (warp == 2) out[kW3 + lane] = acc_x;
     else if (lane == 0) out[kB3] = acc_x;
 }
 
-// grad[p] = sum over blocks of partial[b][p], in block order (deterministic).
+// grad[p] = sum over blocks of partial[b][p], in block order (deterministic).  A serial chain of up to 608
+// additions per parameter: its loads go ahead of it, one warp a block spreads them over the SMs.
 __global__ void mlp_sum_partials_kernel(const float* __restrict__ partial, int nblocks, float* __restrict__ grad) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kParams) return;
     float s = 0.f;
-    for (int b = 0; b < nblocks; ++b) s += partial[(size_t)b * kParams + p];
+    int b = 0;
+    for (; b + 16 <= nblocks; b += 16) {  // (16 loads in flight, added in block order)
+        float v[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) v[r] = partial[(size_t)(b + r) * kParams + p];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) s += v[r];
+    }
+    for (; b < nblocks; ++b) s += partial[(size_t)b * kParams + p];
     grad[p] = s;
 }
 
@@ -312,7 +346,7 @@ lbm_status lbm_mlp_backward(const float* theta, const float* x, const float* g, 
     mlp_backward_kernel<<<used, kBwdThreads, smem, s>>>(theta, x, g, n, nu_scale, per_block, partial);
     e = cudaGetLastError();
     if (e == cudaSuccess) {
-        mlp_sum_partials_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(partial, used, grad_theta);
+        mlp_sum_partials_kernel<<<(kParams + 31) / 32, 32, 0, s>>>(partial, used, grad_theta);
         e = cudaGetLastError();
     }
     const cudaError_t ef = cudaFreeAsync(partial, s);
