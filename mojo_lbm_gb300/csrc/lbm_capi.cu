@@ -78,12 +78,12 @@ __global__ void __launch_bounds__(256) tile_near_kernel(const uint8_t* __restric
 
 // The neighbour-solid masks of every cell in a warp with its mask bit set (256 threads per tile,
 // blocks striding over the tiles: a launch with nothing to do is one short wave), after a change of
-// the flags in this check (*changed == gen), or always.
+// the flags in this check (*changed == gen), or, changed null, always.
 template <class L>
 __global__ void __launch_bounds__(256) cell_mask_kernel(const StepArgs a, uint2* __restrict__ masks,
                                                         const uint32_t* changed, uint32_t gen, uint32_t ntiles,
-                                                        int always, int resting_walls) {
-    if (!always && *changed != gen) return;  // the same value for every thread
+                                                        int resting_walls) {
+    if (changed && *changed != gen) return;  // the same value for every thread
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
         tile_cell_masks<L>(a, tile, masks, resting_walls != 0);
 }
@@ -92,17 +92,15 @@ __global__ void __launch_bounds__(256) cell_mask_kernel(const StepArgs a, uint2*
 // flags of `per_block` tiles (16 at most, 16 bytes a thread) with flags_seen, and for a tile that changed
 // it rebuilds, from the flags themselves, the mask byte and the cell masks of that tile and of the 26
 // around it (periodic), whose cells may pull from it.  A neighbour that differs from flags_seen as well
-// is left to its own block; two blocks that rebuild the same tile write the same values.  always: the
-// cell masks of every warp whose bit is set are rebuilt (a run without its walls at rest).
+// is left to its own block; two blocks that rebuild the same tile write the same values.
 // A single step with the three launches of the first build before it is bound by launches on the host
 // and by their chain on the GPU: a step of a 320 x 128 D2Q9 channel and its link pass, called from a host
 // loop, went from 18.0 to 11.2 us with this one (launched, like the steps, with programmatic dependent
 // launch).
 template <class L>
-__device__ __forceinline__ void rebuild_tile(const StepArgs& a, uint32_t tile, uint8_t* near, uint2* masks, bool resting,
-                                             uint32_t* bits) {
+__device__ __forceinline__ void rebuild_tile(const StepArgs& a, uint32_t tile, uint8_t* near, uint2* masks, uint32_t* bits) {
     uint32_t any;
-    const uint2 m = tile_cell_mask<L>(a, tile, threadIdx.x, resting, any);
+    const uint2 m = tile_cell_mask<L>(a, tile, threadIdx.x, false, any);
     const bool warp_any = __any_sync(0xffffffffu, any != 0u);
     if (warp_any) masks[threadIdx.x + kTileCells * tile] = m;
     if (threadIdx.x == 0) *bits = 0u;
@@ -128,7 +126,7 @@ __device__ __forceinline__ bool differ16(const uint4& x, const uint4& y) {
 
 template <class L>
 __global__ void __launch_bounds__(256) tile_check_kernel(const StepArgs a, uint8_t* seen, uint8_t* near, uint2* masks,
-                                                         uint32_t ntiles, uint32_t per_block, int always, int resting) {
+                                                         uint32_t ntiles, uint32_t per_block) {
     __shared__ uint32_t changed, bits;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -162,19 +160,12 @@ __global__ void __launch_bounds__(256) tile_check_kernel(const StepArgs a, uint8
                     other = differ16(load_flags16(a.flags + o), __ldcg(reinterpret_cast<const uint4*>(seen + o)));
                 }
                 if (__syncthreads_or(other)) continue;
-                rebuild_tile<L>(a, t, near, masks, resting != 0, &bits);
+                rebuild_tile<L>(a, t, near, masks, &bits);
             }
         }
         __syncthreads();
         if (differ) *reinterpret_cast<uint4*>(seen + at) = now;
     }
-    if (always)
-        for (uint32_t k = 0; k < per_block && tile0 + k < ntiles; ++k)
-            if ((near[tile0 + k] >> (threadIdx.x >> 5)) & 1u) {
-                uint32_t any;
-                masks[threadIdx.x + kTileCells * (tile0 + k)] =
-                    tile_cell_mask<L>(a, tile0 + k, threadIdx.x, resting != 0, any);
-            }
 }
 
 // The generic kernel's masks (any tile): bit (n / 32) % 8 of near[n / 256] and the neighbour-solid masks
@@ -262,8 +253,8 @@ lbm_status fail(lbm_status s, const std::string& msg) {
 int lattice_q(int id) { return id == LBM_D2Q9 ? 9 : id == LBM_D3Q19 ? 19 : id == LBM_D3Q27 ? 27 : -1; }
 int lattice_d(int id) { return id == LBM_D2Q9 ? 2 : (id == LBM_D3Q19 || id == LBM_D3Q27) ? 3 : -1; }
 
-// Graph cache key for lbm_run: buffers, tau bits, parity of the first step, chunk length.
-using GraphKey = std::tuple<const void*, const void*, const void*, const void*, uint32_t, int, int64_t, int>;
+// Graph cache key for lbm_run: buffers, tau bits, parity of the first step, chunk length, kernel, masks.
+using GraphKey = std::tuple<const void*, const void*, const void*, const void*, uint32_t, int, int64_t, int, const void*>;
 
 }  // namespace
 
@@ -294,11 +285,14 @@ struct lbm_handle {
     uint32_t* changed;     // device word: summary round in which a box summary last changed
     uint32_t summary_gen;  // summary rounds issued
     int summary_valid;     // box_sum and flags_seen hold a complete summary
-    int masks_resting;     // cell_masks are those of the last run's bc (without_resting_walls)
-    int resting_ok;        // runs may build such masks: one stream, no call captured
-    int run_recorded;      // run_done is recorded: a call on any stream waits for it before it uses the masks
-    cudaStream_t run_stream;
-    cudaEvent_t run_done;  // the last run with such masks, or the rebuild after it
+    // What depends on bc, or on flags that other streams need not share, belongs to the first stream that
+    // steps the handle outside a capture (owner): run_masks (block-per-tile kernels), cell_masks and what
+    // they are built from (generic kernel).
+    int owned;
+    unsigned long long owner;  // cudaStreamGetId
+    uint2* run_masks;      // cell masks of a run without its walls at rest (without_resting_walls), or null
+    int run_masks_failed;  // no memory for them
+    int masks_resting;     // generic kernel: cell_masks are those of the last run's bc
     uint8_t* tile_near;    // per tile: warp_near bits of its 8 warp boxes (block-per-tile kernel)
     uint32_t ntiles;
     uint32_t mx, my, shx, shxy;
@@ -343,8 +337,15 @@ __attribute__((visibility("hidden"))) LayoutDesc make_layout(const lbm_grid_t& g
 
 namespace {
 
+// The masks a step reads: bits per warp and masks per cell, or null (the generic kernel gathers the
+// neighbours' flags then).
+struct Masks {
+    const uint8_t* near;
+    const uint2* cells;
+};
+
 StepArgs step_args(const lbm_handle* h, const void* f_in, void* f_out, float* bc, const uint8_t* flags, float tau,
-                   int even) {
+                   int even, const Masks& m) {
     StepArgs a;
     a.lay = h->lay;
     a.f_in = f_in;
@@ -363,8 +364,8 @@ StepArgs step_args(const lbm_handle* h, const void* f_in, void* f_out, float* bc
     a.even = even;
     a.closure = h->closure_on ? h->closure : nullptr;
     a.cl = h->closure_uniform;
-    a.tile_near = h->tile_near;
-    a.cell_masks = h->cell_masks;
+    a.tile_near = m.near;
+    a.cell_masks = m.cells;
     a.masks_ready = 0;
     a.mx = h->mx;
     a.my = h->my;
@@ -448,14 +449,14 @@ StepLaunch step_fn(const lbm_handle* h, const StepArgs& a) {
 // Brings the per-tile warp masks of the block-per-tile kernel up to date with `flags`: the boxes
 // whose flags changed since the previous call are summarised again, and the masks are rebuilt
 // only if one did (every step of a run with fixed flags costs one pass over the flags).
-lbm_status tile_summary(lbm_handle* h, const uint8_t* flags, float* bc, bool always, bool resting, cudaStream_t s) {
+lbm_status tile_summary(lbm_handle* h, const uint8_t* flags, bool capturing, cudaStream_t s) {
+    const StepArgs a = step_args(h, nullptr, nullptr, nullptr, flags, 1.f, 0, Masks{h->tile_near, h->cell_masks});
     if (h->summary_valid) {
         // one tile a block until every SM has 8 blocks
         const uint32_t per = std::max<uint32_t>(1u, std::min<uint32_t>(16u, h->ntiles / ((uint32_t)h->sm_count * 8u)));
-        const StepArgs a = step_args(h, nullptr, nullptr, bc, flags, 1.f, 0);
         auto go = [&](auto kernel) {
             return launch_pdl(kernel, (h->ntiles + per - 1u) / per, kTileCells, s, a, h->flags_seen, h->tile_near,
-                              h->cell_masks, h->ntiles, per, (int)always, (int)resting);
+                              h->cell_masks, h->ntiles, per);
         };
         LBM_CK(h->grid.lattice == LBM_D2Q9 ? go(tile_check_kernel<D2Q9>)
                : h->grid.lattice == LBM_D3Q19 ? go(tile_check_kernel<D3Q19>)
@@ -466,39 +467,66 @@ lbm_status tile_summary(lbm_handle* h, const uint8_t* flags, float* bc, bool alw
     const uint32_t gen = h->summary_gen;
     const uint32_t nboxes = h->ntiles * kTileWarps;
     box_summary_kernel<<<(nboxes + 255u) / 256u, 256, 0, s>>>(flags, h->flags_seen, h->lay, h->box_sum, h->changed,
-                                                              gen, h->summary_valid ? 0 : 1);
+                                                              gen, 1);
     LBM_CK(cudaGetLastError());
-    h->summary_valid = 1;
+    // (what a capture records has not run: the calls until then build anew)
+    if (!capturing) h->summary_valid = 1;
     tile_near_kernel<<<(nboxes + 255u) / 256u, 256, 0, s>>>(h->box_sum, h->lay, nboxes, h->tile_near, h->changed,
                                                              gen);
     LBM_CK(cudaGetLastError());
-    const StepArgs a = step_args(h, nullptr, nullptr, bc, flags, 1.f, 0);
     const uint32_t grid = std::min<uint32_t>(h->ntiles, (uint32_t)h->sm_count * 8u);
     switch (h->grid.lattice) {
-        case LBM_D2Q9: cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, h->cell_masks, h->changed, gen, h->ntiles, always, resting); break;
-        case LBM_D3Q19: cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, h->cell_masks, h->changed, gen, h->ntiles, always, resting); break;
-        default: cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, h->cell_masks, h->changed, gen, h->ntiles, always, resting); break;
+        case LBM_D2Q9: cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, h->cell_masks, h->changed, gen, h->ntiles, 0); break;
+        case LBM_D3Q19: cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, h->cell_masks, h->changed, gen, h->ntiles, 0); break;
+        default: cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, h->cell_masks, h->changed, gen, h->ntiles, 0); break;
     }
     LBM_CK(cudaGetLastError());
     return LBM_OK;
 }
 
-// The same for the generic kernel's masks (a handle without them gathers the neighbours' flags in every
-// step).
-lbm_status any_summary(lbm_handle* h, const uint8_t* flags, const float* bc, bool always, bool resting, cudaStream_t s) {
-    if (!h->tile_near) return LBM_OK;
+// The cell masks of one run without its walls at rest, in run_masks; false without the memory for them (8
+// bytes per cell, taken by the first such run).
+bool have_run_masks(lbm_handle* h) {
+    if (h->run_masks || h->run_masks_failed) return h->run_masks != nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (another stream may be captured meanwhile)
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaMalloc(&h->run_masks, sizeof(uint2) * (size_t)h->lay.ncells) != cudaSuccess) {
+        cudaGetLastError();  // cleared: the runs take the masks of the flags
+        h->run_masks = nullptr;
+        h->run_masks_failed = 1;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return h->run_masks != nullptr;
+}
+lbm_status build_run_masks(lbm_handle* h, const uint8_t* flags, float* bc, cudaStream_t s) {
+    const StepArgs a = step_args(h, nullptr, nullptr, bc, flags, 1.f, 0, Masks{h->tile_near, h->cell_masks});
+    const uint32_t grid = std::min<uint32_t>(h->ntiles, (uint32_t)h->sm_count * 8u);
+    switch (h->grid.lattice) {
+        case LBM_D2Q9: cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, h->run_masks, nullptr, 0u, h->ntiles, 1); break;
+        case LBM_D3Q19: cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, h->run_masks, nullptr, 0u, h->ntiles, 1); break;
+        default: cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, h->run_masks, nullptr, 0u, h->ntiles, 1); break;
+    }
+    LBM_CK(cudaGetLastError());
+    return LBM_OK;
+}
+
+// The same for the generic kernel's masks, which only the owner's calls use: without the walls at rest
+// (resting) in place of the masks of the flags, until the next call rebuilds them.
+lbm_status any_summary(lbm_handle* h, const uint8_t* flags, const float* bc, bool resting, cudaStream_t s) {
     if (++h->summary_gen == 0u) ++h->summary_gen;  // 0 is the initial value of *changed
     const uint32_t gen = h->summary_gen, n = h->lay.ncells;
     flags_check_kernel<<<(uint32_t)(((uint64_t)n + 4095u) / 4096u), 256, 0, s>>>(flags, h->flags_seen, n, h->changed, gen);
     LBM_CK(cudaGetLastError());
     const uint32_t chunks = (uint32_t)(((uint64_t)n + 255u) / 256u), grid = std::min<uint32_t>(chunks, (uint32_t)h->sm_count * 8u);
     uint2* masks = h->cell_masks;
+    const bool always = resting || h->masks_resting;
     switch (h->grid.lattice) {
         case LBM_D2Q9: any_mask_kernel<D2Q9><<<grid, 256, 0, s>>>(flags, h->lay, h->tile_near, masks, h->changed, gen, always, resting ? bc : nullptr); break;
         case LBM_D3Q19: any_mask_kernel<D3Q19><<<grid, 256, 0, s>>>(flags, h->lay, h->tile_near, masks, h->changed, gen, always, resting ? bc : nullptr); break;
         default: any_mask_kernel<D3Q27><<<grid, 256, 0, s>>>(flags, h->lay, h->tile_near, masks, h->changed, gen, always, resting ? bc : nullptr); break;
     }
     LBM_CK(cudaGetLastError());
+    h->masks_resting = resting;
     return LBM_OK;
 }
 
@@ -507,46 +535,52 @@ lbm_status any_summary(lbm_handle* h, const uint8_t* flags, const float* bc, boo
 // step).
 constexpr int64_t kRestingMinSteps = 32;
 
-// Brings the masks of the kernel that will step n_steps times up to date with `flags` (and bc).
-// Masks that depend on bc serve one run: the next call rebuilds them, after run_done on whatever stream
-// it comes.  A handle that is used on several streams (whose runs may overlap) or captured into a
-// caller's graph (replayed at times the handle does not see) stays with the masks of the flags alone.
-lbm_status summary(lbm_handle* h, const uint8_t* flags, float* bc, int64_t n_steps, cudaStream_t s) {
-    if (!h->tile_near) return LBM_OK;
-    const bool walls = h->cfg.include_moving_boundary && !h->cfg.capture_density && !h->cfg.capture_velocity;
-    bool capturing = false;
-    if (walls) {
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &st) != cudaSuccess) cudaGetLastError();  // (legacy stream during a capture)
-        else capturing = st != cudaStreamCaptureStatusNone;
+// Is s the stream whose calls, outside captures, own the handle's masks (lbm_handle::owner)?  The first one
+// to ask is.  (By its id: the per-thread default streams share a handle value, and a destroyed stream's is
+// given out again.)
+bool owns_masks(lbm_handle* h, cudaStream_t s) {
+    unsigned long long id = 0;
+    if (cudaStreamGetId(s, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
-    if (capturing) h->resting_ok = 0;
-    if (h->run_recorded && !capturing) {
-        LBM_CK(cudaStreamWaitEvent(s, h->run_done, 0));
-        if (s != h->run_stream) h->resting_ok = 0;
+    if (!h->owned) {
+        h->owned = 1;
+        h->owner = id;
     }
-    const bool resting = walls && h->resting_ok && n_steps >= kRestingMinSteps;
-    const bool always = resting || h->masks_resting;
-    const lbm_status st = h->step_tile ? tile_summary(h, flags, bc, always, resting, s)
-                                       : any_summary(h, flags, bc, always, resting, s);
-    if (st != LBM_OK) return st;
-    if (!capturing) {
-        if (h->masks_resting && !resting) {
-            LBM_CK(cudaEventRecord(h->run_done, s));
-            h->run_stream = s;
-        }
-        h->masks_resting = resting;
-    }
-    return LBM_OK;
+    return id == h->owner;
 }
 
-// After the last step of a run: later calls wait for it before they rebuild its masks.
-lbm_status run_enqueued(lbm_handle* h, cudaStream_t s) {
-    if (!h->masks_resting) return LBM_OK;
-    LBM_CK(cudaEventRecord(h->run_done, s));
-    h->run_recorded = 1;
-    h->run_stream = s;
-    return LBM_OK;
+// The masks for n_steps steps of the kernel that the handle is set to, brought up to date with `flags` (and
+// bc) on s.
+// Calls may overlap on several streams with bc of their own (the generic kernel: with flags of their own),
+// and a call captured into a caller's graph is replayed at times and on streams that the handle does not
+// see.  So masks that another call may read while this one builds come from the flags alone: those of the
+// block-per-tile kernels, which all such calls share (a rebuild for the same flags writes the same words).
+// Masks of a run's bc, and all of the generic kernel's, are the owner's, whose calls are ordered by its
+// stream; other streams and captured calls take the masks of the flags, or gather the neighbours' flags.
+lbm_status summary(lbm_handle* h, const uint8_t* flags, float* bc, int64_t n_steps, cudaStream_t s, Masks& m) {
+    m = Masks{nullptr, nullptr};
+    const bool walls = h->cfg.include_moving_boundary && !h->cfg.capture_density && !h->cfg.capture_velocity;
+    bool resting = walls && n_steps >= kRestingMinSteps;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) cudaGetLastError();  // (legacy stream during a capture)
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    const bool own = !capturing && (resting || !use_tile(h)) && owns_masks(h, s);
+    if (!use_tile(h) && !own) return LBM_OK;
+    resting = resting && own;
+    if (!h->step_tile) {
+        if (!h->tile_near) return LBM_OK;
+        m = Masks{h->tile_near, h->cell_masks};
+        return any_summary(h, flags, bc, resting, s);
+    }
+    m = Masks{h->tile_near, h->cell_masks};
+    lbm_status st = tile_summary(h, flags, capturing, s);
+    if (st == LBM_OK && resting && have_run_masks(h)) {
+        m.cells = h->run_masks;
+        st = build_run_masks(h, flags, bc, s);
+    }
+    return st;
 }
 
 lbm_status check_handle(const lbm_handle* h) {
@@ -554,19 +588,22 @@ lbm_status check_handle(const lbm_handle* h) {
     return LBM_OK;
 }
 
-// One step.  with_summary: rebuild the tile summary from `flags` first (single-step calls; a
-// multi-step run builds it once, since flags cannot change inside the run).  masks_ready: the previous
-// kernel in the stream is a step of the same run.
-lbm_status step_once(lbm_handle* h, const void* f_in, void* f_out, float* bc, const uint8_t* flags, float tau,
-                     int even, cudaStream_t s, bool with_summary = true, bool masks_ready = false) {
-    StepArgs a = step_args(h, f_in, f_out, bc, flags, tau, even);
+// One step with the masks m.  masks_ready: the previous kernel in the stream is a step of the same run.
+lbm_status launch_one(lbm_handle* h, const void* f_in, void* f_out, float* bc, const uint8_t* flags, float tau, int even,
+                      const Masks& m, bool masks_ready, cudaStream_t s) {
+    StepArgs a = step_args(h, f_in, f_out, bc, flags, tau, even, m);
     a.masks_ready = masks_ready ? 1 : 0;
-    if (with_summary) {
-        const lbm_status st = summary(h, flags, bc, 1, s);
-        if (st != LBM_OK) return st;
-    }
     LBM_CK(step_fn(h, a)(a, h->threads, s));
     return LBM_OK;
+}
+
+// A call of one step.
+lbm_status step_once(lbm_handle* h, const void* f_in, void* f_out, float* bc, const uint8_t* flags, float tau, int even,
+                     cudaStream_t s) {
+    Masks m;
+    const lbm_status st = summary(h, flags, bc, 1, s, m);
+    if (st != LBM_OK) return st;
+    return launch_one(h, f_in, f_out, bc, flags, tau, even, m, false, s);
 }
 
 // Blocks of a reduction over n items: kReduceBlocks at most, none without an item (a block without one
@@ -728,11 +765,11 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
     h->changed = nullptr;
     h->summary_gen = 0;
     h->summary_valid = 0;
+    h->owned = 0;
+    h->owner = 0;
+    h->run_masks = nullptr;
+    h->run_masks_failed = 0;
     h->masks_resting = 0;
-    h->resting_ok = 1;
-    h->run_recorded = 0;
-    h->run_stream = nullptr;
-    h->run_done = nullptr;
     h->tile_near = nullptr;
     h->threads = any_threads(h->cfg);
     h->scratch = nullptr;
@@ -751,7 +788,6 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device);
     if (e == cudaSuccess) e = cudaMalloc(&h->scratch, sizeof(double) * (kReduceBlocks * kReduceWidth + 8));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->capture_stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->run_done, cudaEventDisableTiming);
     if (e == cudaSuccess && h->step_tile) e = cudaMalloc(&h->box_sum, (size_t)h->ntiles * kTileWarps);
     if (e == cudaSuccess && h->step_tile) e = cudaMalloc(&h->flags_seen, (size_t)h->lay.ncells);
     if (e == cudaSuccess && h->step_tile) e = cudaMalloc(&h->cell_masks, sizeof(uint2) * (size_t)h->lay.ncells);
@@ -804,6 +840,7 @@ lbm_status lbm_destroy(lbm_handle* h) {
     if (h->box_sum) cudaFree(h->box_sum);
     if (h->flags_seen) cudaFree(h->flags_seen);
     if (h->cell_masks) cudaFree(h->cell_masks);
+    if (h->run_masks) cudaFree(h->run_masks);
     if (h->changed) cudaFree(h->changed);
     if (h->tile_near) cudaFree(h->tile_near);
     if (h->closure) cudaFree(h->closure);
@@ -813,7 +850,6 @@ lbm_status lbm_destroy(lbm_handle* h) {
     if (h->stage_segs) cudaFree(h->stage_segs);
     if (h->dev_err) cudaFree(h->dev_err);
     if (h->capture_stream) cudaStreamDestroy(h->capture_stream);
-    if (h->run_done) cudaEventDestroy(h->run_done);
     delete h;
     return LBM_OK;
 }
@@ -991,13 +1027,15 @@ lbm_status lbm_run(lbm_handle* h, void* f_a, void* f_b, float* bc, const uint8_t
         return fail(LBM_EINVAL, "bc is required by this configuration");
     cudaStream_t s = (cudaStream_t)stream;
     if (n_steps == 0) return LBM_OK;
-    const lbm_status sum = summary(h, flags, bc, n_steps, s);
+    // (flags and bc cannot change inside the run: one check and one build of the masks)
+    Masks masks;
+    const lbm_status sum = summary(h, flags, bc, n_steps, s, masks);
     if (sum != LBM_OK) return sum;
-    auto launch_k = [&](int64_t k) -> lbm_status {
+    auto launch_k = [&](int64_t k, cudaStream_t on) -> lbm_status {
         const bool a_is_src = ((first_step + k) % 2) == 0;
-        if (eso) return step_once(h, f_a, f_a, bc, flags, tau, a_is_src ? 1 : 0, s, false, k > 0);
-        return a_is_src ? step_once(h, f_a, f_b, bc, flags, tau, 0, s, false, k > 0)
-                        : step_once(h, f_b, f_a, bc, flags, tau, 0, s, false, k > 0);
+        if (eso) return launch_one(h, f_a, f_a, bc, flags, tau, a_is_src ? 1 : 0, masks, k > 0, on);
+        return a_is_src ? launch_one(h, f_a, f_b, bc, flags, tau, 0, masks, k > 0, on)
+                        : launch_one(h, f_b, f_a, bc, flags, tau, 0, masks, k > 0, on);
     };
     // Chunks of an even number of steps keep the buffer/parity pattern of every replay identical.
     const int64_t chunk = 64;
@@ -1005,21 +1043,13 @@ lbm_status lbm_run(lbm_handle* h, void* f_a, void* f_b, float* bc, const uint8_t
     if (n_steps >= chunk) {
         uint32_t tau_bits;
         std::memcpy(&tau_bits, &tau, 4);
-        const GraphKey key{f_a, f_b, bc, flags, tau_bits, (int)(first_step % 2), chunk, use_tile(h) ? (use_staged(h) ? 4 : use_pair(h) ? 3 : 2) : 1};
+        const GraphKey key{f_a, f_b, bc, flags, tau_bits, (int)(first_step % 2), chunk, use_tile(h) ? (use_staged(h) ? 4 : use_pair(h) ? 3 : 2) : 1, masks.cells};
         auto it = h->graphs.find(key);
         if (it == h->graphs.end()) {
             cudaGraph_t g = nullptr;
             LBM_CK(cudaStreamBeginCapture(h->capture_stream, cudaStreamCaptureModeThreadLocal));
             lbm_status st = LBM_OK;
-            for (int64_t k = 0; k < chunk && st == LBM_OK; ++k) {
-                const bool a_is_src = ((first_step + k) % 2) == 0;
-                StepArgs a = eso ? step_args(h, f_a, f_a, bc, flags, tau, a_is_src ? 1 : 0)
-                                 : (a_is_src ? step_args(h, f_a, f_b, bc, flags, tau, 0)
-                                             : step_args(h, f_b, f_a, bc, flags, tau, 0));
-                a.masks_ready = k > 0 ? 1 : 0;
-                const StepLaunch fn = step_fn(h, a);
-                if (fn(a, h->threads, h->capture_stream) != cudaSuccess) st = LBM_ECUDA;
-            }
+            for (int64_t k = 0; k < chunk && st == LBM_OK; ++k) st = launch_k(k, h->capture_stream);
             cudaError_t e = cudaStreamEndCapture(h->capture_stream, &g);
             if (st != LBM_OK || e != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
@@ -1034,10 +1064,10 @@ lbm_status lbm_run(lbm_handle* h, void* f_a, void* f_b, float* bc, const uint8_t
         for (; done + chunk <= n_steps; done += chunk) LBM_CK(cudaGraphLaunch(it->second, s));
     }
     for (; done < n_steps; ++done) {
-        const lbm_status st = launch_k(done);
+        const lbm_status st = launch_k(done, s);
         if (st != LBM_OK) return st;
     }
-    return run_enqueued(h, s);
+    return LBM_OK;
 }
 
 lbm_status lbm_init_equilibrium(lbm_handle* h, void* f, float rho, float tau, const float* u, const float* grad,
