@@ -23,6 +23,7 @@ struct BatchArgs {
     const StepArgs* dom;          // ndom descriptors for this step's parity
     const uint32_t* unit_begin;   // ndom + 1 offsets of the domains' first tile units
     const uint32_t* unit_domain;  // the domain of each unit
+    const uint2* masks;           // cell masks, 256 per unit: those of the flags, or of this run
     uint32_t ndom, total_units;
     uint32_t per_cta;             // consecutive units of one CTA
     int32_t ready;                // the kernel before this one is part of the same run (its descriptors and
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(256, (batch_min_blocks<L, COLL, LINKS>())) ste
         const uint32_t tile = w.tile(b, &sa);
         const bool general = tile_general(load_near(sa.tile_near + tile), tid);
         uint2 m = make_uint2(0u, 0u);
-        if (general) m = load_masks(sa.cell_masks + (tid + kTileCells * tile));
+        if (general) m = load_masks(b.masks + ((size_t)w.u * kTileCells + tid));
         if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
         waited = true;
         tile_forms<L, METHOD, F16C, COLL, LES, false, LINKS, false>(sa, tile, tid, general, m, nullptr, nullptr, nullptr);
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, LBM_DOUBLE_B
     for (BatchWalk w(b); w.u < w.end; ++w.u) {
         const uint32_t tile = w.tile(b, &sa);
         PairMasks pm;
-        pm.load<false>(load_near(sa.tile_near + tile), sa.cell_masks, tile, t);
+        pm.load<false>(load_near(sa.tile_near + tile), b.masks + (size_t)w.u * kTileCells, 0u, t);
         if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
         waited = true;
         pair_step<L, LBM_DOUBLE_BUFFER, F16C, COLL, LES, false, false>(sa, tile, t, pm);

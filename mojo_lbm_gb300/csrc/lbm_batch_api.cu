@@ -10,6 +10,7 @@
 
 #include "lbm_batch.cuh"
 #include "lbm_link_tables.h"
+#include "lbm_masks.h"
 
 namespace lbm {
 void set_last_error(const char* msg);  // lbm_capi.cu
@@ -49,7 +50,8 @@ struct lbm_batch {
     uint32_t* d_changed = nullptr;    // summary round in which a box summary last changed
     uint32_t summary_gen = 0;
     bool summary_valid = false;
-    bool masks_resting = false;       // the masks are those of the last run's bc (without_resting_walls)
+    MaskOwner owner;
+    SpareBuffer run_masks;            // cell masks of the owner's run without its walls at rest
     bool dirty = true;
     BatchLaunch step = nullptr;
     BatchLaunch step_pair = nullptr;   // two cells per thread (needs 8-byte aligned buffers), or null
@@ -69,7 +71,7 @@ struct lbm_batch {
     int32_t* d_link_id = nullptr;
     int sms = 1;
     cudaStream_t capture_stream = nullptr;
-    std::map<int, cudaGraphExec_t> graphs;  // keyed by the parity of the first step and the step kernel
+    std::map<int, cudaGraphExec_t> graphs;  // keyed by the parity of the first step, the step kernel and the masks
 };
 
 namespace {
@@ -107,16 +109,17 @@ __global__ void batch_near_kernel(const BatchArgs b, const uint8_t* box_sum, uin
 }
 
 // The neighbour-solid masks of the cells of every warp with its mask bit set, one block per unit,
-// after a change of the flags in this check (*changed == gen), or always; resting_walls:
-// without_resting_walls.
+// after a change of the flags in this check (*changed == gen), or, changed null, always; masks: 256 per
+// unit; resting_walls: without_resting_walls.
 template <class L>
-__global__ void __launch_bounds__(256) batch_cell_mask_kernel(const BatchArgs b, const uint32_t* changed,
-                                                              uint32_t gen, int always, int resting_walls) {
-    if (!always && *changed != gen) return;  // the same value for every thread
+__global__ void __launch_bounds__(256) batch_cell_mask_kernel(const BatchArgs b, uint2* masks, const uint32_t* changed,
+                                                              uint32_t gen, int resting_walls) {
+    if (changed && *changed != gen) return;  // the same value for every thread
     for (uint32_t u = blockIdx.x; u < b.total_units; u += gridDim.x) {  // blocks stride over the units
         const uint32_t d = find_domain(b.unit_begin, b.ndom, u);
         const StepArgs& a = b.dom[d];
-        tile_cell_masks<L>(a, u - b.unit_begin[d], const_cast<uint2*>(a.cell_masks), resting_walls != 0);
+        const uint32_t first = b.unit_begin[d];
+        tile_cell_masks<L>(a, u - first, masks + (size_t)first * kTileCells, resting_walls != 0);
     }
 }
 
@@ -171,12 +174,13 @@ uint32_t units_per_cta(const lbm_batch* b, bool pair) {
 // One step of every domain: the step kernel, then the link-wise bounce-back (or the
 // step kernel with the links fused in).
 // ready: the previous kernel in the stream is part of the same run.
-lbm_status batch_step(lbm_batch* b, bool parity_odd, bool ready, cudaStream_t s) {
+lbm_status batch_step(lbm_batch* b, bool parity_odd, const uint2* masks, bool ready, cudaStream_t s) {
     BatchArgs a;
     a.dom = parity_odd ? b->d_odd : b->d_even;
     a.ready = ready ? 1 : 0;
     a.unit_begin = b->d_begin;
     a.unit_domain = b->d_unit_domain;
+    a.masks = masks;
     a.ndom = (uint32_t)b->ndom;
     a.total_units = b->unit_begin.back();
     a.per_cta = units_per_cta(b, use_batch_pair(b) && !fused_links(b));
@@ -332,6 +336,7 @@ lbm_status lbm_batch_destroy(lbm_batch* b) {
     cudaFree(b->d_tile_near);
     cudaFree(b->d_flags_seen);
     cudaFree(b->d_cell_masks);
+    b->run_masks.release();
     cudaFree(b->d_changed);
     free_tables(b);
     if (b->capture_stream) cudaStreamDestroy(b->capture_stream);
@@ -373,7 +378,7 @@ lbm_status lbm_batch_set_domain(lbm_batch* b, int32_t i, void* f_a, void* f_b, f
     a.cap_rho = b->cfg.capture_density;
     a.cap_u = b->cfg.capture_velocity;
     a.tile_near = b->d_tile_near + b->unit_begin[i];
-    a.cell_masks = b->d_cell_masks + (size_t)b->unit_begin[i] * kTileCells;
+    a.cell_masks = nullptr;  // (BatchArgs::masks)
     a.mx = (uint32_t)g.tx - 1u;
     a.my = (uint32_t)g.ty - 1u;
     a.shx = (uint32_t)ilog2(g.tx);
@@ -449,8 +454,11 @@ lbm_status lbm_batch_run(lbm_batch* b, int64_t n_steps, int64_t first_step, void
         LBM_BCK(cudaStreamSynchronize(s));  // the host descriptors may change after return
         b->dirty = false;
     }
+    const uint2* masks = b->d_cell_masks;
     {
+        const bool capturing = is_captured(s);
         BatchArgs a;
+        a.masks = nullptr;
         a.dom = b->d_even;
         a.unit_begin = b->d_begin;
         a.unit_domain = b->d_unit_domain;
@@ -465,38 +473,44 @@ lbm_status lbm_batch_run(lbm_batch* b, int64_t n_steps, int64_t first_step, void
                                                                          b->d_changed, b->summary_gen,
                                                                          b->summary_valid ? 0 : 1);
         LBM_BCK(cudaGetLastError());
-        b->summary_valid = true;
+        if (!capturing) b->summary_valid = true;  // (what a capture records has not run)
         if (nboxes)
             batch_near_kernel<<<(nboxes + 255u) / 256u, 256, 0, s>>>(a, b->d_box_sum, b->d_tile_near, b->d_changed,
                                                                     b->summary_gen);
         LBM_BCK(cudaGetLastError());
         if (nboxes) {
             const uint32_t grid = std::min<uint32_t>(a.total_units, (uint32_t)b->sms * 8u);
+            auto build = [&](uint2* out, const uint32_t* changed, int resting) {
+                if (b->lattice == LBM_D2Q9)
+                    batch_cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, out, changed, b->summary_gen, resting);
+                else if (b->lattice == LBM_D3Q19)
+                    batch_cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, out, changed, b->summary_gen, resting);
+                else
+                    batch_cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, out, changed, b->summary_gen, resting);
+            };
+            build(b->d_cell_masks, b->d_changed, 0);
             // masks without the walls at rest serve this run only (lbm_run)
-            const bool resting = b->cfg.include_moving_boundary && !b->cfg.capture_density &&
-                                 !b->cfg.capture_velocity && n_steps >= 32;
-            const bool always = resting || b->masks_resting;
-            b->masks_resting = resting;
-            if (b->lattice == LBM_D2Q9)
-                batch_cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen, always, resting);
-            else if (b->lattice == LBM_D3Q19)
-                batch_cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen, always, resting);
-            else
-                batch_cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, b->d_changed, b->summary_gen, always, resting);
+            if (b->cfg.include_moving_boundary && !b->cfg.capture_density && !b->cfg.capture_velocity &&
+                n_steps >= kRestingMinSteps && !capturing && b->owner.is(s) &&
+                b->run_masks.get(sizeof(uint2) * (size_t)a.total_units * kTileCells)) {
+                uint2* run = static_cast<uint2*>(b->run_masks.p);
+                build(run, nullptr, 1);
+                masks = run;
+            }
         }
         LBM_BCK(cudaGetLastError());
     }
     const int64_t chunk = 64;
     int64_t done = 0;
     if (n_steps >= chunk) {
-        const int key = (int)(first_step % 2) + (use_batch_pair(b) ? 2 : 0);
+        const int key = (int)(first_step % 2) + (use_batch_pair(b) ? 2 : 0) + (masks != b->d_cell_masks ? 4 : 0);
         auto it = b->graphs.find(key);
         if (it == b->graphs.end()) {
             cudaGraph_t g = nullptr;
             LBM_BCK(cudaStreamBeginCapture(b->capture_stream, cudaStreamCaptureModeThreadLocal));
             lbm_status st = LBM_OK;
             for (int64_t k = 0; k < chunk && st == LBM_OK; ++k)
-                st = batch_step(b, ((first_step + k) % 2) != 0, k > 0, b->capture_stream);
+                st = batch_step(b, ((first_step + k) % 2) != 0, masks, k > 0, b->capture_stream);
             cudaError_t e = cudaStreamEndCapture(b->capture_stream, &g);
             if (st != LBM_OK || e != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
@@ -511,7 +525,7 @@ lbm_status lbm_batch_run(lbm_batch* b, int64_t n_steps, int64_t first_step, void
         for (; done + chunk <= n_steps; done += chunk) LBM_BCK(cudaGraphLaunch(it->second, s));
     }
     for (; done < n_steps; ++done) {
-        const lbm_status st = batch_step(b, ((first_step + done) % 2) != 0, done > 0, s);
+        const lbm_status st = batch_step(b, ((first_step + done) % 2) != 0, masks, done > 0, s);
         if (st != LBM_OK) return st;
     }
     return LBM_OK;

@@ -13,6 +13,7 @@
 
 #include "lbm_aux.cuh"
 #include "lbm_link_tables.h"
+#include "lbm_masks.h"
 #include "lbm_stage.cuh"
 
 namespace lbm {
@@ -285,13 +286,10 @@ struct lbm_handle {
     uint32_t* changed;     // device word: summary round in which a box summary last changed
     uint32_t summary_gen;  // summary rounds issued
     int summary_valid;     // box_sum and flags_seen hold a complete summary
-    // What depends on bc, or on flags that other streams need not share, belongs to the first stream that
-    // steps the handle outside a capture (owner): run_masks (block-per-tile kernels), cell_masks and what
-    // they are built from (generic kernel).
-    int owned;
-    unsigned long long owner;  // cudaStreamGetId
-    uint2* run_masks;      // cell masks of a run without its walls at rest (without_resting_walls), or null
-    int run_masks_failed;  // no memory for them
+    // What depends on bc, or on flags that other streams need not share, belongs to one stream:
+    // run_masks (block-per-tile kernels), cell_masks and what they are built from (generic kernel).
+    MaskOwner owner;
+    SpareBuffer run_masks;  // cell masks of a run without its walls at rest (without_resting_walls)
     int masks_resting;     // generic kernel: cell_masks are those of the last run's bc
     uint8_t* tile_near;    // per tile: warp_near bits of its 8 warp boxes (block-per-tile kernel)
     uint32_t ntiles;
@@ -484,27 +482,16 @@ lbm_status tile_summary(lbm_handle* h, const uint8_t* flags, bool capturing, cud
     return LBM_OK;
 }
 
-// The cell masks of one run without its walls at rest, in run_masks; false without the memory for them (8
-// bytes per cell, taken by the first such run).
-bool have_run_masks(lbm_handle* h) {
-    if (h->run_masks || h->run_masks_failed) return h->run_masks != nullptr;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (another stream may be captured meanwhile)
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (cudaMalloc(&h->run_masks, sizeof(uint2) * (size_t)h->lay.ncells) != cudaSuccess) {
-        cudaGetLastError();  // cleared: the runs take the masks of the flags
-        h->run_masks = nullptr;
-        h->run_masks_failed = 1;
-    }
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    return h->run_masks != nullptr;
-}
+// The cell masks of one run without its walls at rest, in run_masks (8 bytes per cell, taken by the first
+// such run).
 lbm_status build_run_masks(lbm_handle* h, const uint8_t* flags, float* bc, cudaStream_t s) {
     const StepArgs a = step_args(h, nullptr, nullptr, bc, flags, 1.f, 0, Masks{h->tile_near, h->cell_masks});
     const uint32_t grid = std::min<uint32_t>(h->ntiles, (uint32_t)h->sm_count * 8u);
+    uint2* masks = static_cast<uint2*>(h->run_masks.p);
     switch (h->grid.lattice) {
-        case LBM_D2Q9: cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, h->run_masks, nullptr, 0u, h->ntiles, 1); break;
-        case LBM_D3Q19: cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, h->run_masks, nullptr, 0u, h->ntiles, 1); break;
-        default: cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, h->run_masks, nullptr, 0u, h->ntiles, 1); break;
+        case LBM_D2Q9: cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, masks, nullptr, 0u, h->ntiles, 1); break;
+        case LBM_D3Q19: cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, masks, nullptr, 0u, h->ntiles, 1); break;
+        default: cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, masks, nullptr, 0u, h->ntiles, 1); break;
     }
     LBM_CK(cudaGetLastError());
     return LBM_OK;
@@ -530,43 +517,18 @@ lbm_status any_summary(lbm_handle* h, const uint8_t* flags, const float* bc, boo
     return LBM_OK;
 }
 
-// From this many steps on a run builds its masks without the walls at rest: the unconditional rebuild
-// (62 us on 256^3 cells, 4 us on 256^2) costs less than the bc reads it saves (15 to 23 us and 0.4 us a
-// step).
-constexpr int64_t kRestingMinSteps = 32;
-
-// Is s the stream whose calls, outside captures, own the handle's masks (lbm_handle::owner)?  The first one
-// to ask is.  (By its id: the per-thread default streams share a handle value, and a destroyed stream's is
-// given out again.)
-bool owns_masks(lbm_handle* h, cudaStream_t s) {
-    unsigned long long id = 0;
-    if (cudaStreamGetId(s, &id) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (!h->owned) {
-        h->owned = 1;
-        h->owner = id;
-    }
-    return id == h->owner;
-}
-
 // The masks for n_steps steps of the kernel that the handle is set to, brought up to date with `flags` (and
 // bc) on s.
-// Calls may overlap on several streams with bc of their own (the generic kernel: with flags of their own),
-// and a call captured into a caller's graph is replayed at times and on streams that the handle does not
-// see.  So masks that another call may read while this one builds come from the flags alone: those of the
-// block-per-tile kernels, which all such calls share (a rebuild for the same flags writes the same words).
-// Masks of a run's bc, and all of the generic kernel's, are the owner's, whose calls are ordered by its
-// stream; other streams and captured calls take the masks of the flags, or gather the neighbours' flags.
+// The block-per-tile kernels' masks of the flags are shared by all calls (a rebuild for the same flags
+// writes the same words).  Masks of a run's bc, and all of the generic kernel's, whose calls may overlap
+// with flags of their own, are the owner's (lbm_masks.h); other streams and captured calls take the masks
+// of the flags, or gather the neighbours' flags.
 lbm_status summary(lbm_handle* h, const uint8_t* flags, float* bc, int64_t n_steps, cudaStream_t s, Masks& m) {
     m = Masks{nullptr, nullptr};
     const bool walls = h->cfg.include_moving_boundary && !h->cfg.capture_density && !h->cfg.capture_velocity;
     bool resting = walls && n_steps >= kRestingMinSteps;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) cudaGetLastError();  // (legacy stream during a capture)
-    const bool capturing = cs != cudaStreamCaptureStatusNone;
-    const bool own = !capturing && (resting || !use_tile(h)) && owns_masks(h, s);
+    const bool capturing = is_captured(s);
+    const bool own = !capturing && (resting || !use_tile(h)) && h->owner.is(s);
     if (!use_tile(h) && !own) return LBM_OK;
     resting = resting && own;
     if (!h->step_tile) {
@@ -576,8 +538,8 @@ lbm_status summary(lbm_handle* h, const uint8_t* flags, float* bc, int64_t n_ste
     }
     m = Masks{h->tile_near, h->cell_masks};
     lbm_status st = tile_summary(h, flags, capturing, s);
-    if (st == LBM_OK && resting && have_run_masks(h)) {
-        m.cells = h->run_masks;
+    if (st == LBM_OK && resting && h->run_masks.get(sizeof(uint2) * (size_t)h->lay.ncells)) {
+        m.cells = static_cast<const uint2*>(h->run_masks.p);
         st = build_run_masks(h, flags, bc, s);
     }
     return st;
@@ -765,10 +727,6 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
     h->changed = nullptr;
     h->summary_gen = 0;
     h->summary_valid = 0;
-    h->owned = 0;
-    h->owner = 0;
-    h->run_masks = nullptr;
-    h->run_masks_failed = 0;
     h->masks_resting = 0;
     h->tile_near = nullptr;
     h->threads = any_threads(h->cfg);
@@ -840,7 +798,7 @@ lbm_status lbm_destroy(lbm_handle* h) {
     if (h->box_sum) cudaFree(h->box_sum);
     if (h->flags_seen) cudaFree(h->flags_seen);
     if (h->cell_masks) cudaFree(h->cell_masks);
-    if (h->run_masks) cudaFree(h->run_masks);
+    h->run_masks.release();
     if (h->changed) cudaFree(h->changed);
     if (h->tile_near) cudaFree(h->tile_near);
     if (h->closure) cudaFree(h->closure);

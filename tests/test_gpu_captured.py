@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from mojo_lbm_gb300 import Flags, LBM_Config, LBM_method
+from mojo_lbm_gb300.batch import BatchSolver
 from mojo_lbm_gb300.solver import Solver
 from tests.lbm_cases import initial_f, make_grid, mixed_flags
 from tests.test_gpu_step import to_dev
@@ -65,3 +66,32 @@ def test_captured_runs_equal_single_steps(lat, shape, tile, meth, f16, order):
 
     _play(order, lambda n, stream: s.run(a1, b1, bc, fl, 0.8, n, 0, stream),
           lambda rest: bc.copy_(torch.from_numpy(_bc(grid, rng, rest))), check)
+
+
+@pytest.mark.parametrize("order", [o for o in ORDERS if o[0] == "r"])
+def test_captured_batch_runs_equal_single_steps(order):
+    """(The first run of a batch uploads its descriptors and cannot be captured.)"""
+    grids = [make_grid("D2Q9", (32, 16 * k, 1), (16, 16, 1)) for k in (1, 3, 2)]
+    cfg = LBM_Config(LBM_method.DOUBLE_BUFFER, BCs={Flags.EQUILIBRIUM})
+    rng = np.random.default_rng(7)
+    batch = BatchSolver(grids, cfg)
+    doms = []
+    for i, g in enumerate(grids):
+        flags, _ = mixed_flags(g, rng)
+        f0 = initial_f(g, cfg, rng)
+        d = dict(grid=g, solver=Solver(g, cfg), fl=to_dev(flags), bc=to_dev(_bc(g, rng, 0.6)),
+                 f=[to_dev(f0) for _ in range(4)])
+        batch.set_domain(i, d["f"][0], d["f"][1], d["bc"], d["fl"], 0.8)
+        doms.append(d)
+
+    def new_bc(rest):
+        for d in doms:
+            d["bc"].copy_(torch.from_numpy(_bc(d["grid"], rng, rest)))
+
+    def check(n, what):
+        for d in doms:
+            _one_by_one(d["solver"], cfg, d["f"][2], d["f"][3], d["bc"], d["fl"], 0.8, n)
+            for k in (0, 1):
+                assert torch.equal(d["f"][k].view(torch.int32), d["f"][2 + k].view(torch.int32)), what
+
+    _play(order, lambda n, stream: batch.run(n, 0, stream), new_bc, check)
