@@ -109,17 +109,19 @@ __global__ void batch_near_kernel(const BatchArgs b, const uint8_t* box_sum, uin
 }
 
 // The neighbour-solid masks of the cells of every warp with its mask bit set, one block per unit,
-// after a change of the flags in this check (*changed == gen), or, changed null, always; masks: 256 per
-// unit; resting_walls: without_resting_walls.
+// after a change of the flags in this check (*changed == gen), and with run always those without the walls
+// at rest (without_resting_walls); 256 per unit each.
 template <class L>
-__global__ void __launch_bounds__(256) batch_cell_mask_kernel(const BatchArgs b, uint2* masks, const uint32_t* changed,
-                                                              uint32_t gen, int resting_walls) {
-    if (changed && *changed != gen) return;  // the same value for every thread
+__global__ void __launch_bounds__(256) batch_cell_mask_kernel(const BatchArgs b, uint2* masks, uint2* run,
+                                                              const uint32_t* changed, uint32_t gen) {
+    const bool rebuild = *changed == gen;  // the same value for every thread
+    if (!rebuild && !run) return;
     for (uint32_t u = blockIdx.x; u < b.total_units; u += gridDim.x) {  // blocks stride over the units
         const uint32_t d = find_domain(b.unit_begin, b.ndom, u);
         const StepArgs& a = b.dom[d];
         const uint32_t first = b.unit_begin[d];
-        tile_cell_masks<L>(a, u - first, masks + (size_t)first * kTileCells, resting_walls != 0);
+        if (rebuild) tile_cell_masks<L>(a, u - first, masks + (size_t)first * kTileCells, false);
+        if (run) tile_cell_masks<L>(a, u - first, run + (size_t)first * kTileCells, true);
     }
 }
 
@@ -480,23 +482,18 @@ lbm_status lbm_batch_run(lbm_batch* b, int64_t n_steps, int64_t first_step, void
         LBM_BCK(cudaGetLastError());
         if (nboxes) {
             const uint32_t grid = std::min<uint32_t>(a.total_units, (uint32_t)b->sms * 8u);
-            auto build = [&](uint2* out, const uint32_t* changed, int resting) {
-                if (b->lattice == LBM_D2Q9)
-                    batch_cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, out, changed, b->summary_gen, resting);
-                else if (b->lattice == LBM_D3Q19)
-                    batch_cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, out, changed, b->summary_gen, resting);
-                else
-                    batch_cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, out, changed, b->summary_gen, resting);
-            };
-            build(b->d_cell_masks, b->d_changed, 0);
             // masks without the walls at rest serve this run only (lbm_run)
+            uint2* run = nullptr;
             if (b->cfg.include_moving_boundary && !b->cfg.capture_density && !b->cfg.capture_velocity &&
                 n_steps >= kRestingMinSteps && !capturing && b->owner.is(s) &&
-                b->run_masks.get(sizeof(uint2) * (size_t)a.total_units * kTileCells)) {
-                uint2* run = static_cast<uint2*>(b->run_masks.p);
-                build(run, nullptr, 1);
-                masks = run;
-            }
+                b->run_masks.get(sizeof(uint2) * (size_t)a.total_units * kTileCells))
+                masks = run = static_cast<uint2*>(b->run_masks.p);
+            if (b->lattice == LBM_D2Q9)
+                batch_cell_mask_kernel<D2Q9><<<grid, kTileCells, 0, s>>>(a, b->d_cell_masks, run, b->d_changed, b->summary_gen);
+            else if (b->lattice == LBM_D3Q19)
+                batch_cell_mask_kernel<D3Q19><<<grid, kTileCells, 0, s>>>(a, b->d_cell_masks, run, b->d_changed, b->summary_gen);
+            else
+                batch_cell_mask_kernel<D3Q27><<<grid, kTileCells, 0, s>>>(a, b->d_cell_masks, run, b->d_changed, b->summary_gen);
         }
         LBM_BCK(cudaGetLastError());
     }
