@@ -303,6 +303,7 @@ struct lbm_handle {
     // run_masks (block-per-tile kernels), cell_masks and what they are built from (generic kernel).
     MaskOwner owner;
     SpareBuffer run_masks;  // cell masks of a run without its walls at rest (without_resting_walls)
+    SpareBuffer any;        // the generic kernel's masks on a grid that is not tiled for the others (any_masks)
     int masks_resting;     // generic kernel: cell_masks are those of the last run's bc
     uint8_t* tile_near;    // per tile: warp_near bits of its 8 warp boxes (block-per-tile kernel)
     uint32_t ntiles;
@@ -500,6 +501,25 @@ lbm_status tile_summary(lbm_handle* h, const uint8_t* flags, float* bc, uint2* r
     return LBM_OK;
 }
 
+// The generic kernel's masks on a grid that is not tiled for the others, 9 bytes per cell taken by the first
+// call that uses them; false without the memory.
+bool any_masks(lbm_handle* h, cudaStream_t s) {
+    if (h->any.p) return true;
+    auto up = [](size_t v) { return (v + 15u) & ~(size_t)15u; };
+    const size_t n = h->lay.ncells, cells = up(sizeof(uint2) * n), seen = up(n), near = up((n + 255u) / 256u);
+    if (!h->any.get(cells + seen + near + sizeof(uint32_t))) return false;
+    char* p = static_cast<char*>(h->any.p);
+    if (cudaMemsetAsync(p + cells, 0, seen + near + sizeof(uint32_t), s) != cudaSuccess) {
+        h->any.release();
+        return false;
+    }
+    h->cell_masks = reinterpret_cast<uint2*>(p);
+    h->flags_seen = reinterpret_cast<uint8_t*>(p + cells);
+    h->tile_near = reinterpret_cast<uint8_t*>(p + cells + seen);
+    h->changed = reinterpret_cast<uint32_t*>(p + cells + seen + near);
+    return true;
+}
+
 // The same for the generic kernel's masks, which only the owner's calls use: without the walls at rest
 // (resting) in place of the masks of the flags, until the next call rebuilds them.
 lbm_status any_summary(lbm_handle* h, const uint8_t* flags, const float* bc, bool resting, cudaStream_t s) {
@@ -520,6 +540,22 @@ lbm_status any_summary(lbm_handle* h, const uint8_t* flags, const float* bc, boo
     return LBM_OK;
 }
 
+// Does a call of n steps of the generic kernel use its masks?  Checking the flags and building the masks are
+// two launches before the first step; gathering the neighbours' flags costs every step.  us a step, gather /
+// masks, float32 cavities:
+//   1 step    33 x 17 3.4 / 10.3, 1001 x 999 21.1 / 24.6, 63 x 61 x 65 13.8 / 18.5, 150 x 131 x 97 75.9 / 76.7
+//   2 steps   511 x 513 11.1 / 12.4, 1001 x 999 24.5 / 23.6, 33 x 35 x 31 9.1 / 11.0, 63 x 61 x 65 17.4 / 16.9
+//   4 steps   255 x 257 5.4 / 6.3, 511 x 513 9.1 / 8.9, 33 x 35 x 31 7.2 / 7.7
+//   8 steps   100 x 80 3.8 / 4.0, 255 x 257 4.5 / 4.9, 33 x 35 x 31 6.3 / 6.1, D3Q27 7.6 / 7.5
+//   16 steps  33 x 17 3.1 / 3.2, 100 x 80 3.4 / 3.2, 255 x 257 4.2 / 4.0, 20^3 5.5 / 5.3
+//   64 steps  33 x 17 2.3 / 2.1, 1001 x 999 20.5 / 16.9, 150 x 131 x 97 75.3 / 60.8
+bool masks_pay(const lbm_handle* h, int64_t n) {
+    const bool flat = lattice_d(h->grid.lattice) == 2;
+    const int64_t cells = h->lay.ncells;
+    if (n == 1) return cells >= (flat ? 1 << 22 : 1 << 21);
+    return n >= 16 || n * (cells + (flat ? 1 << 16 : 1 << 15)) >= (flat ? 1 << 20 : 1 << 19);
+}
+
 // The masks for n_steps steps of the kernel that the handle is set to, brought up to date with `flags` (and
 // bc) on s.
 // The block-per-tile kernels' masks of the flags are shared by all calls (a rebuild for the same flags
@@ -531,11 +567,11 @@ lbm_status summary(lbm_handle* h, const uint8_t* flags, float* bc, int64_t n_ste
     const bool walls = h->cfg.include_moving_boundary && !h->cfg.capture_density && !h->cfg.capture_velocity;
     bool resting = walls && n_steps >= kRestingMinSteps;
     const bool capturing = is_captured(s);
-    const bool own = !capturing && (resting || !use_tile(h)) && h->owner.is(s);
+    const bool own = !capturing && (use_tile(h) ? resting : masks_pay(h, n_steps)) && h->owner.is(s);
     if (!use_tile(h) && !own) return LBM_OK;
     resting = resting && own;
     if (!h->step_tile) {
-        if (!h->tile_near) return LBM_OK;
+        if (!any_masks(h, s)) return LBM_OK;
         m = Masks{h->tile_near, h->cell_masks};
         return any_summary(h, flags, bc, resting, s);
     }
@@ -757,32 +793,6 @@ lbm_status lbm_create(const lbm_config_t* cfg, const lbm_grid_t* grid, lbm_handl
     if (e == cudaSuccess && !segs.empty()) e = cudaMalloc(&h->stage_segs, sizeof(StageSeg) * segs.size());
     if (e == cudaSuccess && !segs.empty())
         e = cudaMemcpy(h->stage_segs, segs.data(), sizeof(StageSeg) * segs.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !h->step_tile) {
-        // the generic kernel's masks, 9 bytes per cell: without the memory for them every step gathers
-        // the neighbours' flags instead
-        const size_t n = h->lay.ncells, chunks = (n + 255u) / 256u;
-        cudaError_t m = cudaMalloc(&h->flags_seen, n);
-        if (m == cudaSuccess) m = cudaMalloc(&h->cell_masks, sizeof(uint2) * n);
-        if (m == cudaSuccess) m = cudaMalloc(&h->changed, sizeof(uint32_t));
-        if (m == cudaSuccess) m = cudaMalloc(&h->tile_near, chunks);
-        if (m == cudaSuccess) {
-            e = cudaMemset(h->flags_seen, 0, n);
-            if (e == cudaSuccess) e = cudaMemset(h->changed, 0, sizeof(uint32_t));
-            if (e == cudaSuccess) e = cudaMemset(h->tile_near, 0, chunks);
-        } else if (m == cudaErrorMemoryAllocation) {
-            cudaGetLastError();  // cleared: the handle works without
-            cudaFree(h->flags_seen);
-            cudaFree(h->cell_masks);
-            cudaFree(h->changed);
-            cudaFree(h->tile_near);
-            h->flags_seen = nullptr;
-            h->cell_masks = nullptr;
-            h->changed = nullptr;
-            h->tile_near = nullptr;
-        } else {
-            e = m;
-        }
-    }
     if (e != cudaSuccess) {
         lbm_destroy(h);
         return fail(LBM_ECUDA, std::string("lbm_create: ") + cudaGetErrorString(e));
@@ -796,11 +806,14 @@ lbm_status lbm_destroy(lbm_handle* h) {
     for (auto& kv : h->graphs) cudaGraphExecDestroy(kv.second);
     if (h->scratch) cudaFree(h->scratch);
     if (h->box_sum) cudaFree(h->box_sum);
-    if (h->flags_seen) cudaFree(h->flags_seen);
-    if (h->cell_masks) cudaFree(h->cell_masks);
+    if (h->step_tile) {  // (else parts of h->any)
+        if (h->flags_seen) cudaFree(h->flags_seen);
+        if (h->cell_masks) cudaFree(h->cell_masks);
+        if (h->changed) cudaFree(h->changed);
+        if (h->tile_near) cudaFree(h->tile_near);
+    }
+    h->any.release();
     h->run_masks.release();
-    if (h->changed) cudaFree(h->changed);
-    if (h->tile_near) cudaFree(h->tile_near);
     if (h->closure) cudaFree(h->closure);
     if (h->link_table) cudaFree(h->link_table);
     if (h->link_dist) cudaFree(h->link_dist);
