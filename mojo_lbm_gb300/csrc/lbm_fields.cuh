@@ -40,7 +40,8 @@ __device__ __forceinline__ void cell_nbr(const LayoutDesc& lay, const Cell& c, N
 
 // The bricks of a grid.  A warp's 32 lanes are 2^sbx cells along x times 2^sby along y.  3D: a
 // brick has 2^sp planes along z, field row g = lx 2^sby + ly, fast index z.  2D: its planes follow
-// each other along y, row g = lx, fast index y (2^(sp + sby) of them).
+// each other along y, row g = lx, fast index y (2^(sp + sby) of them); a brick is in one plane z (of the
+// only one, unless the 2D lattice's grid extends along z: CellDeltas).
 struct Brick {
     uint32_t sbx, sby;        // sbx + sby = 5
     uint32_t sp, sf;          // log2 of the planes and of a field row's length
@@ -98,7 +99,7 @@ __device__ __forceinline__ void brick_origin(const Brick& b, int D, int32_t& x0,
     const uint32_t k = blockIdx.x, r = k / b.nbx;
     x0 = (int32_t)((k - r * b.nbx) << b.sbx);
     y0 = (int32_t)((r % b.nby) << (D == 3 ? b.sby : b.sby + b.sp));
-    z0 = (int32_t)((r / b.nby) << b.sp);
+    z0 = (int32_t)((r / b.nby) << (D == 3 ? b.sp : 0u));
 }
 
 __device__ __forceinline__ Cell locate_cell(const LayoutDesc& l, const Brick& b, int32_t x, int32_t y, int32_t z) {
@@ -140,6 +141,13 @@ __device__ __forceinline__ void fill_planes(const LayoutDesc& l, const Brick& b,
     __syncthreads();
 }
 
+// The part of plane z in a cell's flag index (per = T) or population offset (per = T Q).
+template <class Off>
+__device__ __forceinline__ Off plane_offset(const LayoutDesc& l, const Brick& b, int32_t z, Off per) {
+    const uint32_t bz = b.d_tz.div((uint32_t)z), lz = (uint32_t)z - bz * (uint32_t)l.tz;
+    return (Off)lz * (Off)(l.tx * l.ty) + per * (Off)bz * (Off)(l.ntx * l.nty);
+}
+
 // The flags of the brick and its rim (periodic) into fl[rx + RX (ry + RY rz)] (2D: rz = 0); cells more
 // than one past the grid's end are nobody's neighbour and read 0.  Returns (block-wide) whether any
 // is not 0.  Each thread keeps one (x, y) of the rim's cross-section (3D) or one x (2D) and walks the
@@ -168,12 +176,13 @@ __device__ __forceinline__ bool stage_brick_flags(const uint8_t* __restrict__ fl
                 any = any || v != 0;
             }
         } else {
+            const uint32_t nz = plane_offset(l, b, z0, l.T);
             for (uint32_t k = grp; k < b.ry; k += groups) {
                 const int32_t y = y0 + (int32_t)k - 1;
                 const uint32_t wy = (uint32_t)col(y, l.ny), by = l.d_ty.div(wy);
                 uint8_t v = 0;
                 if (x <= l.nx && y <= l.ny)
-                    v = __ldg(flags + nx + (wy - by * (uint32_t)l.ty) * (uint32_t)l.tx + l.T * by * (uint32_t)l.ntx);
+                    v = __ldg(flags + nz + nx + (wy - by * (uint32_t)l.ty) * (uint32_t)l.tx + l.T * by * (uint32_t)l.ntx);
                 fl[s + S * k] = v;
                 any = any || v != 0;
             }
@@ -252,7 +261,8 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
     int32_t x0, y0, z0;
     brick_origin(b, D, x0, y0, z0);
     if constexpr (D == 3) fill_planes<Off>(a.lay, b, z0, TQ, planes);
-    const bool flagged = stage_brick_flags<D, Off>(a.flags, a.lay, b, x0, y0, z0, planes, fl);
+    const bool other_plane = D == 2 && a.lay.nz > 1;  // the neighbours are not those of the staged plane
+    const bool flagged = stage_brick_flags<D, Off>(a.flags, a.lay, b, x0, y0, z0, planes, fl) || other_plane;
 
     const uint32_t lane = threadIdx.x & 31u;
     const int32_t lx = (int32_t)(lane & ((1u << b.sbx) - 1u)), ly = (int32_t)(lane >> b.sbx);
@@ -260,7 +270,8 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
     const S* fin = (const S*)a.f;
     const bool ddf = a.ddf != 0;
     const int32_t x = x0 + lx;
-    CellDeltas<Off> d;
+    CellDeltas<Off, D> d;
+    const Off own_z = D == 2 && a.lay.nz > 1 ? plane_offset(a.lay, b, z0, TQ) : 0;  // (3D: planes.own)
     Off own_xy;  // the cell's population offset without the planes' (3D) or rows' (2D) part
     auto row_deltas = [&](int32_t y) -> Off {
         const uint32_t by = a.lay.d_ty.div((uint32_t)y), iy = (uint32_t)y - by * (uint32_t)a.lay.ty;
@@ -275,7 +286,7 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
     }
 #pragma unroll 1
     for (int32_t p = (int32_t)(threadIdx.x >> 5); p < (1 << b.sp); p += (int32_t)(kBrickThreads / 32u)) {
-        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : 0;
+        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : z0;
         if (x >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
         const uint32_t slot = D == 3 ? ((uint32_t)((lx << b.sby) + ly) * ((1u << sf) + 1u) + (uint32_t)p)
                                      : (uint32_t)lx * ((1u << sf) + 1u) + (uint32_t)((p << b.sby) + ly);
@@ -286,7 +297,8 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
             d.z[0] = planes.own[p] - oz;
             d.z[2] = planes.own[p + 2] - oz;
         } else {
-            d.own = own_xy + row_deltas(y);
+            d.flat = own_xy + row_deltas(y);
+            d.own = d.flat + own_z;
         }
         if constexpr (!QCRIT) {
             if (flagged && fl[at] == LBM_FLAG_SOLID) {
@@ -319,13 +331,23 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
         }
         if (flagged) {
             uint32_t raw_solid = 0u, nib_solid = 0u;
-            static_for<1, Q>([&](auto qc) {
-                constexpr int q = qc.value;
-                const int32_t o = -L::c(q, 0) - (int32_t)b.rx * (L::c(q, 1) + (int32_t)b.ry * L::c(q, 2));
-                const uint8_t pf = fl[(int32_t)at + o];
-                if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
-                if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
-            });
+            if (other_plane) {
+                Nbr nb;
+                const Cell c = locate_cell(a.lay, b, x, y, z);
+                cell_nbr<L>(a.lay, c, nb);
+                uint32_t any;
+                const uint2 m = any_solid_masks<L>(a.flags, 0u, a.lay, nb, any);
+                raw_solid = m.x & ~1u;
+                nib_solid = m.y & ~1u;
+            } else {
+                static_for<1, Q>([&](auto qc) {
+                    constexpr int q = qc.value;
+                    const int32_t o = -L::c(q, 0) - (int32_t)b.rx * (L::c(q, 1) + (int32_t)b.ry * L::c(q, 2));
+                    const uint8_t pf = fl[(int32_t)at + o];
+                    if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
+                    if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
+                });
+            }
             if constexpr (!ESO) {
                 if (raw_solid)
                     static_for<1, Q>([&](auto qc) {
@@ -401,7 +423,7 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
         const uint32_t fast = i & ((1u << sf) - 1u), g = i >> sf;
         const int32_t cx = (int32_t)(D == 3 ? g >> b.sby : g);
         const int32_t fx = x0 + cx;
-        const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : 0;
+        const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : z0;
         if (fx >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
         const uint32_t slot = g * ((1u << sf) + 1u) + fast;
         const uint32_t r = ((uint32_t)fx * (uint32_t)a.lay.ny + (uint32_t)y) * (uint32_t)a.lay.nz + (uint32_t)z;
@@ -471,7 +493,7 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
         for (uint32_t i = threadIdx.x; i < (32u << b.sp); i += kBrickThreads) {
             const uint32_t fast = i & ((1u << sf) - 1u), g = i >> sf;
             const int32_t x = x0 + (int32_t)(D == 3 ? g >> b.sby : g);
-            const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : 0;
+            const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : z0;
             if (x >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
             const uint32_t slot = g * ((1u << sf) + 1u) + fast;
             const uint32_t r = ((uint32_t)x * (uint32_t)a.lay.ny + (uint32_t)y) * (uint32_t)a.lay.nz + (uint32_t)z;
@@ -490,7 +512,8 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
     const int32_t lx = (int32_t)(lane & ((1u << b.sbx) - 1u)), ly = (int32_t)(lane >> b.sbx);
     const int32_t x = x0 + lx;
     S* fs = (S*)a.f;
-    CellDeltas<Off> d;
+    CellDeltas<Off, D> d;
+    const Off own_z = D == 2 && a.lay.nz > 1 ? plane_offset(a.lay, b, z0, TQ) : 0;  // (3D: planes.own)
     Off own_xy;
     auto row_deltas = [&](int32_t y) -> Off {
         const uint32_t by = a.lay.d_ty.div((uint32_t)y), iy = (uint32_t)y - by * (uint32_t)a.lay.ty;
@@ -505,7 +528,7 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
     }
 #pragma unroll 1
     for (int32_t p = (int32_t)(threadIdx.x >> 5); p < (1 << b.sp); p += (int32_t)(kBrickThreads / 32u)) {
-        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : 0;
+        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : z0;
         if (x >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
         const uint32_t slot = D == 3 ? ((uint32_t)((lx << b.sby) + ly) * ((1u << sf) + 1u) + (uint32_t)p)
                                      : (uint32_t)lx * ((1u << sf) + 1u) + (uint32_t)((p << b.sby) + ly);
@@ -515,7 +538,8 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
             d.z[0] = planes.own[p] - oz;
             d.z[2] = planes.own[p + 2] - oz;
         } else {
-            d.own = own_xy + row_deltas(y);
+            d.flat = own_xy + row_deltas(y);
+            d.own = d.flat + own_z;
         }
         float u[3] = {0.f, 0.f, 0.f};
         if (a.u) static_for<0, D>([&](auto dc) { u[dc.value] = field[dc.value][slot]; });

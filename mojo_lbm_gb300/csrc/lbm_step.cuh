@@ -128,12 +128,14 @@ __device__ __forceinline__ void axis_deltas(uint32_t l, uint32_t t, uint32_t b, 
 
 // Population offsets of a cell and its neighbours.  Off: int32_t when the lattice has fewer than
 // 2^31 elements (one three-input add and one wide multiply-add per load), else int64_t.
-template <class Off>
+// The neighbours of a 2D lattice are those in the plane z = 0 (get_adjacent_idx takes z = 0 for it), also on
+// a grid that extends along z and x or y only: flat is the cell's place in that plane.
+template <class Off, int D>
 struct CellDeltas {
-    Off own, x[3], y[3], z[3];
+    Off own, flat, x[3], y[3], z[3];
     template <int SX, int SY, int SZ>
     __device__ __forceinline__ Off at() const {
-        Off o = own;
+        Off o = D == 3 ? own : flat;
         if constexpr (SY != 0) o += y[SY + 1];
         if constexpr (SZ != 0) o += z[SZ + 1];
         if constexpr (SX != 0) o += x[SX + 1];
@@ -680,21 +682,24 @@ cudaError_t launch_pdl(void (*kernel)(P...), uint32_t grid, uint32_t block, cuda
 template <class L, class Off>
 struct AnyCell {
     uint32_t loc, tile, lx, ly, lz, bx, by, bz;
-    CellDeltas<Off> d;
+    CellDeltas<Off, L::D> d;
     __device__ __forceinline__ AnyCell(const LayoutDesc& l, uint32_t n) {
         constexpr int D = L::D;
         tile = l.d_T.div(n);
         loc = n - tile * l.T;
         const uint32_t lyz = l.d_tx.div(loc);
         lx = loc - lyz * (uint32_t)l.tx;
-        lz = D == 3 ? l.d_ty.div(lyz) : 0u;
+        const bool deep = D == 3 || l.nz > 1;  // (uniform)
+        lz = deep ? l.d_ty.div(lyz) : 0u;
         ly = lyz - lz * (uint32_t)l.ty;
         const uint32_t byz = l.d_ntx.div(tile);
         bx = tile - byz * (uint32_t)l.ntx;
-        bz = D == 3 ? l.d_nty.div(byz) : 0u;
+        bz = deep ? l.d_nty.div(byz) : 0u;
         by = byz - bz * (uint32_t)l.nty;
         const Off TQ = (Off)l.T * L::Q;
         d.own = (Off)loc + TQ * (Off)tile;
+        if constexpr (D == 2)
+            d.flat = d.own - ((Off)lz * (Off)(l.tx * l.ty) + TQ * (Off)bz * (Off)(l.ntx * l.nty));
         axis_deltas<Off>(lx, (uint32_t)l.tx, bx, (uint32_t)l.ntx, 1, TQ, d.x);
         axis_deltas<Off>(ly, (uint32_t)l.ty, by, (uint32_t)l.nty, (Off)l.tx, TQ * (Off)l.ntx, d.y);
         if constexpr (D == 3)
