@@ -85,10 +85,12 @@ __device__ __forceinline__ void block_sum_store(double (&v)[W], double* dst) {
 // needs in float64 took 2.35 ms on 256^3 cells (the populations are read in 0.19 ms); this form
 // takes 0.265 ms.
 // Each population is split exactly against two fixed grids (adding and subtracting 1.5 * 2^k rounds to
-// a multiple of 2^(k - 23)): f = h + m + l with h a multiple of 2^-21, m of 2^-42 (|m| <= 2^-22) and
-// |l| <= 2^-43.  While sum |f| < 2 a cell's sums of h and of m are exact in float32 and pass as
-// integers into 32-bit accumulators, which hold them exactly for kMassFlush cells; only the sums of l
-// round, at 2^-66, far below the float64 rounding of a sum of order 1 (2^-53).  A cell with sum |f| of
+// a multiple of 2^(k - 23)): f = h + m + l with h a multiple of 2^-21, m of 2^-41 and |l| <= 2^-42.  While
+// sum |f| < 2 a cell's sums of h are exact in float32, and so are those of m: |m| <= 2^-22, 27 of which
+// are 27 * 2^19 units of 2^-41, below 2^24 (with units of 2^-42 the sums of 17 or more could round).  Both
+// pass as integers into 32-bit accumulators, which hold them exactly for kMassFlush cells (27 * 2^25 <
+// 2^31); only the sums of l round, in float32 and at 2^-56 or below (64 cells of 27 sum to less than
+// 2^-31), where float64 holds a sum of order 1 to 2^-53.  A cell with sum |f| of
 // 2 or more, NaN, or so small that float64's relative precision would beat those absolute errors
 // (0 < sum |f| < 2^-10) is added in float64.
 constexpr int kMassFlush = 64;
@@ -103,7 +105,7 @@ struct MassSum {
     __device__ __forceinline__ void flush() {
         static_for<0, D + 1>([&](auto kc) {
             constexpr int k = kc.value;
-            acc[k] += (double)hi[k] * 0x1p-21 + ((double)mid[k] * 0x1p-42 + (double)lo[k]);
+            acc[k] += (double)hi[k] * 0x1p-21 + ((double)mid[k] * 0x1p-41 + (double)lo[k]);
             hi[k] = mid[k] = 0;
             lo[k] = 0.f;
         });
@@ -134,7 +136,7 @@ struct MassSum {
         float H[4] = {0.f, 0.f, 0.f, 0.f}, M[4] = {0.f, 0.f, 0.f, 0.f}, R[4] = {0.f, 0.f, 0.f, 0.f};
         static_for<0, Q>([&](auto qc) {
             constexpr int q = qc.value;
-            constexpr float k1 = 6.f, k2 = 1.5f * 0x1p-19f;  // multiples of 2^-21 and of 2^-42
+            constexpr float k1 = 6.f, k2 = 1.5f * 0x1p-18f;  // multiples of 2^-21 and of 2^-41
             const float h = (f[q] + k1) - k1, r = f[q] - h;
             const float m = (r + k2) - k2, l = r - m;
             H[0] += h;
@@ -149,7 +151,7 @@ struct MassSum {
         static_for<0, D + 1>([&](auto kc) {
             constexpr int k = kc.value;
             hi[k] += __float2int_rn(H[k] * 0x1p21f);
-            mid[k] += __float2int_rn(M[k] * 0x1p42f);
+            mid[k] += __float2int_rn(M[k] * 0x1p41f);
             lo[k] += R[k];
         });
         shifted += ddf ? 1 : 0;
