@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(256, (batch_min_blocks<L, COLL, LINKS>())) ste
     bool waited = !b.ready;
     for (BatchWalk w(b); w.u < w.end; ++w.u) {
         const uint32_t tile = w.tile(b, &sa);
-        const bool general = tile_general(load_near(sa.tile_near + tile), tid);
+        const bool general = tile_general(load_byte(sa.tile_near + tile), tid);
         uint2 m = make_uint2(0u, 0u);
         if (general) m = load_masks(b.masks + ((size_t)w.u * kTileCells + tid));
         if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, LBM_DOUBLE_B
     for (BatchWalk w(b); w.u < w.end; ++w.u) {
         const uint32_t tile = w.tile(b, &sa);
         PairMasks pm;
-        pm.load<false>(load_near(sa.tile_near + tile), b.masks + (size_t)w.u * kTileCells, 0u, t);
+        pm.load<false>(load_byte(sa.tile_near + tile), b.masks + (size_t)w.u * kTileCells, 0u, t);
         if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
         waited = true;
         pair_step<L, LBM_DOUBLE_BUFFER, F16C, COLL, LES, false, false>(sa, tile, t, pm);

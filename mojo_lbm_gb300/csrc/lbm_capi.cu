@@ -117,14 +117,19 @@ __device__ __forceinline__ void rebuild_tile(const StepArgs& a, uint32_t tile, u
     if (threadIdx.x == 0) near[tile] = (uint8_t)*bits;
 }
 
-// 16 flag bytes from p (byte loads when it is not 16-byte aligned).
+// 16 flag bytes from p (byte loads when it is not 16-byte aligned), in order with the grid wait: the kernel
+// before may be the one that wrote them.
 __device__ __forceinline__ uint4 load_flags16(const uint8_t* p) {
-    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0u) return __ldg(reinterpret_cast<const uint4*>(p));
+    uint4 v;
+    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0u) {
+        asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+        return v;
+    }
     uint32_t w[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-        w[k] = (uint32_t)__ldg(p + 4 * k) | ((uint32_t)__ldg(p + 4 * k + 1) << 8) | ((uint32_t)__ldg(p + 4 * k + 2) << 16) |
-               ((uint32_t)__ldg(p + 4 * k + 3) << 24);
+        w[k] = load_byte(p + 4 * k) | (load_byte(p + 4 * k + 1) << 8) | (load_byte(p + 4 * k + 2) << 16) |
+               (load_byte(p + 4 * k + 3) << 24);
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 __device__ __forceinline__ bool differ16(const uint4& x, const uint4& y) {

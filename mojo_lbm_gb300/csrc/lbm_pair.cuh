@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kPairThreads, (pair_min_blocks<L, METHOD, F16C
     pdl_wait_before_masks(a);
     constexpr bool BY_CELL = pair_by_cell<L, METHOD, F16C, COLL, LES, FAST>();
     PairMasks pm;
-    pm.load<BY_CELL>(load_near(a.tile_near + tile), a.cell_masks, tile, t);
+    pm.load<BY_CELL>(load_byte(a.tile_near + tile), a.cell_masks, tile, t);
     pdl_wait_after_masks(a);
     pair_step<L, METHOD, F16C, COLL, LES, FAST, BY_CELL>(a, tile, t, pm);
 }

@@ -638,10 +638,10 @@ __device__ __forceinline__ void pdl_wait_after_masks(const StepArgs& a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The masks' loads and the pointer to the populations, kept in order with those waits: a plain __ldg is
-// free to move above an asm statement, since the compiler takes what it reads for constant.  (volatile
-// asm statements keep their order among themselves.)
-__device__ __forceinline__ uint32_t load_near(const uint8_t* p) {
+// The loads of flags and masks and the pointer to the populations, kept in order with those waits: a plain
+// __ldg is free to move above an asm statement, since the compiler takes what it reads for constant.
+// (volatile asm statements keep their order among themselves.)
+__device__ __forceinline__ uint32_t load_byte(const uint8_t* p) {
     uint32_t v;
     asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
@@ -765,16 +765,16 @@ __device__ __forceinline__ void add_resting_walls(float (&f)[L::Q], uint32_t cle
 }
 
 // set_adjacent_flags (ops/load_and_store.mojo:270-291) of a cell of any layout: its masks; any: an own
-// or neighbouring flag is not 0.
+// or neighbouring flag is not 0.  (Flags by load_byte: a step calls this behind its grid wait.)
 template <class L>
-__device__ __forceinline__ uint2 any_solid_masks(const uint8_t* __restrict__ flags, uint32_t own, const LayoutDesc& l,
+__device__ __forceinline__ uint2 any_solid_masks(const uint8_t* flags, uint32_t own, const LayoutDesc& l,
                                                  const Nbr& nb, uint32_t& any) {
     uint32_t raw_solid = 0u, nib_solid = 0u;
     any = own;
     static_for<1, L::Q>([&](auto qc) {
         constexpr int q = qc.value;
         constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
-        const uint8_t pf = __ldg(flags + (nb.template loc<sx, sy, sz>() + l.T * nb.template til<sx, sy, sz>()));
+        const uint32_t pf = load_byte(flags + (nb.template loc<sx, sy, sz>() + l.T * nb.template til<sx, sy, sz>()));
         any |= pf;
         if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
         if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(256, (any_min_blocks<L, COLL>())) step_kernel(
     const bool in = n < a.lay.ncells;
     pdl_wait_before_masks(a);
     // (uniform over the warp: blocks are multiples of 32 threads)
-    const bool general = !a.tile_near || ((load_near(a.tile_near + (min(n, a.lay.ncells - 1u) >> 8)) >> ((n >> 5) & 7u)) & 1u) != 0u;
+    const bool general = !a.tile_near || ((load_byte(a.tile_near + (min(n, a.lay.ncells - 1u) >> 8)) >> ((n >> 5) & 7u)) & 1u) != 0u;
     uint2 m = make_uint2(0u, 0u);
     if (general && a.cell_masks && in) m = load_masks(a.cell_masks + n);
     pdl_wait_after_masks(a);
@@ -902,7 +902,7 @@ __global__ void __launch_bounds__(256, (any_min_blocks<L, COLL>())) step_kernel(
         Nbr nb;
         AnyCell<L, Off>(a.lay, n).nbr(a.lay, nb);
         uint32_t any;
-        m = any_solid_masks<L>(a.flags, __ldg(a.flags + n), a.lay, nb, any);
+        m = any_solid_masks<L>(a.flags, load_byte(a.flags + n), a.lay, nb, any);
     }
     any_cell<L, METHOD, F16C, COLL, LES, Off, true>(a, n, m);
 }
@@ -1103,17 +1103,18 @@ __device__ __forceinline__ void write_near_mask(uint32_t i, uint32_t nboxes, uin
 }
 
 // set_adjacent_flags (ops/load_and_store.mojo:270-291) for the cell at flag offset n with cell
-// deltas dc: its masks (cell_masks_of); any: an own or neighbouring flag is not 0.
+// deltas dc: its masks (cell_masks_of); any: an own or neighbouring flag is not 0.  (Flags by load_byte: the
+// check before a single step calls this behind its grid wait.)
 template <class L>
-__device__ __forceinline__ uint2 cell_solid_masks(const uint8_t* __restrict__ flags, uint32_t n,
+__device__ __forceinline__ uint2 cell_solid_masks(const uint8_t* flags, uint32_t n,
                                                   const int32_t (&dc)[3][3], uint32_t& any) {
     uint32_t raw_solid = 0u, nib_solid = 0u;
-    const uint32_t own = __ldg(flags + n);
+    const uint32_t own = load_byte(flags + n);
     any = own;
     static_for<1, L::Q>([&](auto qc) {
         constexpr int q = qc.value;
         constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
-        const uint8_t pf = __ldg(flags + ((int32_t)n + dc[0][sx + 1] + dc[1][sy + 1] + dc[2][sz + 1]));
+        const uint32_t pf = load_byte(flags + ((int32_t)n + dc[0][sx + 1] + dc[1][sy + 1] + dc[2][sz + 1]));
         any |= pf;
         if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
         if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
@@ -1490,7 +1491,7 @@ __global__ void __launch_bounds__((tile_threads<L, METHOD, F16C, COLL, LES, FAST
     constexpr uint32_t PARTS = kTileCells / NT;
     const uint32_t tile = blockIdx.x / PARTS, tid = threadIdx.x + NT * (blockIdx.x % PARTS);
     pdl_wait_before_masks(a);
-    const bool general = tile_general(load_near(a.tile_near + tile), tid);
+    const bool general = tile_general(load_byte(a.tile_near + tile), tid);
     uint2 m = make_uint2(0u, 0u);
     if (general) m = load_masks(a.cell_masks + (tid + kTileCells * tile));
     pdl_wait_after_masks(a);
