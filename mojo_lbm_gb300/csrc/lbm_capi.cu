@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) any_mask_kernel(const uint8_t* __restrict
         if (in) {
             Nbr nb;
             AnyCell<L, int64_t>(l, n).nbr(l, nb);
-            m = any_solid_masks<L>(flags, __ldg(flags + n), l, nb, any);
+            m = any_solid_masks<L, false>(flags, __ldg(flags + n), l, nb, any);
             if (bc) {
                 const uint64_t TK = (uint64_t)l.T * (L::D + 1);
                 m = without_resting_walls<L>(m, bc, l.T, [&](auto qc) -> uint64_t {

@@ -11,7 +11,8 @@
 // 256^3 D3Q19 float32 cells); what bounds them is the load latency and about 500 instructions a cell.
 // Measured there, one thread per cell in tile order before, bricks now: rho and u 1160 -> 391 us, the
 // Q-criterion 2112 -> 627 us (452 and 1120 us with the layout decoded per flag byte, 64-bit offsets
-// and the gradient weights per derivative).
+// and the gradient weights per derivative).  Few cells, thin grids and tiles of short rows do better with
+// one thread per cell and have kernels of that form (by_cell).
 #pragma once
 
 #include "lbm_step.cuh"
@@ -40,8 +41,7 @@ __device__ __forceinline__ void cell_nbr(const LayoutDesc& lay, const Cell& c, N
 
 // The bricks of a grid.  A warp's 32 lanes are 2^sbx cells along x times 2^sby along y.  3D: a
 // brick has 2^sp planes along z, field row g = lx 2^sby + ly, fast index z.  2D: its planes follow
-// each other along y, row g = lx, fast index y (2^(sp + sby) of them); a brick is in one plane z (of the
-// only one, unless the 2D lattice's grid extends along z: CellDeltas).
+// each other along y, row g = lx, fast index y (2^(sp + sby) of them).
 struct Brick {
     uint32_t sbx, sby;        // sbx + sby = 5
     uint32_t sp, sf;          // log2 of the planes and of a field row's length
@@ -68,11 +68,11 @@ constexpr uint32_t kBrickFlags = 3472;
 // warp then reads runs of 2^sbx consecutive cells of the tile.
 // Planes: 32 (whole 128-byte lines of the fields) on grids that give every resident block one such
 // brick, else 8, one per warp: on a small grid the number of blocks and the serial planes of a warp
-// count, not the width of a store (rho and u of 256^2 D2Q9 cells: 64 blocks of 32 planes took 5 us
-// more than one thread per cell, 256 blocks of 8 do not).
+// count, not the width of a store (rho and u of 256^2 D2Q9 cells: 8.5 us with 64 blocks of 32 planes, 6.3
+// with 256 blocks of 8).  So do 3D grids of up to 8 planes (512 x 512 x 8: 103 / 81 us, x 12: 136 / 158).
 inline Brick make_brick(const LayoutDesc& l, int D) {
     Brick b;
-    b.sp = l.ncells >= 1024u * 4u * 152u ? 5u : 3u;
+    b.sp = l.ncells >= 1024u * 4u * 152u && (D == 2 || l.nz > 8) ? 5u : 3u;
     uint32_t sx = 0;
     while (sx < 5u && (2u << sx) <= (uint32_t)l.tx) ++sx;
     auto waste = [&](uint32_t s) {
@@ -94,12 +94,35 @@ inline Brick make_brick(const LayoutDesc& l, int D) {
     return b;
 }
 
+// Does one thread per cell, in tile order, do without bricks?  us per call, cell / brick (D3Q19 float32 where
+// nothing else is said):
+//   few cells, where a brick's barriers and serial planes count: rho and u of 16^3 6.4 / 6.8, 32^3 6.5 / 8.3, 48^3
+//     10.6 / 8.6, D2Q9 64^2 4.4 / 6.3, 256^2 6.3 / 6.3; Q of 24^3 6.5 / 8.4, 40^3 9.3 / 10.0, 48^3 13.5 / 10.6 (the
+//     initial state gains nothing: 32^3 4.4 / 4.4, with u and grad 6.6 / 6.3)
+//   few planes: rho and u of 512 x 512 x 2 28.9 / 49.5, x 4 55.0 / 64.1, x 6 88.9 / 74.2; in 2D rows of a brick past
+//     the grid's end: rho and u of 65536 x 16 D2Q9 22.7 / 24.9, Q of x 40 69.9 / 86.5, initial state of x 4 6.3 / 8.4,
+//     x 24 16.7 / 14.6
+//   short runs of a warp's cells in the tile, where the stores of the cell's order, or all of it, are the better
+//     ones: 128^3 in tiles of 1 x 1 x 1 initial state 160 / 293, in place 197 / 357, rho and u 134 / 188, in place
+//     Float16C 112 / 186; 2 x 1 x 1 in place 82 / 198, rho and u 111 / 116; 2 x 2 x 2 initial state 41 / 78, in place 51 / 104
+//     (with u and grad 97 / 81 and 113 / 123), rho and u 113 / 87; 8 x 1 x 1 and 4 x 4 x 4 40 / 28
+// A 2D lattice on a grid that extends along z has its neighbours in another plane (CellDeltas).
+enum FieldOp { kInitOp, kRhoUOp, kQOp };
+inline bool by_cell(const LayoutDesc& l, const Brick& b, int D, FieldOp op, bool eso, bool reads = false) {
+    const uint32_t tx = (uint32_t)l.tx, ty = (uint32_t)l.ty, wx = 1u << b.sbx, wy = 1u << b.sby;
+    const uint32_t run = wx < tx ? wx : tx * (ty < wy ? ty : wy);  // consecutive cells of a tile in a warp
+    const uint64_t rows = D == 2 ? (uint64_t)b.nby << (b.sby + b.sp) : 0u, ny = (uint64_t)l.ny;
+    if (D == 2 ? l.nz > 1 : l.nz <= 4) return true;
+    if (op == kInitOp) return rows > 2u * ny || run == 1u || (run <= 4u && (eso || !reads));
+    return l.ncells <= 1u << 16 || rows * 4u > ny * 5u || run <= (op == kRhoUOp ? 2u : 1u);
+}
+
 // First cell of brick blockIdx.x.
 __device__ __forceinline__ void brick_origin(const Brick& b, int D, int32_t& x0, int32_t& y0, int32_t& z0) {
     const uint32_t k = blockIdx.x, r = k / b.nbx;
     x0 = (int32_t)((k - r * b.nbx) << b.sbx);
     y0 = (int32_t)((r % b.nby) << (D == 3 ? b.sby : b.sby + b.sp));
-    z0 = (int32_t)((r / b.nby) << (D == 3 ? b.sp : 0u));
+    z0 = (int32_t)((r / b.nby) << b.sp);
 }
 
 __device__ __forceinline__ Cell locate_cell(const LayoutDesc& l, const Brick& b, int32_t x, int32_t y, int32_t z) {
@@ -141,13 +164,6 @@ __device__ __forceinline__ void fill_planes(const LayoutDesc& l, const Brick& b,
     __syncthreads();
 }
 
-// The part of plane z in a cell's flag index (per = T) or population offset (per = T Q).
-template <class Off>
-__device__ __forceinline__ Off plane_offset(const LayoutDesc& l, const Brick& b, int32_t z, Off per) {
-    const uint32_t bz = b.d_tz.div((uint32_t)z), lz = (uint32_t)z - bz * (uint32_t)l.tz;
-    return (Off)lz * (Off)(l.tx * l.ty) + per * (Off)bz * (Off)(l.ntx * l.nty);
-}
-
 // The flags of the brick and its rim (periodic) into fl[rx + RX (ry + RY rz)] (2D: rz = 0); cells more
 // than one past the grid's end are nobody's neighbour and read 0.  Returns (block-wide) whether any
 // is not 0.  Each thread keeps one (x, y) of the rim's cross-section (3D) or one x (2D) and walks the
@@ -176,13 +192,12 @@ __device__ __forceinline__ bool stage_brick_flags(const uint8_t* __restrict__ fl
                 any = any || v != 0;
             }
         } else {
-            const uint32_t nz = plane_offset(l, b, z0, l.T);
             for (uint32_t k = grp; k < b.ry; k += groups) {
                 const int32_t y = y0 + (int32_t)k - 1;
                 const uint32_t wy = (uint32_t)col(y, l.ny), by = l.d_ty.div(wy);
                 uint8_t v = 0;
                 if (x <= l.nx && y <= l.ny)
-                    v = __ldg(flags + nz + nx + (wy - by * (uint32_t)l.ty) * (uint32_t)l.tx + l.T * by * (uint32_t)l.ntx);
+                    v = __ldg(flags + nx + (wy - by * (uint32_t)l.ty) * (uint32_t)l.tx + l.T * by * (uint32_t)l.ntx);
                 fl[s + S * k] = v;
                 any = any || v != 0;
             }
@@ -235,6 +250,77 @@ struct AxisGradient {
     }
 };
 
+// calculate_vorticity (Q_criterion.mojo:26-85) and Vector.norm_squared (sequential sum); u0: the cell's first
+// component of the stored velocity.
+template <int D>
+__device__ __forceinline__ float vorticity_squared(const LayoutDesc& l, const float* u0, const AxisGradient& gx,
+                                                   const AxisGradient& gy, const AxisGradient& gz) {
+    const size_t N = l.ncells, sx = (size_t)l.ny * (size_t)l.nz, sy = (size_t)l.nz;
+    const float *u1 = u0 + N, *u2 = u1 + N;
+    float w2 = 0.f;
+    if constexpr (D == 2) {
+        const float wz = gx.of(u1, sx) - gy.of(u0, sy);
+        w2 += wz * wz;
+    } else {
+        const float wx = gy.of(u2, sy) - gz.of(u1, 1);
+        const float wy = gz.of(u0, 1) - gx.of(u2, sx);
+        const float wz = gx.of(u1, sx) - gy.of(u0, sy);
+        w2 += wx * wx;
+        w2 += wy * wy;
+        w2 += wz * wz;
+    }
+    return w2;
+}
+
+// Density and velocity of a cell's streamed populations.
+template <class L>
+__device__ __forceinline__ void cell_moments(const float (&f)[L::Q], bool ddf, float& rho, float (&u)[3]) {
+    rho = 0.f;
+    static_for<0, L::Q>([&](auto qc) { rho += f[qc.value]; });
+    if (ddf) rho += 1.f;
+    float mom[3] = {0.f, 0.f, 0.f};
+    static_for<0, L::Q>([&](auto qc) {
+        constexpr int q = qc.value;
+        static_for<0, L::D>([&](auto dc) {
+            constexpr int d = dc.value;
+            if constexpr (L::c(q, d) > 0) mom[d] += f[q];
+            else if constexpr (L::c(q, d) < 0) mom[d] -= f[q];
+        });
+    });
+    u[0] = u[1] = u[2] = 0.f;
+    static_for<0, L::D>([&](auto dc) { u[dc.value] = mom[dc.value] / rho; });
+}
+
+// get_f_noneq_vec (post_collision False), get_non_eq_second_order_moment, get_strain_rate_tensor and its
+// norm (kernels/utils/{equilibrium,moment}.mojo), as collide: |S|^2.
+template <class L>
+__device__ __forceinline__ float strain_norm_squared(const float (&f)[L::Q], float rho, const float (&u)[3], bool ddf,
+                                                     float tau) {
+    float uu = 0.f;
+    static_for<0, L::D>([&](auto dc) { uu += u[dc.value] * u[dc.value]; });
+    float Pi[L::NS];
+    static_for<0, L::NS>([&](auto nc) { Pi[nc.value] = 0.f; });
+    for_each_feq<L>(rho, u, uu, ddf, [&](auto qc, float e) {
+        constexpr int q = decltype(qc)::value;
+        const float fn = f[q] - e;
+        static_for<0, L::NS>([&](auto nc) {
+            constexpr int n = nc.value;
+            constexpr int cc = L::c(q, sa<L>(n)) * L::c(q, sb<L>(n));
+            if constexpr (cc > 0) Pi[n] += fn;
+            else if constexpr (cc < 0) Pi[n] -= fn;
+        });
+    });
+    const float k = -1.f / (2.f * rho * (float)(1.0 / 3.0) * tau);
+    float s2 = 0.f;
+    static_for<0, L::NS>([&](auto nc) {
+        constexpr int n = nc.value;
+        const float Sn = Pi[n] * k;
+        if constexpr (sa<L>(n) != sb<L>(n)) s2 += (Sn * Sn) * 2.f;
+        else s2 += Sn * Sn;
+    });
+    return s2;
+}
+
 // calculate_rho_and_velocity (src/lbm/output/velocity.mojo:25-125): the next step's stream and
 // boundary conditions, then density and velocity; SOLID cells (raw compare) report their bc.
 // With QCRIT, calculate_Q_criterion (src/lbm/output/Q_criterion.mojo:90-216) instead: the same
@@ -261,8 +347,7 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
     int32_t x0, y0, z0;
     brick_origin(b, D, x0, y0, z0);
     if constexpr (D == 3) fill_planes<Off>(a.lay, b, z0, TQ, planes);
-    const bool other_plane = D == 2 && a.lay.nz > 1;  // the neighbours are not those of the staged plane
-    const bool flagged = stage_brick_flags<D, Off>(a.flags, a.lay, b, x0, y0, z0, planes, fl) || other_plane;
+    const bool flagged = stage_brick_flags<D, Off>(a.flags, a.lay, b, x0, y0, z0, planes, fl);
 
     const uint32_t lane = threadIdx.x & 31u;
     const int32_t lx = (int32_t)(lane & ((1u << b.sbx) - 1u)), ly = (int32_t)(lane >> b.sbx);
@@ -271,7 +356,6 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
     const bool ddf = a.ddf != 0;
     const int32_t x = x0 + lx;
     CellDeltas<Off, D> d;
-    const Off own_z = D == 2 && a.lay.nz > 1 ? plane_offset(a.lay, b, z0, TQ) : 0;  // (3D: planes.own)
     Off own_xy;  // the cell's population offset without the planes' (3D) or rows' (2D) part
     auto row_deltas = [&](int32_t y) -> Off {
         const uint32_t by = a.lay.d_ty.div((uint32_t)y), iy = (uint32_t)y - by * (uint32_t)a.lay.ty;
@@ -286,7 +370,7 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
     }
 #pragma unroll 1
     for (int32_t p = (int32_t)(threadIdx.x >> 5); p < (1 << b.sp); p += (int32_t)(kBrickThreads / 32u)) {
-        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : z0;
+        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : 0;
         if (x >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
         const uint32_t slot = D == 3 ? ((uint32_t)((lx << b.sby) + ly) * ((1u << sf) + 1u) + (uint32_t)p)
                                      : (uint32_t)lx * ((1u << sf) + 1u) + (uint32_t)((p << b.sby) + ly);
@@ -297,17 +381,16 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
             d.z[0] = planes.own[p] - oz;
             d.z[2] = planes.own[p + 2] - oz;
         } else {
-            d.flat = own_xy + row_deltas(y);
-            d.own = d.flat + own_z;
+            d.own = d.flat = own_xy + row_deltas(y);
         }
-        if constexpr (!QCRIT) {
-            if (flagged && fl[at] == LBM_FLAG_SOLID) {
+        if (flagged && fl[at] == LBM_FLAG_SOLID) {
+            if constexpr (!QCRIT) {
                 const Cell c = locate_cell(a.lay, b, x, y, z);
                 const uint64_t own_bc = c.loc + (uint64_t)T * K * c.tile;
                 static_for<0, D>([&](auto dc) { field[dc.value][slot] = a.bc[own_bc + (uint64_t)T * dc.value]; });
                 field[D][slot] = a.bc[own_bc + (uint64_t)T * D];
-                continue;
             }
+            continue;
         }
 
         // ---- stream (the loads do not wait for the flags)
@@ -331,23 +414,13 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
         }
         if (flagged) {
             uint32_t raw_solid = 0u, nib_solid = 0u;
-            if (other_plane) {
-                Nbr nb;
-                const Cell c = locate_cell(a.lay, b, x, y, z);
-                cell_nbr<L>(a.lay, c, nb);
-                uint32_t any;
-                const uint2 m = any_solid_masks<L>(a.flags, 0u, a.lay, nb, any);
-                raw_solid = m.x & ~1u;
-                nib_solid = m.y & ~1u;
-            } else {
-                static_for<1, Q>([&](auto qc) {
-                    constexpr int q = qc.value;
-                    const int32_t o = -L::c(q, 0) - (int32_t)b.rx * (L::c(q, 1) + (int32_t)b.ry * L::c(q, 2));
-                    const uint8_t pf = fl[(int32_t)at + o];
-                    if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
-                    if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
-                });
-            }
+            static_for<1, Q>([&](auto qc) {
+                constexpr int q = qc.value;
+                const int32_t o = -L::c(q, 0) - (int32_t)b.rx * (L::c(q, 1) + (int32_t)b.ry * L::c(q, 2));
+                const uint8_t pf = fl[(int32_t)at + o];
+                if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
+                if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
+            });
             if constexpr (!ESO) {
                 if (raw_solid)
                     static_for<1, Q>([&](auto qc) {
@@ -370,49 +443,13 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
                 equilibrium_bc<L>(f, a.bc, c.loc + (uint64_t)T * K * c.tile, T, x, y, z, a.lay, ddf);
             }
         }
-        float rho = 0.f;
-        static_for<0, Q>([&](auto qc) { rho += f[qc.value]; });
-        if (ddf) rho += 1.f;
-        float mom[3] = {0.f, 0.f, 0.f};
-        static_for<0, Q>([&](auto qc) {
-            constexpr int q = qc.value;
-            static_for<0, D>([&](auto dc) {
-                constexpr int d = dc.value;
-                if constexpr (L::c(q, d) > 0) mom[d] += f[q];
-                else if constexpr (L::c(q, d) < 0) mom[d] -= f[q];
-            });
-        });
+        float rho, u[3];
+        cell_moments<L>(f, ddf, rho, u);
         if constexpr (!QCRIT) {
-            static_for<0, D>([&](auto dc) { field[dc.value][slot] = mom[dc.value] / rho; });
+            static_for<0, D>([&](auto dc) { field[dc.value][slot] = u[dc.value]; });
             field[D][slot] = rho;
         } else {
-            // get_f_noneq_vec (post_collision False), get_non_eq_second_order_moment,
-            // get_strain_rate_tensor and its norm (kernels/utils/{equilibrium,moment}.mojo), as collide
-            float u[3] = {0.f, 0.f, 0.f};
-            static_for<0, D>([&](auto dc) { u[dc.value] = mom[dc.value] / rho; });
-            float uu = 0.f;
-            static_for<0, D>([&](auto dc) { uu += u[dc.value] * u[dc.value]; });
-            float Pi[L::NS];
-            static_for<0, L::NS>([&](auto nc) { Pi[nc.value] = 0.f; });
-            for_each_feq<L>(rho, u, uu, ddf, [&](auto qc, float e) {
-                constexpr int q = decltype(qc)::value;
-                const float fn = f[q] - e;
-                static_for<0, L::NS>([&](auto nc) {
-                    constexpr int n = nc.value;
-                    constexpr int cc = L::c(q, sa<L>(n)) * L::c(q, sb<L>(n));
-                    if constexpr (cc > 0) Pi[n] += fn;
-                    else if constexpr (cc < 0) Pi[n] -= fn;
-                });
-            });
-            const float k = -1.f / (2.f * rho * (float)(1.0 / 3.0) * a.tau);
-            float s2 = 0.f;
-            static_for<0, L::NS>([&](auto nc) {
-                constexpr int n = nc.value;
-                const float Sn = Pi[n] * k;
-                if constexpr (sa<L>(n) != sb<L>(n)) s2 += (Sn * Sn) * 2.f;
-                else s2 += Sn * Sn;
-            });
-            field[0][slot] = s2;
+            field[0][slot] = strain_norm_squared<L>(f, rho, u, ddf, a.tau);
         }
     }
     __syncthreads();
@@ -423,7 +460,7 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
         const uint32_t fast = i & ((1u << sf) - 1u), g = i >> sf;
         const int32_t cx = (int32_t)(D == 3 ? g >> b.sby : g);
         const int32_t fx = x0 + cx;
-        const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : z0;
+        const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : 0;
         if (fx >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
         const uint32_t slot = g * ((1u << sf) + 1u) + fast;
         const uint32_t r = ((uint32_t)fx * (uint32_t)a.lay.ny + (uint32_t)y) * (uint32_t)a.lay.nz + (uint32_t)z;
@@ -433,27 +470,97 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
         } else {
             const uint32_t at = (uint32_t)(cx + 1) + b.rx * ((uint32_t)(y - y0 + 1) + (D == 3 ? b.ry * (fast + 1u) : 0u));
             if (fl[at] == LBM_FLAG_SOLID) continue;
-            // calculate_vorticity (Q_criterion.mojo:26-85) and Vector.norm_squared (sequential sum)
             AxisGradient gx, gy, gz;
             gx.init(fx, a.lay.nx, fl[at - 1u], fl[at + 1u]);
             gy.init(y, a.lay.ny, fl[at - b.rx], fl[at + b.rx]);
             if constexpr (D == 3) gz.init(z, a.lay.nz, fl[at - b.rx * b.ry], fl[at + b.rx * b.ry]);
-            const size_t sx = (size_t)a.lay.ny * (size_t)a.lay.nz, sy = (size_t)a.lay.nz;
-            const float *u0 = a.u + r, *u1 = u0 + N, *u2 = u1 + N;
-            float w2 = 0.f;
-            if constexpr (D == 2) {
-                const float wz = gx.of(u1, sx) - gy.of(u0, sy);
-                w2 += wz * wz;
-            } else {
-                const float wx = gy.of(u2, sy) - gz.of(u1, 1);
-                const float wy = gz.of(u0, 1) - gx.of(u2, sx);
-                const float wz = gx.of(u1, sx) - gy.of(u0, sy);
-                w2 += wx * wx;
-                w2 += wy * wy;
-                w2 += wz * wz;
-            }
-            a.q[r] = 0.25f * w2 - 0.5f * field[0][slot];
+            a.q[r] = 0.25f * vorticity_squared<D>(a.lay, a.u + r, gx, gy, gz) - 0.5f * field[0][slot];
         }
+    }
+}
+
+// The same, one thread per cell in tile order (by_cell).
+template <class L, bool F16C, bool ESO, bool QCRIT, class Off>
+__global__ void __launch_bounds__(256) rho_u_cell_kernel(const __grid_constant__ RhoUArgs a) {
+    using P = Pop<F16C>;
+    using S = typename P::T;
+    constexpr int Q = L::Q, D = L::D, K = D + 1;
+    const LayoutDesc& l = a.lay;
+    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x, N = l.ncells, T = l.T;
+    if (n >= N) return;
+    const AnyCell<L, Off> c(l, n);
+    const uint32_t r = c.row(l);
+    const uint64_t own_bc = c.loc + (uint64_t)T * K * c.tile;
+    const uint8_t flag = a.flags[n];
+    if (flag == LBM_FLAG_SOLID) {
+        if constexpr (!QCRIT) {
+            static_for<0, D>([&](auto dc) { a.u[(size_t)N * dc.value + r] = a.bc[own_bc + (uint64_t)T * dc.value]; });
+            a.rho[r] = a.bc[own_bc + (uint64_t)T * D];
+        }
+        return;
+    }
+    Nbr nb;
+    c.nbr(l, nb);
+    [[maybe_unused]] uint32_t any;
+    uint2 m = make_uint2(0u, 0u);
+    if constexpr (!ESO) m = any_solid_masks<L, false>(a.flags, 0u, l, nb, any);
+    [[maybe_unused]] const uint32_t raw_solid = m.x;
+    const Off oT = (Off)T;
+    const S* fin = (const S*)a.f;
+    float f[Q];
+    if constexpr (!ESO) {
+        static_for<0, Q>([&](auto qc) {
+            constexpr int q = qc.value;
+            Off o = c.d.template at<-L::c(q, 0), -L::c(q, 1), -L::c(q, 2)>();
+            if constexpr (q > 0) {
+                if ((raw_solid >> q) & 1u) o = c.d.own + (opp<L>(q) > q ? oT : -oT);  // slot q +- 1
+            }
+            f[q] = P::ld(fin + (o + oT * q));
+        });
+    } else {
+        const bool ev = a.even != 0;
+        const S* fA = fin + (ev ? 0u : T);
+        const S* fB = fin + (ev ? T : 0u);
+        f[0] = P::ld(fin + c.d.own);
+        static_for<1, Q - 1, 2>([&](auto qc) {
+            constexpr int pos = qc.value, neg = pos + 1;
+            f[pos] = P::ld(fA + (c.d.own + oT * pos));
+            f[neg] = P::ld(fB + (c.d.template at<L::c(pos, 0), L::c(pos, 1), L::c(pos, 2)>() + oT * pos));
+        });
+        if (a.moving) m = any_solid_masks<L, false>(a.flags, 0u, l, nb, any);
+    }
+    const uint32_t nib_solid = a.moving ? m.y & ~1u : 0u;
+    if (nib_solid) {
+        const uint64_t TK = (uint64_t)T * K;
+        moving_wall<L>(f, nib_solid, a.bc, T, [&](auto qc) -> uint64_t {
+            constexpr int q = decltype(qc)::value;
+            constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
+            return nb.template loc<sx, sy, sz>() + TK * nb.template til<sx, sy, sz>();
+        });
+    }
+    const int32_t x = (int32_t)(c.bx * l.tx + c.lx), y = (int32_t)(c.by * l.ty + c.ly), z = (int32_t)(c.bz * l.tz + c.lz);
+    if (a.eqbc && (flag & 0x0F) == LBM_FLAG_EQUILIBRIUM) equilibrium_bc<L>(f, a.bc, own_bc, T, x, y, z, l, a.ddf != 0);
+    float rho, u[3];
+    cell_moments<L>(f, a.ddf != 0, rho, u);
+    if constexpr (!QCRIT) {
+        static_for<0, D>([&](auto dc) { a.u[(size_t)N * dc.value + r] = u[dc.value]; });
+        a.rho[r] = rho;
+    } else {
+        const float s2 = strain_norm_squared<L>(f, rho, u, a.ddf != 0, a.tau);
+        // the flags of the neighbours in the cell's own plane
+        const uint32_t own_z = D == 2 ? c.lz * (uint32_t)(l.tx * l.ty) + T * c.bz * (uint32_t)(l.ntx * l.nty) : 0u;
+        auto flag_at = [&](auto sx, auto sy, auto sz) {
+            constexpr int X = decltype(sx)::value, Y = decltype(sy)::value, Z = decltype(sz)::value;
+            return a.flags[own_z + nb.template loc<X, Y, Z>() + T * nb.template til<X, Y, Z>()];
+        };
+        constexpr std::integral_constant<int, 0> O{};
+        constexpr std::integral_constant<int, 1> up{};
+        constexpr std::integral_constant<int, -1> down{};
+        AxisGradient gx, gy, gz;
+        gx.init(x, l.nx, flag_at(down, O, O), flag_at(up, O, O));
+        gy.init(y, l.ny, flag_at(O, down, O), flag_at(O, up, O));
+        if constexpr (D == 3) gz.init(z, l.nz, flag_at(O, O, down), flag_at(O, O, up));
+        a.q[r] = 0.25f * vorticity_squared<D>(l, a.u + r, gx, gy, gz) - 0.5f * s2;
     }
 }
 
@@ -466,6 +573,44 @@ struct InitArgs {
     float rho, tau;
     int32_t ddf, esoteric;
 };
+
+// The initial populations of a cell with velocity u and symmetric velocity gradient S_, stored.
+template <class L, bool F16C, class Off>
+__device__ __forceinline__ void store_initial(const InitArgs& a, typename Pop<F16C>::T* fs, const CellDeltas<Off, L::D>& d,
+                                              const float (&u)[3], const float (&S_)[3][3]) {
+    using P = Pop<F16C>;
+    constexpr int Q = L::Q, D = L::D;
+    const Off oT = (Off)a.lay.T;
+    float uu = 0.f;
+    static_for<0, D>([&](auto dc) { uu += u[dc.value] * u[dc.value]; });
+    auto population = [&](auto qc) -> float {
+        constexpr int q = decltype(qc)::value;
+        float fi = feq<L, q>(a.rho, u, uu, a.ddf != 0);
+        if (a.grad) {
+            float neq = 0.f;
+            static_for<0, D>([&](auto ac) {
+                static_for<0, D>([&](auto bc) {
+                    constexpr int A = ac.value, B = bc.value;
+                    constexpr float Qab = (float)(L::c(q, A) * L::c(q, B)) - (A == B ? (float)(1.0 / 3.0) : 0.f);
+                    neq += Qab * S_[A][B];
+                });
+            });
+            neq *= (-wf<L>(q) * a.rho * a.tau * 3.f) * ((a.tau - 1.f) / a.tau);
+            fi += neq;
+        }
+        return fi;
+    };
+    if (!a.esoteric) {
+        static_for<0, Q>([&](auto qc) { P::st(fs + (d.own + oT * qc.value), population(qc)); });
+    } else {
+        P::st(fs + d.own, population(std::integral_constant<int, 0>{}));
+        static_for<1, Q - 1, 2>([&](auto qc) {
+            constexpr int pos = qc.value, neg = pos + 1;
+            P::st(fs + (d.template at<L::c(pos, 0), L::c(pos, 1), L::c(pos, 2)>() + oT * pos), population(qc));
+            P::st(fs + (d.own + oT * neg), population(std::integral_constant<int, neg>{}));
+        });
+    }
+}
 
 // initialize_f_from_func (src/lbm/preprocess/initial_condition.mojo:86-179) with fi_neq
 // (:182-234); esoteric pull stores with the odd-step pattern (:172-174).
@@ -493,7 +638,7 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
         for (uint32_t i = threadIdx.x; i < (32u << b.sp); i += kBrickThreads) {
             const uint32_t fast = i & ((1u << sf) - 1u), g = i >> sf;
             const int32_t x = x0 + (int32_t)(D == 3 ? g >> b.sby : g);
-            const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : z0;
+            const int32_t y = y0 + (int32_t)(D == 3 ? g & ((1u << b.sby) - 1u) : fast), z = D == 3 ? z0 + (int32_t)fast : 0;
             if (x >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
             const uint32_t slot = g * ((1u << sf) + 1u) + fast;
             const uint32_t r = ((uint32_t)x * (uint32_t)a.lay.ny + (uint32_t)y) * (uint32_t)a.lay.nz + (uint32_t)z;
@@ -513,7 +658,6 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
     const int32_t x = x0 + lx;
     S* fs = (S*)a.f;
     CellDeltas<Off, D> d;
-    const Off own_z = D == 2 && a.lay.nz > 1 ? plane_offset(a.lay, b, z0, TQ) : 0;  // (3D: planes.own)
     Off own_xy;
     auto row_deltas = [&](int32_t y) -> Off {
         const uint32_t by = a.lay.d_ty.div((uint32_t)y), iy = (uint32_t)y - by * (uint32_t)a.lay.ty;
@@ -528,7 +672,7 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
     }
 #pragma unroll 1
     for (int32_t p = (int32_t)(threadIdx.x >> 5); p < (1 << b.sp); p += (int32_t)(kBrickThreads / 32u)) {
-        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : z0;
+        const int32_t y = D == 3 ? y0 + ly : y0 + (p << b.sby) + ly, z = D == 3 ? z0 + p : 0;
         if (x >= a.lay.nx || y >= a.lay.ny || z >= a.lay.nz) continue;
         const uint32_t slot = D == 3 ? ((uint32_t)((lx << b.sby) + ly) * ((1u << sf) + 1u) + (uint32_t)p)
                                      : (uint32_t)lx * ((1u << sf) + 1u) + (uint32_t)((p << b.sby) + ly);
@@ -538,69 +682,67 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
             d.z[0] = planes.own[p] - oz;
             d.z[2] = planes.own[p + 2] - oz;
         } else {
-            d.flat = own_xy + row_deltas(y);
-            d.own = d.flat + own_z;
+            d.own = d.flat = own_xy + row_deltas(y);
         }
         float u[3] = {0.f, 0.f, 0.f};
         if (a.u) static_for<0, D>([&](auto dc) { u[dc.value] = field[dc.value][slot]; });
-        float uu = 0.f;
-        static_for<0, D>([&](auto dc) { uu += u[dc.value] * u[dc.value]; });
         float S_[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
         if (a.grad)
             static_for<0, NS>([&](auto nc) {
                 constexpr int n = nc.value, A = sa<L>(n), B = sb<L>(n);
                 S_[A][B] = S_[B][A] = field[D + n][slot];
             });
-        auto population = [&](auto qc) -> float {
-            constexpr int q = decltype(qc)::value;
-            float fi = feq<L, q>(a.rho, u, uu, a.ddf != 0);
-            if (a.grad) {
-                float neq = 0.f;
-                static_for<0, D>([&](auto ac) {
-                    static_for<0, D>([&](auto bc) {
-                        constexpr int A = ac.value, B = bc.value;
-                        constexpr float Qab = (float)(L::c(q, A) * L::c(q, B)) - (A == B ? (float)(1.0 / 3.0) : 0.f);
-                        neq += Qab * S_[A][B];
-                    });
-                });
-                neq *= (-wf<L>(q) * a.rho * a.tau * 3.f) * ((a.tau - 1.f) / a.tau);
-                fi += neq;
-            }
-            return fi;
-        };
-        if (!a.esoteric) {
-            static_for<0, Q>([&](auto qc) { P::st(fs + (d.own + oT * qc.value), population(qc)); });
-        } else {
-            P::st(fs + d.own, population(std::integral_constant<int, 0>{}));
-            static_for<1, Q - 1, 2>([&](auto qc) {
-                constexpr int pos = qc.value, neg = pos + 1;
-                P::st(fs + (d.template at<L::c(pos, 0), L::c(pos, 1), L::c(pos, 2)>() + oT * pos), population(qc));
-                P::st(fs + (d.own + oT * neg), population(std::integral_constant<int, neg>{}));
-            });
-        }
+        store_initial<L, F16C>(a, fs, d, u, S_);
     }
+}
+
+// The same, one thread per cell in tile order (by_cell).
+template <class L, bool F16C, class Off>
+__global__ void __launch_bounds__(256) init_cell_kernel(const __grid_constant__ InitArgs a) {
+    constexpr int D = L::D;
+    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x, N = a.lay.ncells;
+    if (n >= N) return;
+    const AnyCell<L, Off> c(a.lay, n);
+    const uint32_t r = c.row(a.lay);
+    float u[3] = {0.f, 0.f, 0.f}, S_[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+    if (a.u) static_for<0, D>([&](auto dc) { u[dc.value] = __ldg(a.u + (size_t)N * dc.value + r); });
+    if (a.grad)
+        static_for<0, L::NS>([&](auto nc) {
+            constexpr int k = nc.value, A = sa<L>(k), B = sb<L>(k);
+            S_[A][B] = S_[B][A] = 0.5f * (__ldg(a.grad + (size_t)N * (A * D + B) + r) + __ldg(a.grad + (size_t)N * (B * D + A) + r));
+        });
+    store_initial<L, F16C>(a, (typename Pop<F16C>::T*)a.f, c.d, u, S_);
 }
 
 template <class L>
 cudaError_t launch_init(const InitArgs& a, bool f16, cudaStream_t s) {
-    const uint32_t blocks = a.brick.nbx * a.brick.nby * a.brick.nbz;
     const bool narrow = (uint64_t)a.lay.ncells * L::Q < (1ull << 31);
-    if (f16) {
-        if (narrow) init_kernel<L, true, int32_t><<<blocks, kBrickThreads, 0, s>>>(a);
-        else init_kernel<L, true, int64_t><<<blocks, kBrickThreads, 0, s>>>(a);
-    } else {
-        if (narrow) init_kernel<L, false, int32_t><<<blocks, kBrickThreads, 0, s>>>(a);
-        else init_kernel<L, false, int64_t><<<blocks, kBrickThreads, 0, s>>>(a);
-    }
-    return cudaGetLastError();
+    const bool cells = by_cell(a.lay, a.brick, L::D, kInitOp, a.esoteric != 0, a.u || a.grad);
+    const uint32_t blocks = cells ? (a.lay.ncells - 1u) / 256u + 1u : a.brick.nbx * a.brick.nby * a.brick.nbz;
+    auto go = [&](auto f16c, auto off) {
+        constexpr bool F = decltype(f16c)::value;
+        using Off = decltype(off);
+        if (cells) init_cell_kernel<L, F, Off><<<blocks, 256, 0, s>>>(a);
+        else init_kernel<L, F, Off><<<blocks, kBrickThreads, 0, s>>>(a);
+        return cudaGetLastError();
+    };
+    if (f16) return narrow ? go(std::true_type{}, int32_t{}) : go(std::true_type{}, int64_t{});
+    return narrow ? go(std::false_type{}, int32_t{}) : go(std::false_type{}, int64_t{});
 }
 
 // Launches the outputs of one lattice (lbm_fields_*.cu): rho and u, or with qcrit the Q-criterion.
 template <class L, bool F16C, bool ESO, bool QCRIT>
 cudaError_t launch_rho_u_impl(const RhoUArgs& a, cudaStream_t s) {
-    const uint32_t blocks = a.brick.nbx * a.brick.nby * a.brick.nbz;
-    if ((uint64_t)a.lay.ncells * L::Q < (1ull << 31)) rho_u_kernel<L, F16C, ESO, QCRIT, int32_t><<<blocks, kBrickThreads, 0, s>>>(a);
-    else rho_u_kernel<L, F16C, ESO, QCRIT, int64_t><<<blocks, kBrickThreads, 0, s>>>(a);
+    const bool narrow = (uint64_t)a.lay.ncells * L::Q < (1ull << 31);
+    if (by_cell(a.lay, a.brick, L::D, QCRIT ? kQOp : kRhoUOp, ESO)) {
+        const uint32_t blocks = (a.lay.ncells - 1u) / 256u + 1u;
+        if (narrow) rho_u_cell_kernel<L, F16C, ESO, QCRIT, int32_t><<<blocks, 256, 0, s>>>(a);
+        else rho_u_cell_kernel<L, F16C, ESO, QCRIT, int64_t><<<blocks, 256, 0, s>>>(a);
+    } else {
+        const uint32_t blocks = a.brick.nbx * a.brick.nby * a.brick.nbz;
+        if (narrow) rho_u_kernel<L, F16C, ESO, QCRIT, int32_t><<<blocks, kBrickThreads, 0, s>>>(a);
+        else rho_u_kernel<L, F16C, ESO, QCRIT, int64_t><<<blocks, kBrickThreads, 0, s>>>(a);
+    }
     return cudaGetLastError();
 }
 template <class L>

@@ -706,6 +706,11 @@ struct AnyCell {
             axis_deltas<Off>(lz, (uint32_t)l.tz, bz, (uint32_t)l.ntz, (Off)l.tx * (Off)l.ty,
                              TQ * (Off)l.ntx * (Off)l.nty, d.z);
     }
+    // row-major index (x ny + y) nz + z
+    __device__ __forceinline__ uint32_t row(const LayoutDesc& l) const {
+        return ((bx * (uint32_t)l.tx + lx) * (uint32_t)l.ny + by * (uint32_t)l.ty + ly) * (uint32_t)l.nz +
+               bz * (uint32_t)l.tz + lz;
+    }
     // neighbour tables (flag and bc indices), for the cells next to a flag
     __device__ __forceinline__ void nbr(const LayoutDesc& l, Nbr& nb) const {
         nb.ax.init(lx, bx, l.tx, l.ntx, 1u, 1u);
@@ -765,8 +770,8 @@ __device__ __forceinline__ void add_resting_walls(float (&f)[L::Q], uint32_t cle
 }
 
 // set_adjacent_flags (ops/load_and_store.mojo:270-291) of a cell of any layout: its masks; any: an own
-// or neighbouring flag is not 0.  (Flags by load_byte: a step calls this behind its grid wait.)
-template <class L>
+// or neighbouring flag is not 0.  WAITED: flags by load_byte (a step calls this behind its grid wait).
+template <class L, bool WAITED>
 __device__ __forceinline__ uint2 any_solid_masks(const uint8_t* flags, uint32_t own, const LayoutDesc& l,
                                                  const Nbr& nb, uint32_t& any) {
     uint32_t raw_solid = 0u, nib_solid = 0u;
@@ -774,7 +779,10 @@ __device__ __forceinline__ uint2 any_solid_masks(const uint8_t* flags, uint32_t 
     static_for<1, L::Q>([&](auto qc) {
         constexpr int q = qc.value;
         constexpr int sx = -L::c(q, 0), sy = -L::c(q, 1), sz = -L::c(q, 2);
-        const uint32_t pf = load_byte(flags + (nb.template loc<sx, sy, sz>() + l.T * nb.template til<sx, sy, sz>()));
+        const uint8_t* p = flags + (nb.template loc<sx, sy, sz>() + l.T * nb.template til<sx, sy, sz>());
+        uint32_t pf;
+        if constexpr (WAITED) pf = load_byte(p);
+        else pf = *p;
         any |= pf;
         if (pf == LBM_FLAG_SOLID) raw_solid |= 1u << q;
         if ((pf & 0x0F) == LBM_FLAG_SOLID) nib_solid |= 1u << q;
@@ -902,7 +910,7 @@ __global__ void __launch_bounds__(256, (any_min_blocks<L, COLL>())) step_kernel(
         Nbr nb;
         AnyCell<L, Off>(a.lay, n).nbr(a.lay, nb);
         uint32_t any;
-        m = any_solid_masks<L>(a.flags, load_byte(a.flags + n), a.lay, nb, any);
+        m = any_solid_masks<L, true>(a.flags, load_byte(a.flags + n), a.lay, nb, any);
     }
     any_cell<L, METHOD, F16C, COLL, LES, Off, true>(a, n, m);
 }
