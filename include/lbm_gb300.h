@@ -109,7 +109,7 @@ typedef struct lbm_config_t {
 /* lbm_grid_t mirrors LBM_Grid's comptime shape and tile (src/lbm/grid.mojo:55-107). */
 typedef struct lbm_grid_t {
     int32_t lattice;           /* LBM_D2Q9 / LBM_D3Q19 / LBM_D3Q27                 */
-    int32_t nx, ny, nz;        /* nz == 1 for D2Q9                                  */
+    int32_t nx, ny, nz;        /* D2Q9: two extents above 1, as a rule nx and ny    */
     int32_t tx, ty, tz;        /* tile shape; each must divide its extent           */
 } lbm_grid_t;
 
@@ -200,7 +200,11 @@ lbm_status lbm_double_buffer_step(lbm_handle* h, void* f_out, const void* f_in, 
 lbm_status lbm_esoteric_pull_step(lbm_handle* h, void* f, float* bc, const uint8_t* flags,
                                   float tau, int32_t is_even_step, void* stream);
 
-/* The host time loop of examples/LDC.mojo:133-135 as one call: n_steps steps replayed from a
+/* Step calls and runs of fewer than 64 steps may be captured into a graph of the caller's, and calls on
+ * several streams may overlap, each with its own buffers and boundary values; on the block-per-tile kernels
+ * overlapping calls must pass the same flags, as a call that is complete has seen them.
+ *
+ * The host time loop of examples/LDC.mojo:133-135 as one call: n_steps steps replayed from a
  * CUDA graph captured per (buffers, tau, parity).  Double buffer: step k reads f_a when
  * (first_step + k) is even, else f_b.  Esoteric pull: f_b is ignored and step k is even when
  * (first_step + k) is even. */

@@ -52,7 +52,7 @@ def best_tile(config, lattice, nx: int, ny: int, nz: int, *, flags=None, bc=None
 def batch_tile(shapes, build, *, steps: int = 50, stream=None, samples: int = 4):
     """Tile for a batch of domains of one lattice and configuration: the candidates that divide
     every shape, each timed as a batch of about the same total size made of replicas of `samples`
-    domains at evenly spaced quantiles of the size distribution (one persistent launch per step,
+    domains at evenly spaced quantiles of the size distribution (one launch per step,
     graph-replayed).  Every replica has its own copy of its domain's flags and boundary values, so
     their reads cost what they cost in the real batch.  build(shape, tile) returns (grid, config,
     flags, bc, tau, links) with host arrays in that tile's layout, links None or (fluid ids,

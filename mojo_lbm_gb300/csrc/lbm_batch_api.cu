@@ -167,7 +167,7 @@ bool use_batch_pair(const lbm_batch* b) {
 // form, 8 in the per-cell one.  More units share a descriptor and its load latency, fewer balance the
 // SMs (us a step of 128 / 16 / 4 channels, 58,000 / 7,200 / 1,800 units; cell pairs: 1 unit 217 / 36.2 / 11.6,
 // 2 196 / 35.3 / 12.8, 4 190 / 35.8 / 13.4, 8 195 / 40.4 / 18.4; per cell: 4 213 / 37.2 / 13.7, 8 213 / 41.6 /
-// 15.1, 16 216 / 45.2 / 21.9).
+// 15.1, 16 216 / 45.2 / 21.9).  The form with fused links was not swept and takes the per-cell line.
 uint32_t units_per_cta(const lbm_batch* b, bool pair) {
     const uint32_t waves = 3u * 8u * (uint32_t)b->sms;
     return std::max(1u, std::min(pair ? 4u : 8u, b->unit_begin.back() / waves));

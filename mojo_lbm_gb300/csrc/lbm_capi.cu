@@ -412,7 +412,12 @@ int any_threads(const lbm_config_t& c) { return c.collision_op == LBM_KBC ? 256 
 
 bool use_tile(const lbm_handle* h) { return h->step_tile != nullptr && h->path != 1; }
 
-// Two waves of the cell-pair kernel's CTAs (8 per SM) on the 152 SMs of a GB300.
+// Two waves of the cell-pair kernel's CTAs (8 per SM) on the 152 SMs of a GB300.  us a step in graph replays,
+// per cell / pair, float32 SRT cavities unless said: D2Q9 256 tiles 2.17 / 2.90, 640 3.20 / 4.08, 1024 4.13 / 4.17,
+// 1600 5.38 / 5.52, 2112 6.47 / 6.39, 2500 7.30 / 7.24, 4096 11.53 / 10.83 (Float16C fast 1024 4.03 / 3.80, 2112
+// 6.40 / 5.56); D3Q19 1024 6.68 / 7.50, 2000 11.17 / 11.85, 2640 17.10 / 17.17, 4096 26.31 / 26.23 (Float16C fast 1296
+// 7.72 / 7.99, 2000 10.68 / 10.39, 2640 13.26 / 12.51; TRT 2640 18.22 / 20.02, 4096 27.44 / 29.56; Smagorinsky 19.62 /
+// 22.63 and 28.92 / 32.12: for those two the line lies above 4096).
 constexpr uint32_t kPairAutoMinTiles = 2u * 8u * 152u;
 
 // Where the cell-pair kernel measured faster than the per-cell one on large grids (us a step, pair / per
@@ -443,8 +448,7 @@ bool use_staged(const lbm_handle* h) {
 // The cell-pair kernel is chosen (path 3) and can run: no learned closure, no fused links.
 // The automatic choice (path 0) takes it where it measured faster than the per-cell kernel: the
 // configurations of pair_pays on grids of at least kPairAutoMinTiles tiles.  On fewer tiles the step
-// is latency-bound, and the per-cell kernel, which gives each pair two threads, finishes sooner
-// (the 256^2 D2Q9 cavity, 256 tiles: 3.2 against 4.3 us a step).
+// is latency-bound, and the per-cell kernel, which gives each pair two threads, finishes sooner.
 bool use_pair(const lbm_handle* h) {
     return ((h->path == 3 && h->step_pair != nullptr) || (h->path == 0 && h->pair_auto)) && !h->closure_on &&
            !h->link_table;

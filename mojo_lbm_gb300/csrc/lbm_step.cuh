@@ -738,9 +738,9 @@ __device__ __forceinline__ uint2 cell_masks_of(uint32_t own, uint32_t raw_solid,
 // moving-wall term of the wall's bc is exactly +0 (velocity component 0, a positive finite density), so
 // that the step neither reads that bc nor adds the term; it only adds the +0 (a bounced -0 becomes +0).
 // Valid for the bc values at the time of the call: a multi-step run builds these masks at its start.
-// moving_wall_bc reads 2 to 4 words of the wall's bc one direction after the other, and took 4 % of a
-// step of the 256^3 float32 cavity, 9 % of the Float16C one and 14 % of the 256^2 D2Q9 one, whose walls
-// all rest but the lid.  bc_base(q): element offset of component 0 of the pull neighbour's bc.
+// moving_wall_bc reads 2 to 4 words of the wall's bc one direction after the other, and takes 2 % of a
+// step of the 256^3 float32 cavity, 7 % of the Float16C one and 11 to 18 % at 96^3, whose walls all rest
+// but the lid (lbm_masks.h).  bc_base(q): element offset of component 0 of the pull neighbour's bc.
 template <class L, class BcBase>
 __device__ __forceinline__ uint2 without_resting_walls(uint2 m, const float* __restrict__ bc, uint32_t T, BcBase&& bc_base) {
     static_for<1, L::Q>([&](auto qc) {
@@ -1468,7 +1468,7 @@ constexpr int tile_min_blocks() {
 // Whole CTAs stay where they are the faster ones: exact KBC (256^3 D3Q27 1864 / 2061, D3Q19 in place 842 /
 // 869: its code is the longest, and the warps of one CTA run through it together), D2Q9 in place (256^2 2.40 /
 // 2.46) and fast (1.96 / 2.09), D3Q19 in place Float16C without LES (402 / 408) and fast (420 / 423).  (The
-// fused-link kernels were not measured and keep them.)
+// fused-link kernels were not measured in half CTAs and keep whole ones.)
 template <class L, int METHOD, bool F16C, int COLL, int LES, bool FAST, bool LINKS>
 constexpr int tile_threads() {
     constexpr bool ESO = METHOD == LBM_ESOTERIC_PULL;
