@@ -575,7 +575,8 @@ lbm_status summary(lbm_handle* h, const uint8_t* flags, float* bc, int64_t n_ste
     m = Masks{nullptr, nullptr};
     const bool walls = h->cfg.include_moving_boundary && !h->cfg.capture_density && !h->cfg.capture_velocity;
     bool resting = walls && n_steps >= kRestingMinSteps;
-    const bool capturing = is_captured(s);
+    // (asked only where it matters: the query costs a run of few steps about a microsecond)
+    const bool capturing = (use_tile(h) ? resting || !h->summary_valid : masks_pay(h, n_steps)) && is_captured(s);
     const bool own = !capturing && (use_tile(h) ? resting : masks_pay(h, n_steps)) && h->owner.is(s);
     if (!use_tile(h) && !own) return LBM_OK;
     resting = resting && own;
