@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kBrickThreads, L::Q == 27 ? 3 : LBM_FIELDS_MIN
             d.z[0] = planes.own[p] - oz;
             d.z[2] = planes.own[p + 2] - oz;
         } else {
-            d.own = d.flat = own_xy + row_deltas(y);
+            d.own = d.flat = own_xy + row_deltas(y);  // (2D bricks lie in the plane z = 0)
         }
         if (flagged && fl[at] == LBM_FLAG_SOLID) {
             if constexpr (!QCRIT) {
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(kBrickThreads) init_kernel(const __grid_consta
             d.z[0] = planes.own[p] - oz;
             d.z[2] = planes.own[p + 2] - oz;
         } else {
-            d.own = d.flat = own_xy + row_deltas(y);
+            d.own = d.flat = own_xy + row_deltas(y);  // (2D bricks lie in the plane z = 0)
         }
         float u[3] = {0.f, 0.f, 0.f};
         if (a.u) static_for<0, D>([&](auto dc) { u[dc.value] = field[dc.value][slot]; });
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(256) init_cell_kernel(const __grid_constant__ 
 
 template <class L>
 cudaError_t launch_init(const InitArgs& a, bool f16, cudaStream_t s) {
-    const bool narrow = (uint64_t)a.lay.ncells * L::Q < (1ull << 31);
+    const bool narrow = offsets32<L>(a.lay);
     const bool cells = by_cell(a.lay, a.brick, L::D, kInitOp, a.esoteric != 0, a.u || a.grad);
     const uint32_t blocks = cells ? (a.lay.ncells - 1u) / 256u + 1u : a.brick.nbx * a.brick.nby * a.brick.nbz;
     auto go = [&](auto f16c, auto off) {
@@ -733,7 +733,7 @@ cudaError_t launch_init(const InitArgs& a, bool f16, cudaStream_t s) {
 // Launches the outputs of one lattice (lbm_fields_*.cu): rho and u, or with qcrit the Q-criterion.
 template <class L, bool F16C, bool ESO, bool QCRIT>
 cudaError_t launch_rho_u_impl(const RhoUArgs& a, cudaStream_t s) {
-    const bool narrow = (uint64_t)a.lay.ncells * L::Q < (1ull << 31);
+    const bool narrow = offsets32<L>(a.lay);
     if (by_cell(a.lay, a.brick, L::D, QCRIT ? kQOp : kRhoUOp, ESO)) {
         const uint32_t blocks = (a.lay.ncells - 1u) / 256u + 1u;
         if (narrow) rho_u_cell_kernel<L, F16C, ESO, QCRIT, int32_t><<<blocks, 256, 0, s>>>(a);

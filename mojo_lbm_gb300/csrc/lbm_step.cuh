@@ -129,13 +129,15 @@ __device__ __forceinline__ void axis_deltas(uint32_t l, uint32_t t, uint32_t b, 
 // Population offsets of a cell and its neighbours.  Off: int32_t when the lattice has fewer than
 // 2^31 elements (one three-input add and one wide multiply-add per load), else int64_t.
 // The neighbours of a 2D lattice are those in the plane z = 0 (get_adjacent_idx takes z = 0 for it), also on
-// a grid that extends along z and x or y only: flat is the cell's place in that plane.
+// a grid that extends along z and x or y only: flat is the cell's place in that plane.  Such grids take the
+// 64-bit offsets (offsets32): in the 32-bit ones the second address cost a 718 x 755 D2Q9 cavity 1 %.
 template <class Off, int D>
 struct CellDeltas {
+    static constexpr bool FLAT = D == 2 && sizeof(Off) == 8;
     Off own, flat, x[3], y[3], z[3];
     template <int SX, int SY, int SZ>
     __device__ __forceinline__ Off at() const {
-        Off o = D == 3 ? own : flat;
+        Off o = FLAT ? flat : own;
         if constexpr (SY != 0) o += y[SY + 1];
         if constexpr (SZ != 0) o += z[SZ + 1];
         if constexpr (SX != 0) o += x[SX + 1];
@@ -678,6 +680,12 @@ cudaError_t launch_pdl(void (*kernel)(P...), uint32_t grid, uint32_t block, cuda
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Do 32-bit population offsets serve the grid?
+template <class L>
+inline bool offsets32(const LayoutDesc& l) {
+    return (uint64_t)l.ncells * L::Q < (1ull << 31) && (L::D == 3 || l.nz == 1);
+}
+
 // Position of cell n of any layout, and its population offsets.
 template <class L, class Off>
 struct AnyCell {
@@ -689,7 +697,7 @@ struct AnyCell {
         loc = n - tile * l.T;
         const uint32_t lyz = l.d_tx.div(loc);
         lx = loc - lyz * (uint32_t)l.tx;
-        const bool deep = D == 3 || l.nz > 1;  // (uniform)
+        constexpr bool deep = D == 3 || CellDeltas<Off, D>::FLAT;
         lz = deep ? l.d_ty.div(lyz) : 0u;
         ly = lyz - lz * (uint32_t)l.ty;
         const uint32_t byz = l.d_ntx.div(tile);
@@ -698,7 +706,7 @@ struct AnyCell {
         by = byz - bz * (uint32_t)l.nty;
         const Off TQ = (Off)l.T * L::Q;
         d.own = (Off)loc + TQ * (Off)tile;
-        if constexpr (D == 2)
+        if constexpr (CellDeltas<Off, D>::FLAT)
             d.flat = d.own - ((Off)lz * (Off)(l.tx * l.ty) + TQ * (Off)bz * (Off)(l.ntx * l.nty));
         axis_deltas<Off>(lx, (uint32_t)l.tx, bx, (uint32_t)l.ntx, 1, TQ, d.x);
         axis_deltas<Off>(ly, (uint32_t)l.ty, by, (uint32_t)l.nty, (Off)l.tx, TQ * (Off)l.ntx, d.y);
@@ -1543,7 +1551,7 @@ using StepLaunch = cudaError_t (*)(const StepArgs&, int threads, cudaStream_t);
 template <class L, int METHOD, bool F16C, int COLL, int LES>
 cudaError_t launch_step(const StepArgs& a, int threads, cudaStream_t s) {
     const uint32_t blocks = (a.lay.ncells + (uint32_t)threads - 1u) / (uint32_t)threads;
-    if ((uint64_t)a.lay.ncells * L::Q < (1ull << 31))
+    if (offsets32<L>(a.lay))
         return launch_pdl(step_kernel<L, METHOD, F16C, COLL, LES, int32_t>, blocks, (uint32_t)threads, s, a);
     return launch_pdl(step_kernel<L, METHOD, F16C, COLL, LES, int64_t>, blocks, (uint32_t)threads, s, a);
 }
